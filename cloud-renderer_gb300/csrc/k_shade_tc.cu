@@ -302,7 +302,8 @@ __global__ void __launch_bounds__(128 * SHADE_GROUPS, ctas_per_sm<NL>())
             ntile = nntile;
             nslot = nnslot;
         } else {
-            ntile = *s_claim;  // written at layer 0, one barrier ago
+            group_sync_or(g, false);  // thread 0's claim of this tile's only layer
+            ntile = *s_claim;
         }
     }
     if (!failed) failed = group_sync_for_mma(g, bad);  // the last tile's waits
