@@ -185,7 +185,7 @@ struct SampleBuf {
     float2* light_lane;
     float* contrib;   // per slot: the sample's shaded contribution (surrogate path)
     unsigned* count;  // samples per region
-    // flat order (written by the march): each march CTA's 8 regions occupy a
+    // flat order (written by the march): each march CTA's regions occupy a
     // contiguous range, padded to 32-sample chunks; slot_of[i] = slot
     // (region * capacity + j) of flat row i, or CG_NO_SLOT for padding;
     // *flat_total = padded total (zeroed before the march)

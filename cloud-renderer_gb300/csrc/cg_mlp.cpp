@@ -257,8 +257,9 @@ cg_status ensure_samples(cg_context* ctx, int width, int height, int view_steps,
     CG_CHECK(n < (size_t)0xFFFFFFFFu, CG_ERR_OUT_OF_RANGE,
              "render: %zu sample slots (pixels x view_steps) exceed 2^32", n);
     // counts, step counts, flat total, step tables (2 words each), flat slots
-    // (the padded flat order has at most 31 padding rows per 8 regions)
-    const size_t flat = n + 32 * (regions / 8 + 1);
+    // (each march CTA's samples are padded to whole 32-row chunks, which its
+    // regions' capacity, a multiple of 32, already covers)
+    const size_t flat = n + 32;
     const size_t idx_words = 2 * regions + 2 + 2 * regions * view_steps + 2 + flat;
     const size_t pixels = (size_t)width * height;
     if (ctx->samples_pw.bytes < n * 16 || ctx->samples_gl.bytes < n * 8 ||

@@ -166,6 +166,40 @@ __device__ __forceinline__ float2 quad_hw(const VolDesc& vd, float px, float py,
     return a;
 }
 
+// Occupancy along a ray, linear in the march step k: brick coordinates
+// a + k b per axis in the grid of one level.
+struct OccRay {
+    float a[3], b[3];
+    const uint8_t* grid;
+    int nb, bound;
+
+    // Positions v(k) = v0 + k dv (level-0 voxels), bricks of edge S voxels whose
+    // first one starts `shift` voxels before the volume.
+    __device__ __forceinline__ void set(const VolDesc& vd, int l, const float v0[3],
+                                        const float dv[3], float S, float shift) {
+        const float r = 1.f / S;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            a[i] = (v0[i] + shift) * r;
+            b[i] = dv[i] * r;
+        }
+        grid = vd.occ + vd.occ_off[l];
+        nb = vd.occ_nb[l];
+        bound = vd.occ_total - vd.occ_off[l];
+    }
+    // The flag of the brick holding step k (clamped to the grid).
+    __device__ __forceinline__ bool at(float k) const {
+        constexpr float MAGIC = 12582912.f;  // 1.5 * 2^23: floor and integer in one addition
+        constexpr int BIAS = 0x4B400000;
+        const int x = __vimin_s32_relu(__float_as_int(__fadd_rd(fmaf(k, b[0], a[0]), MAGIC)) - BIAS, nb - 1);
+        const int y = __vimin_s32_relu(__float_as_int(__fadd_rd(fmaf(k, b[1], a[1]), MAGIC)) - BIAS, nb - 1);
+        const int z = __vimin_s32_relu(__float_as_int(__fadd_rd(fmaf(k, b[2], a[2]), MAGIC)) - BIAS, nb - 1);
+        const int i = (z * nb + y) * nb + x;
+        if (!CG_IN_BOUNDS(i, bound)) return false;
+        return __ldg(grid + i) != 0;
+    }
+};
+
 // View-march steps k (sample at t_k = tin + (k + 1/2) dt along the unit
 // direction d from the eye) that can meet the occupied level-0 box (widened by
 // one voxel, and by one step at either end): [k0, k1], empty (k0 > k1) when
