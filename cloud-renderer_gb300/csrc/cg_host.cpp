@@ -1191,10 +1191,13 @@ extern "C" cg_status cg_render(cg_context* ctx, const cg_volume* v, const cg_cam
         SampleBuf sb;
         st = ensure_samples(ctx, cam->width, cam->height, params->view_steps, sb);
         if (st != CG_OK) return st;
-        // the shading status block is cleared before the march, so that the
-        // shading kernel directly follows it (a dependent launch)
-        if (params->use_mlp) CG_CUDA(cudaMemsetAsync(ctx->fallbacks.p, 0, 32, s));
-        CG_LAUNCH(ctx, launch_march(vd, cd, tp, sb, params->use_mlp != 0, s));
+        // (the surrogate's march also clears the shading status block: the
+        // shading kernel directly follows it, a dependent launch)
+        if (params->use_mlp)
+            CG_LAUNCH(ctx, launch_march_mlp(vd, cd, tp, sb, dst,
+                                            ctx->fallbacks.as<unsigned long long>(), s));
+        else
+            CG_LAUNCH(ctx, launch_march(vd, cd, tp, sb, s));
         stage_mark(ctx, s, "march");
         if (params->use_mlp) {
             ctx->shaded_valid = true;
@@ -1274,7 +1277,7 @@ extern "C" cg_status cg_march_samples(cg_context* ctx, const cg_volume* v, const
     SampleBuf sb;
     st = ensure_samples(ctx, cam->width, cam->height, params->view_steps, sb);
     if (st != CG_OK) return st;
-    CG_LAUNCH(ctx, launch_march(desc_of(v), cd, tp, sb, false, s));
+    CG_LAUNCH(ctx, launch_march(desc_of(v), cd, tp, sb, s));
     const size_t regions = (size_t)((cam->width + 15) / 16) * ((cam->height + 15) / 16) * 8;
     std::vector<unsigned> cnt(regions);
     CG_CUDA(cudaMemcpyAsync(cnt.data(), sb.count, regions * 4, cudaMemcpyDeviceToHost, s));

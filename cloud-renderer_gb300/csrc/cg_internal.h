@@ -188,9 +188,13 @@ struct SampleBuf {
     // flat order (written by the march): each march CTA's regions occupy a
     // contiguous range, padded to 32-sample chunks; slot_of[i] = slot
     // (region * capacity + j) of flat row i, or CG_NO_SLOT for padding;
-    // *flat_total = padded total (zeroed before the march)
+    // *flat_total = padded total (zeroed, with n_busy behind it, before the march)
     unsigned* slot_of;
     unsigned* flat_total;
+    // surrogate march: the *n_busy regions that recorded samples, in any order
+    // (the pixels of the others are finished by the march itself)
+    unsigned* n_busy;  // flat_total + 1
+    unsigned* busy;
     uint2* steps;     // per region, per emitting step: (first slot, lane ballot)
     unsigned* nsteps; // emitting steps per region
     float* alpha;     // per pixel (row-major, W x H): 1 - T after the march
@@ -339,8 +343,11 @@ struct TrainArgs {
 };
 
 // The view march (writes the samples, the step tables and sb.alpha).
-cudaError_t launch_march(VolDesc vd, CamDesc cam, TraceParams tp, SampleBuf sb, bool hw,
-                         cudaStream_t st);
+cudaError_t launch_march(VolDesc vd, CamDesc cam, TraceParams tp, SampleBuf sb, cudaStream_t st);
+// The surrogate's view march: also clears the shading status (4 words), lists
+// the regions with samples and writes the finished pixels of the others to dst.
+cudaError_t launch_march_mlp(VolDesc vd, CamDesc cam, TraceParams tp, SampleBuf sb, float4* dst,
+                             unsigned long long* status, cudaStream_t st);
 cudaError_t launch_shade_exact(VolDesc vd, CamDesc cam, TraceParams tp, SampleBuf sb,
                                float4* out, cudaStream_t st);
 cudaError_t launch_pack_level(VolDesc vd, int l, cudaSurfaceObject_t surf, cudaStream_t st);

@@ -256,11 +256,12 @@ cg_status ensure_samples(cg_context* ctx, int width, int height, int view_steps,
     const size_t n = regions * cap;
     CG_CHECK(n < (size_t)0xFFFFFFFFu, CG_ERR_OUT_OF_RANGE,
              "render: %zu sample slots (pixels x view_steps) exceed 2^32", n);
-    // counts, step counts, flat total, step tables (2 words each), flat slots
+    // counts, step counts, flat total and busy count, step tables (2 words
+    // each), flat slots, busy regions
     // (each march CTA's samples are padded to whole 32-row chunks, which its
     // regions' capacity, a multiple of 32, already covers)
     const size_t flat = n + 32;
-    const size_t idx_words = 2 * regions + 2 + 2 * regions * view_steps + 2 + flat;
+    const size_t idx_words = 2 * regions + 2 + 2 * regions * view_steps + 2 + flat + regions;
     const size_t pixels = (size_t)width * height;
     if (ctx->samples_pw.bytes < n * 16 || ctx->samples_gl.bytes < n * 8 ||
         ctx->samples_c.bytes < n * 4 || ctx->samples_cnt.bytes < idx_words * 4 ||
@@ -280,11 +281,13 @@ cg_status ensure_samples(cg_context* ctx, int width, int height, int view_steps,
     sb.count = ctx->samples_cnt.as<unsigned>();
     sb.nsteps = sb.count + regions;
     sb.flat_total = sb.nsteps + regions;
+    sb.n_busy = sb.flat_total + 1;
     // 8-byte aligned start for the (slot, ballot) pairs
-    size_t at = (size_t)(sb.flat_total + 1 - ctx->samples_cnt.as<unsigned>());
+    size_t at = (size_t)(sb.n_busy + 1 - ctx->samples_cnt.as<unsigned>());
     at = (at + 1) & ~(size_t)1;
     sb.steps = reinterpret_cast<uint2*>(ctx->samples_cnt.as<unsigned>() + at);
     sb.slot_of = ctx->samples_cnt.as<unsigned>() + at + 2 * regions * (size_t)view_steps;
+    sb.busy = sb.slot_of + flat;
     sb.capacity = (int)cap;
     sb.nslots = n;
     return CG_OK;

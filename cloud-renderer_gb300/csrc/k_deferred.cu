@@ -18,6 +18,8 @@
 // in 128-sample tiles, computing features, running the network and writing
 // each sample's contribution to the compact per-slot array; k_accumulate then
 // sums each pixel's contributions in step order.
+#include <algorithm>
+
 #include "cg_internal.h"
 #include "cg_mlp.cuh"
 #include "cg_sample.cuh"
@@ -71,10 +73,13 @@ constexpr int MARCH_FLAGS = 8;
 // HW: view samples and noise filtered by the texture unit (surrogate renderer).
 template <int FMT, bool HW>
 __global__ void __launch_bounds__(32 * MARCH_WARPS, 32 / MARCH_WARPS)
-    k_march(VolDesc vd, CamDesc cam, TraceParams tp, SampleBuf sb) {
+    k_march(VolDesc vd, CamDesc cam, TraceParams tp, SampleBuf sb, float4* dst,
+            unsigned long long* status) {
     // the shading pass may be scheduled once every march CTA has started: its
-    // CTAs stage their network while the last wave of the march runs
+    // CTAs stage their network while the last wave of the march runs (and read
+    // the samples and the status only once the march has completed)
     grid_dep_trigger();
+    if (HW && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < 4) status[threadIdx.x] = 0ull;
     constexpr int SHARE = 8 / MARCH_WARPS;
     const int lane = threadIdx.x & 31;
     const int region = (int)((blockIdx.y * (gridDim.x / SHARE) + blockIdx.x / SHARE) * 8 +
@@ -228,7 +233,16 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, 32 / MARCH_WARPS)
         sb.count[region] = cnt;
         sb.nsteps[region] = nsteps;
     }
-    if (valid) sb.alpha[(size_t)py * cam.W + px] = 1.f - T;
+    if (HW && cnt == 0u) {
+        // no sample in the region (nine tenths of a 1080p view): its pixels are
+        // done, and the accumulate pass neither reads nor writes them
+        if (valid)
+            dst[(size_t)py * cam.W + px] = make_float4(
+                0.f * tp.sun_color[0], 0.f * tp.sun_color[1], 0.f * tp.sun_color[2], 1.f - T);
+    } else {
+        if (HW && lane == 0) sb.busy[atomicAdd(sb.n_busy, 1u)] = (unsigned)region;
+        if (valid) sb.alpha[(size_t)py * cam.W + px] = 1.f - T;
+    }
     // Flat order for the shading pass: the CTA's regions take one contiguous
     // range (reserved with one atomic, padded to whole 32-sample chunks), and
     // every flat row records its sample's slot.
@@ -307,70 +321,82 @@ __global__ void __launch_bounds__(128) k_shade_exact(VolDesc vd, CamDesc cam, Tr
     write_rgb(sb.alpha, out, cam, px, py, acc + comp, tp);
 }
 
-// Per region: each pixel sums the contributions of its own samples in step
-// order, locating them through the march's step table (base slot, ballot).
+// Per busy region (one with samples; one warp each): each pixel sums the
+// contributions of its own samples in step order, locating them through the
+// march's step table (base slot, ballot).  A grid of warps walks the march's
+// list, so the regions without samples cost nothing here (1080p: 26 -> 19 us).
 __global__ void __launch_bounds__(128) k_accumulate(CamDesc cam, TraceParams tp, SampleBuf sb,
-                                                    int regions, int tiles_x, int view_steps,
-                                                    float4* dst) {
-    const int region = blockIdx.x * 4 + (threadIdx.x >> 5);
+                                                    int tiles_x, int view_steps, float4* dst) {
     grid_dep_wait();  // the contributions of the shading pass
-    if (region >= regions) return;
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
-    const unsigned ns = sb.nsteps[region];
-    const uint2* steps = sb.steps + (size_t)region * view_steps;
-    const float* cw = sb.contrib + (size_t)region * sb.capacity;
-    float acc = 0.f, comp = 0.f;
-    // the step table in coalesced chunks of 32 entries (lane e holds entry e),
-    // broadcast by shuffles; eight steps' contributions are fetched before
-    // any is summed, and the sums run in step order
-    for (unsigned base = 0; base < ns; base += 32u) {
-        const unsigned m = min(32u, ns - base);
-        const uint2 st_l = lane < (int)m ? steps[base + lane] : make_uint2(0u, 0u);
-        for (unsigned e0 = 0; e0 < m; e0 += 8u) {
-            float v[8];
-            unsigned have = 0u;
+    const unsigned nb = *sb.n_busy;
+    for (unsigned i = blockIdx.x * 4u + (threadIdx.x >> 5); i < nb; i += gridDim.x * 4u) {
+        const int region = (int)sb.busy[i];
+        const unsigned ns = sb.nsteps[region];
+        const uint2* steps = sb.steps + (size_t)region * view_steps;
+        const float* cw = sb.contrib + (size_t)region * sb.capacity;
+        float acc = 0.f, comp = 0.f;
+        // the step table in coalesced chunks of 32 entries (lane e holds entry
+        // e), broadcast by shuffles; eight steps' contributions are fetched
+        // before any is summed, and the sums run in step order
+        for (unsigned base = 0; base < ns; base += 32u) {
+            const unsigned m = min(32u, ns - base);
+            const uint2 st_l = lane < (int)m ? steps[base + lane] : make_uint2(0u, 0u);
+            for (unsigned e0 = 0; e0 < m; e0 += 8u) {
+                float v[8];
+                unsigned have = 0u;
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const int src = (int)(e0 + q) & 31;
-                const unsigned sx = __shfl_sync(0xffffffffu, st_l.x, src);
-                const unsigned sy = __shfl_sync(0xffffffffu, st_l.y, src);
-                v[q] = 0.f;
-                // entries past m are (0, 0): no lane emitted there
-                if (e0 + q < m && ((sy >> lane) & 1u) &&
-                    CG_IN_BOUNDS((size_t)region * sb.capacity + sx + __popc(sy & below),
-                                 sb.nslots)) {
-                    v[q] = cw[sx + __popc(sy & below)];
-                    have |= 1u << q;
+                for (int q = 0; q < 8; ++q) {
+                    const int src = (int)(e0 + q) & 31;
+                    const unsigned sx = __shfl_sync(0xffffffffu, st_l.x, src);
+                    const unsigned sy = __shfl_sync(0xffffffffu, st_l.y, src);
+                    v[q] = 0.f;
+                    // entries past m are (0, 0): no lane emitted there
+                    if (e0 + q < m && ((sy >> lane) & 1u) &&
+                        CG_IN_BOUNDS((size_t)region * sb.capacity + sx + __popc(sy & below),
+                                     sb.nslots)) {
+                        v[q] = cw[sx + __popc(sy & below)];
+                        have |= 1u << q;
+                    }
                 }
-            }
 #pragma unroll
-            for (int q = 0; q < 8; ++q)
-                if ((have >> q) & 1u) cgs::neumaier(acc, comp, v[q]);
+                for (int q = 0; q < 8; ++q)
+                    if ((have >> q) & 1u) cgs::neumaier(acc, comp, v[q]);
+            }
         }
+        int px, py;
+        region_pixel(region, lane, tiles_x, px, py);
+        write_rgb(sb.alpha, dst, cam, px, py, acc + comp, tp);
     }
-    int px, py;
-    region_pixel(region, lane, tiles_x, px, py);
-    write_rgb(sb.alpha, dst, cam, px, py, acc + comp, tp);
 }
 
 }  // namespace
 
 static int regions_of(const CamDesc& cam) { return ((cam.W + 15) / 16) * ((cam.H + 15) / 16) * 8; }
 
-cudaError_t launch_march(VolDesc vd, CamDesc cam, TraceParams tp, SampleBuf sb, bool hw,
-                         cudaStream_t st) {
+static dim3 march_grid(const CamDesc& cam) {
+    return dim3((cam.W + 15) / 16 * (8 / MARCH_WARPS), (cam.H + 15) / 16);
+}
+
+cudaError_t launch_march(VolDesc vd, CamDesc cam, TraceParams tp, SampleBuf sb, cudaStream_t st) {
     // the flat-order reservation counter starts from zero on every launch
     cudaError_t e = cudaMemsetAsync(sb.flat_total, 0, sizeof(unsigned), st);
     if (e != cudaSuccess) return e;
-    dim3 grd((cam.W + 15) / 16 * (8 / MARCH_WARPS), (cam.H + 15) / 16);
     constexpr int threads = 32 * MARCH_WARPS;
-    if (hw)
-        k_march<0, true><<<grd, threads, 0, st>>>(vd, cam, tp, sb);
-    else if (vd.fmt == 0)
-        k_march<0, false><<<grd, threads, 0, st>>>(vd, cam, tp, sb);
+    if (vd.fmt == 0)
+        k_march<0, false><<<march_grid(cam), threads, 0, st>>>(vd, cam, tp, sb, nullptr, nullptr);
     else
-        k_march<1, false><<<grd, threads, 0, st>>>(vd, cam, tp, sb);
+        k_march<1, false><<<march_grid(cam), threads, 0, st>>>(vd, cam, tp, sb, nullptr, nullptr);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_march_mlp(VolDesc vd, CamDesc cam, TraceParams tp, SampleBuf sb, float4* dst,
+                             unsigned long long* status, cudaStream_t st) {
+    // the flat-order reservation counter and the busy count start from zero
+    cudaError_t e = cudaMemsetAsync(sb.flat_total, 0, 2 * sizeof(unsigned), st);
+    if (e != cudaSuccess) return e;
+    k_march<0, true><<<march_grid(cam), 32 * MARCH_WARPS, 0, st>>>(vd, cam, tp, sb, dst, status);
     return cudaGetLastError();
 }
 
@@ -388,9 +414,11 @@ cudaError_t launch_shade_exact(VolDesc vd, CamDesc cam, TraceParams tp, SampleBu
 
 cudaError_t launch_accumulate(CamDesc cam, TraceParams tp, SampleBuf sb, float4* dst,
                               cudaStream_t st) {
-    const int regions = regions_of(cam), tiles_x = (cam.W + 15) / 16;
-    return launch_dependent(k_accumulate, dim3((regions + 3) / 4), dim3(128), 0, st, cam, tp, sb,
-                            regions, tiles_x, (int)tp.view_steps, dst);
+    // at most twelve CTAs per SM (152 SMs), which take the busy regions in turn
+    const int tiles_x = (cam.W + 15) / 16;
+    const int blocks = std::min((regions_of(cam) + 3) / 4, 152 * 12);
+    return launch_dependent(k_accumulate, dim3(blocks), dim3(128), 0, st, cam, tp, sb, tiles_x,
+                            (int)tp.view_steps, dst);
 }
 
 CG_OOB_TU(k_deferred)
