@@ -452,6 +452,23 @@ extern "C" cg_status cg_volume_create(cg_context* ctx, int dimension, float boun
         raw_total += nbl * nbl * nbl;
     }
     v->raw_total = raw_total;
+    // the density quads: levels the default cone (radius floor of two voxels)
+    // samples; finer ones would multiply the largest levels' memory and stores
+    v->quad_base = CG_QUAD_BASE;
+    size_t cells = 0;
+    for (int l = CG_QUAD_BASE; l < mips; ++l) {
+        const size_t p = (size_t)v->dims[l] + 3;
+        v->quad_p[l] = (int)p;
+        v->quad_off[l] = (int)cells;
+        cells += p * p * (p + 1);
+    }
+    v->quad_total = (int)cells;
+    if (cells > 0) {
+        const size_t bytes = cells * (format == CG_FORMAT_RGBA32F ? 16 : 8);
+        if (e == cudaSuccess) e = v->quads.ensure(bytes);
+        if (e == cudaSuccess) e = cudaMemsetAsync(v->quads.p, 0, bytes, ctx->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    }
     set_occ_layout(v, 4);  // the autotuner's pick on the batching and 1080p workloads
     // + the level-0 occupied box (6 ints) after the grids, 16-byte aligned
     if (e == cudaSuccess) e = v->occ.ensure(occ_box_offset(raw_total) + 32);
@@ -483,7 +500,7 @@ extern "C" void cg_volume_destroy(cg_volume* v) {
     DevBuf* bufs[] = {&v->pyr, &v->count, &v->dq, &v->mask, &v->boards,
                       &v->bcount, &v->boff, &v->bcursor, &v->blist,
                       &v->bdirty, &v->bhl,
-                      &v->keys, &v->posmap, &v->scratch, &v->occ};
+                      &v->keys, &v->posmap, &v->scratch, &v->occ, &v->quads};
     for (DevBuf* b : bufs) b->release();
     v->h_stage.release();
     if (v->boards_ready) cudaEventDestroy(v->boards_ready);
@@ -685,6 +702,13 @@ VolDesc desc_of(const cg_volume* v) {
     d.nvox = (long long)v->offs[v->L - 1] +
              (long long)v->dims[v->L - 1] * v->dims[v->L - 1] * v->dims[v->L - 1];
     d.occ_total = (int)v->occ_total;
+    d.quad = v->quads.p;
+    d.quad_base = v->quad_base;
+    d.quad_total = v->quad_total;
+    for (int l = 0; l < CG_MAX_LEVELS; ++l) {
+        d.quad_off[l] = v->quad_off[l];
+        d.quad_p[l] = v->quad_p[l];
+    }
     return d;
 }
 

@@ -170,6 +170,11 @@ struct cg_volume {
     SunFrame frame{};
     float sun_dir[3] = {0, 1, 0};
     DevBuf scratch;  // small scalars (active voxel count)
+    // density quads of levels quad_base .. L-1 (VolDesc), zeroed at creation;
+    // every voxel store of those levels also writes its four cells
+    DevBuf quads;
+    int quad_base = 0, quad_total = 0;
+    int quad_off[CG_MAX_LEVELS] = {}, quad_p[CG_MAX_LEVELS] = {};
     DevBuf occ;      // raw occupancy cells (OccRaw), then the brick grids (VolDesc)
     int raw_nb[CG_MAX_LEVELS];
     int raw_off[CG_MAX_LEVELS];

@@ -15,6 +15,7 @@
 #define CG_MAX_SUN_STEPS 64
 #define CG_BRICK 8           // splat brick edge (voxels)
 #define CG_FUSED_MIPS 3      // levels produced inside the splat kernel
+#define CG_QUAD_BASE 2       // first level with density quads
 #define CG_SPLAT_CHUNK 256   // boards staged in shared memory per pass
 
 // ---- programmatic dependent launch: a kernel launched with
@@ -85,6 +86,17 @@ struct VolDesc {
     // the bounds-check build)
     long long nvox;
     int occ_total;
+    // density quads of levels quad_base .. L-1 for the exact sun cone (NULL:
+    // none): cell (i, j, k) of level l holds the stored R of texels (i, j),
+    // (i+1, j), (i, j+1), (i+1, j+1) of slice k, 0 outside the level, for
+    // i, j in [-2, N_l] and k in [-2, N_l + 1]: a trilinear sample is two
+    // loads, and a clamped cell index reads zeros outside the box.  Cells are
+    // four floats (RGBA32F) or four bf16 (BF16_FP16: the bits the level
+    // stores).  Level l starts at cell quad_off[l], x fastest, rows and slices
+    // of quad_p[l] = N_l + 3 cells.
+    void* quad;
+    int quad_base, quad_total;
+    int quad_off[CG_MAX_LEVELS], quad_p[CG_MAX_LEVELS];
 };
 
 // Hash-noise lattice values tabulated per octave over the world box: octave
@@ -129,18 +141,31 @@ struct TraceParams {
 };
 
 // Sun-cone schedule.  The cone's heights and radii do not depend on the
-// volume, so they are computed once per launch on the host (FP64) and read
-// from the kernel parameters: step i samples at v + h[i] * s with lod l0[i] +
-// frac[i] and weight w[i] (r_i * voxel_world for the transmittance cone,
-// i / (steps * downScaling) for the reference cone).
+// volume, so they are computed once per launch on the host (FP64): step i
+// samples at v + h * s with lod l0 + frac and weight w (r_i * voxel_world for
+// the transmittance cone, i / (steps * downScaling) for the reference cone).
+// The quad fields describe levels l0 and l1 = min(l0 + 1, L - 1) in the density
+// quads (sc = N_l / D, first cell, row length); set when `quads` is.
+struct __align__(16) ConeStep {
+    float h, w, frac;
+    int l0;
+    float sc0;
+    int off0, p0;
+    float sc1;
+    int off1, p1;
+    int pad[2];
+};
 struct ConeSchedule {
     int steps;
     int mode;         // 0 transmittance (border 0), 1 reference (clamp to edge)
     float edge;       // break when a sample lies further than this outside the box
-    float h[CG_MAX_SUN_STEPS];
-    float w[CG_MAX_SUN_STEPS];
-    float frac[CG_MAX_SUN_STEPS];
-    unsigned char l0[CG_MAX_SUN_STEPS];
+    // transmittance cones whose every level has density quads sample those;
+    // a sample further than `reach` outside the box then reads exactly 0.  An
+    // odd number of steps is followed by one of weight 0 (they go in pairs)
+    int quads;
+    float reach;
+    int pad[3];
+    ConeStep st[CG_MAX_SUN_STEPS];
 };
 
 // Per-board device arrays (SoA).

@@ -244,7 +244,7 @@ __device__ bool compat_fragment(const VolDesc& vd, const ConeSchedule& cs, const
         const float vx = D * ((px + bx * r * sc - vd.wmin[0]) / vd.range[0]);
         const float vy = D * ((py + by * r * sc - vd.wmin[1]) / vd.range[1]);
         const float vz = D * ((pz + bz * r * sc - vd.wmin[2]) / vd.range[2]);
-        const float ind = cgs::sun_cone<FMT>(vd, cs, vx, vy, vz, P.sun[0], P.sun[1], P.sun[2]);
+        const float ind = cgs::cone_reference<FMT>(vd, cs, vx, vy, vz, P.sun[0], P.sun[1], P.sun[2]);
         if (P.do_noise) {
             o.x *= ind;
             o.y *= ind;

@@ -292,9 +292,10 @@ __device__ __forceinline__ void write_rgb(const float* alpha, float4* dst, const
 }
 
 template <int FMT>
-__global__ void __launch_bounds__(128) k_shade_exact(VolDesc vd, CamDesc cam, TraceParams tp,
-                                                     ConeSchedule cs, SampleBuf sb, int regions,
-                                                     int tiles_x, float4* out) {
+__global__ void __launch_bounds__(128)
+    k_shade_exact(const __grid_constant__ VolDesc vd, const __grid_constant__ CamDesc cam,
+                  const __grid_constant__ TraceParams tp, const __grid_constant__ ConeSchedule cs,
+                  SampleBuf sb, int regions, int tiles_x, float4* out) {
     const int region = blockIdx.x * 4 + (threadIdx.x >> 5);
     if (region >= regions) return;
     const int lane = threadIdx.x & 31;

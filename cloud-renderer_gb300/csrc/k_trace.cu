@@ -51,9 +51,10 @@ __device__ __forceinline__ void bump(unsigned long long* stats, int i, unsigned 
 }
 
 template <int FMT, bool STATS>
-__global__ void __launch_bounds__(256) k_trace_fused(VolDesc vd, CamDesc cam, TraceParams tp,
-                                                     ConeSchedule cs, float4* out,
-                                                     unsigned long long* stats) {
+__global__ void __launch_bounds__(256)
+    k_trace_fused(const __grid_constant__ VolDesc vd, const __grid_constant__ CamDesc cam,
+                  const __grid_constant__ TraceParams tp, const __grid_constant__ ConeSchedule cs,
+                  float4* out, unsigned long long* stats) {
     int px, py;
     tile_pixel(px, py);
     if (px >= cam.W || py >= cam.H) return;
@@ -115,8 +116,8 @@ __global__ void __launch_bounds__(256) k_trace_fused(VolDesc vd, CamDesc cam, Tr
 template <int FMT>
 __device__ __forceinline__ float quad_split_ref(const VolDesc& vd, const ConeSchedule& cs, int i,
                                                 float x, float y, float z) {
-    return cgs::quad_split<FMT, true, false, false>(vd, x, y, z, cs.l0[i], cs.frac[i]).y *
-           cs.w[i];
+    return cgs::quad_split<FMT, true, false, false>(vd, x, y, z, cs.st[i].l0, cs.st[i].frac).y *
+           cs.st[i].w;
 }
 
 // One lane's share of a sun cone traced by the whole warp: the weighted
@@ -133,13 +134,23 @@ __device__ __forceinline__ float cone_part(const VolDesc& vd, const ConeSchedule
     for (int r = 0; r < CG_MAX_SUN_STEPS / 32; ++r) {
         const int i = lane + 32 * r;
         if (i >= cs.steps) break;
-        const float h = cs.h[i];
+        const float h = cs.st[i].h;
         const float x = vx + h * sx, y = vy + h * sy, z = vz + h * sz;
-        if (cs.mode == 1) {
+        if (cs.quads) {
+            const ConeStep& s = cs.st[i];
+            float a = cgs::tri_quads<FMT>(vd, s.sc0, s.off0, s.p0, x, y, z);
+            if (s.frac > 0.f) {
+                const float b = cgs::tri_quads<FMT>(vd, s.sc1, s.off1, s.p1, x, y, z);
+                a = a + s.frac * (b - a);
+            }
+            part += a * s.w;
+        } else if (cs.mode == 1) {
             part += quad_split_ref<FMT>(vd, cs, i, x, y, z);
         } else if (!(x < -E || y < -E || z < -E || x > D + E || y > D + E || z > D + E)) {
-            part += cgs::quad_split<FMT, false, true, true>(vd, x, y, z, cs.l0[i], cs.frac[i]).x *
-                    cs.w[i];
+            part += cgs::quad_split<FMT, false, true, true>(vd, x, y, z, cs.st[i].l0,
+                                                            cs.st[i].frac)
+                        .x *
+                    cs.st[i].w;
         }
     }
     return part;
@@ -154,8 +165,16 @@ __device__ __forceinline__ float cone_part(const VolDesc& vd, const ConeSchedule
 // order are k_trace_fused's; only the order in which a cooperative cone's
 // terms are added differs.
 template <int FMT>
-__global__ void __launch_bounds__(256) k_trace_coop(VolDesc vd, CamDesc cam, TraceParams tp,
-                                                    ConeSchedule cs, float4* out, int coop_max) {
+__global__ void __launch_bounds__(256)
+    k_trace_coop(const __grid_constant__ VolDesc vd, const __grid_constant__ CamDesc cam,
+                 const __grid_constant__ TraceParams tp,
+                 const __grid_constant__ ConeSchedule cone, float4* out, int coop_max) {
+    // the schedule in shared memory: a cooperative cone's lanes read
+    // different steps, which the constant bank would serve one by one
+    __shared__ ConeSchedule cs;
+    for (int i = threadIdx.x; i < (int)(sizeof(ConeSchedule) / 16); i += blockDim.x)
+        reinterpret_cast<uint4*>(&cs)[i] = reinterpret_cast<const uint4*>(&cone)[i];
+    __syncthreads();
     int px, py;
     tile_pixel(px, py);
     const int lane = threadIdx.x & 31;
@@ -240,19 +259,26 @@ __global__ void __launch_bounds__(256) k_trace_coop(VolDesc vd, CamDesc cam, Tra
 }
 
 template <int FMT>
-__global__ void k_trace_cones(VolDesc vd, TraceParams tp, ConeSchedule cs, const float* pos,
-                              int n, float* out) {
+__global__ void k_trace_cones(const __grid_constant__ VolDesc vd,
+                              const __grid_constant__ TraceParams tp,
+                              const __grid_constant__ ConeSchedule cs, const float* pos, int n,
+                              float* out) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    out[i] = cgs::sun_cone<FMT>(vd, cs, pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], tp.sun[0],
-                                tp.sun[1], tp.sun[2]);
+    const float x = pos[3 * i], y = pos[3 * i + 1], z = pos[3 * i + 2];
+    // a caller's position may be a NaN, which the pyramid's own walk carries
+    // through only where it samples something
+    if (cs.quads && !isnan(x + y + z))
+        out[i] = cgs::cone_quads<FMT>(vd, cs, x, y, z, tp.sun[0], tp.sun[1], tp.sun[2]);
+    else
+        out[i] = cgs::cone_general<FMT>(vd, cs, x, y, z, tp.sun[0], tp.sun[1], tp.sun[2]);
 }
 
 }  // namespace
 
 // Cone schedule in FP64 on the host (see ConeSchedule).
 ConeSchedule make_cone_schedule(const VolDesc& vd, const TraceParams& tp) {
-    ConeSchedule cs;
+    ConeSchedule cs{};
     cs.steps = tp.sun_steps;
     cs.mode = tp.cone_mode;
     cs.edge = (float)vd.D / (float)vd.dims[vd.L - 1];
@@ -276,11 +302,35 @@ ConeSchedule make_cone_schedule(const VolDesc& vd, const TraceParams& tp) {
         if (!(lod > 0.0)) lod = 0.0;
         if (lod > maxl) lod = maxl;
         int l0 = (int)floor(lod);
-        cs.h[i] = (float)h;
-        cs.w[i] = (float)w;
-        cs.l0[i] = (unsigned char)l0;
-        cs.frac[i] = (float)(lod - (double)l0);
+        cs.st[i].h = (float)h;
+        cs.st[i].w = (float)w;
+        cs.st[i].l0 = l0;
+        cs.st[i].frac = (float)(lod - (double)l0);
         h += r;
+    }
+    // density quads: every level the cone reads must have them.  reach: half a
+    // texel of the coarsest level read, plus a voxel for the rounding of the
+    // distance to the box
+    bool quads = tp.cone_mode != 1 && vd.quad != nullptr && tp.sun_steps > 0;
+    for (int i = 0; i < cs.steps && quads; ++i) quads = cs.st[i].l0 >= vd.quad_base;
+    cs.quads = quads ? 1 : 0;
+    if (quads) {
+        for (int i = 0; i < cs.steps; ++i) {
+            ConeStep& s = cs.st[i];
+            const int l1 = s.l0 + 1 < vd.L ? s.l0 + 1 : vd.L - 1;
+            s.sc0 = vd.lsc[s.l0];
+            s.off0 = vd.quad_off[s.l0];
+            s.p0 = vd.quad_p[s.l0];
+            s.sc1 = vd.lsc[l1];
+            s.off1 = vd.quad_off[l1];
+            s.p1 = vd.quad_p[l1];
+            const float half = 0.5f * (float)vd.D / (float)vd.dims[s.frac > 0.f ? l1 : s.l0];
+            if (half + 1.f > cs.reach) cs.reach = half + 1.f;
+        }
+        if (cs.steps & 1) {
+            cs.st[cs.steps] = cs.st[cs.steps - 1];
+            cs.st[cs.steps].w = 0.f;
+        }
     }
     return cs;
 }

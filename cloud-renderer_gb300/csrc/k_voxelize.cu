@@ -410,14 +410,36 @@ __device__ __forceinline__ void store_voxel(const VolDesc& vd, void* pyr, int l,
     size_t idx = (size_t)vd.offs[l] + ((size_t)z * N + y) * N + x;
     if (!CG_IN_BOUNDS(idx, vd.nvox)) return;
     __half2 h;
+    unsigned short r16 = 0;  // the density bits of a half-precision level
     if (vd.fmt == 0) {
         reinterpret_cast<float4*>(pyr)[idx] = v;
         h = __floats2half2_rn(v.x, v.y);
     } else {
         const uint32_t w = pack_bf16_fp16(v.x, v.y);
         reinterpret_cast<uint32_t*>(pyr)[idx] = w;
+        r16 = (unsigned short)(w & 0xFFFFu);
         h = __halves2half2(__float2half_rn(__uint_as_float(w << 16)),
                            __ushort_as_half((unsigned short)(w >> 16)));
+    }
+    // the texel's component of the four density quads that hold it
+    if (l >= vd.quad_base) {
+        const int p = vd.quad_p[l];
+        const int at = vd.quad_off[l] + ((z + 2) * p + y + 2) * p + x + 2;
+        if (CG_IN_BOUNDS(at, vd.quad_total) && CG_IN_BOUNDS(at - p - 1, vd.quad_total)) {
+            if (vd.fmt == 0) {
+                float* q = reinterpret_cast<float*>(vd.quad) + 4 * (size_t)at;
+                q[0] = v.x;
+                q[-4 + 1] = v.x;
+                q[-4 * p + 2] = v.x;
+                q[-4 * (p + 1) + 3] = v.x;
+            } else {
+                unsigned short* q = reinterpret_cast<unsigned short*>(vd.quad) + 4 * (size_t)at;
+                q[0] = r16;
+                q[-4 + 1] = r16;
+                q[-4 * p + 2] = r16;
+                q[-4 * (p + 1) + 3] = r16;
+            }
+        }
     }
     // the half2 texture copy holds exactly what the level stores (the same
     // conversion as the copy pass of k_textures.cu)
