@@ -442,6 +442,7 @@ extern "C" cg_status cg_volume_create(cg_context* ctx, int dimension, float boun
     if (e == cudaSuccess) e = v->dq.ensure(n0 * 4);
     if (e == cudaSuccess) e = v->mask.ensure(n0);
     if (e == cudaSuccess) e = v->scratch.ensure(64);
+    if (e == cudaSuccess) e = cudaMemsetAsync(v->scratch.p, 0, 64, ctx->stream);
     // raw 4^3-cell grids (written by the splat) followed by the dilated brick
     // grids (at most as many bytes as the raw ones: bricks are >= 4 texels)
     int raw_total = 0;
@@ -467,8 +468,8 @@ extern "C" cg_status cg_volume_create(cg_context* ctx, int dimension, float boun
         const size_t bytes = cells * (format == CG_FORMAT_RGBA32F ? 16 : 8);
         if (e == cudaSuccess) e = v->quads.ensure(bytes);
         if (e == cudaSuccess) e = cudaMemsetAsync(v->quads.p, 0, bytes, ctx->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     set_occ_layout(v, 4);  // the autotuner's pick on the batching and 1080p workloads
     // + the level-0 occupied box (6 ints) after the grids, 16-byte aligned
     if (e == cudaSuccess) e = v->occ.ensure(occ_box_offset(raw_total) + 32);
@@ -886,13 +887,10 @@ extern "C" cg_status cg_voxelize(cg_volume* v, const cg_sun* sun, void* stream) 
     CG_CUDA(cudaEventRecord(ctx->join_ev, sd));
     // remaining mips (glGenerateMipmap, VoxelizeShader.cpp:105)
     {
-        int l = fused;
-        for (; l + 1 < v->L; ++l) {
-            const long long np = v->dims[l + 1];
-            if (np * np * np <= CG_MIP_TAIL_MAX) break;
-            CG_LAUNCH(ctx, launch_mip_level(vd, v->pyr.p, l, s));
+        for (int l = fused; l + 1 < v->L; l += 3) {
+            CG_LAUNCH(ctx, launch_mip_rest(vd, v->pyr.p, l, v->scratch.as<unsigned>() + 8, s));
+            if (v->dims[l] <= CG_MIP_LAST) break;  // that launch made every level left
         }
-        if (l + 1 < v->L) CG_LAUNCH(ctx, launch_mip_tail(vd, v->pyr.p, l, s));
     }
     CG_CUDA(cudaStreamWaitEvent(s, ctx->join_ev, 0));
     stage_mark(ctx, s, "mips");

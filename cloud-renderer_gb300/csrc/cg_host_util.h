@@ -169,7 +169,7 @@ struct cg_volume {
     bool voxelized = false;
     SunFrame frame{};
     float sun_dir[3] = {0, 1, 0};
-    DevBuf scratch;  // small scalars (active voxel count)
+    DevBuf scratch;  // small scalars (word 0-1: active voxel count, 8: mip ticket)
     // density quads of levels quad_base .. L-1 (VolDesc), zeroed at creation;
     // every voxel store of those levels also writes its four cells
     DevBuf quads;

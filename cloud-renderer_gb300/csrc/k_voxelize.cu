@@ -669,12 +669,104 @@ __global__ void __launch_bounds__(64) k_splat(BoardsDev b, Bins bins, const uint
 }
 
 // Dilated occupancy: occ[l][c] = 1 when a raw 4^3 cell of level l inside
-// brick c (B = 1 << occ_shift texels) or one of its 26 neighbours is set; one
-// thread per brick of every level.  The occupied level-0 bricks also grow the
-// level-0 box (box[0..2] = D - lo, box[3..5] = hi, atomic maxima from zero).
-__global__ void __launch_bounds__(256) k_occ_dilate(VolDesc vd, OccRaw raw, uint8_t* occ,
-                                                    int total, int* box) {
+// brick c (B = 1 << occ_shift texels) or one of its 26 neighbours is set.  The
+// occupied level-0 bricks also grow the level-0 box (box[0..2] = D - lo,
+// box[3..5] = hi, atomic maxima from zero).
+
+// Block maxima of the box terms m (warp reductions, then warp 0), one atomic
+// per value per block.
+__device__ __forceinline__ void grow_box(unsigned (&m)[6], int* box) {
     __shared__ unsigned s_box[8][6];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+    for (int a = 0; a < 6; ++a) m[a] = __reduce_max_sync(0xffffffffu, m[a]);
+    if (lane == 0)
+#pragma unroll
+        for (int a = 0; a < 6; ++a) s_box[w][a] = m[a];
+    __syncthreads();
+    if (w == 0) {
+        const int nw = blockDim.x >> 5;
+#pragma unroll
+        for (int a = 0; a < 6; ++a) {
+            const unsigned v = __reduce_max_sync(0xffffffffu, lane < nw ? s_box[lane][a] : 0u);
+            if (lane == 0 && v > 0u) atomicMax(box + a, (int)v);
+        }
+    }
+}
+
+// Bricks of the raw cells' own size (the default): a warp takes 32 bricks along
+// x and a run of slices along z (dilate_run), keeps the OR of the 3 x 3 cells of the last
+// three slices in registers and takes the x neighbours from the neighbouring
+// lanes: 3.75 byte loads per brick in runs of eight instead of up to 27.  Small
+// grids take shorter runs, for more warps.
+__host__ __device__ __forceinline__ int dilate_run(int nb) {
+    return nb >= 128 ? 8 : (nb >= 32 ? nb / 16 : 1);
+}
+struct DilateUnits {
+    int first[CG_MAX_LEVELS + 1];  // first warp unit of each level
+};
+
+__global__ void __launch_bounds__(256) k_occ_dilate(const __grid_constant__ VolDesc vd,
+                                                    const __grid_constant__ OccRaw raw,
+                                                    const __grid_constant__ DilateUnits units,
+                                                    uint8_t* occ, int* box) {
+    const int lane = threadIdx.x & 31;
+    const int unit = blockIdx.x * 8 + (threadIdx.x >> 5);
+    unsigned m[6] = {0u, 0u, 0u, 0u, 0u, 0u};  // this thread's box terms (0 = none)
+    if (unit < units.first[vd.L]) {
+        int l = 0;
+        while (unit >= units.first[l + 1]) ++l;
+        const int nb = vd.occ_nb[l], nx = (nb + 31) / 32;
+        const int r = unit - units.first[l];
+        const int x = (r % nx) * 32 + lane, y = (r / nx) % nb;
+        const int run = dilate_run(nb), z0 = (r / (nx * nb)) * run;
+        const uint8_t* g = raw.raw + raw.off[l];
+        // OR of the nine cells around (x, y) in slice z, 0 outside the grid
+        auto slice = [&](int z) -> unsigned {
+            unsigned v = 0u, e = 0u;
+            const int xe = lane == 0 ? x - 1 : x + 1;  // the end lanes' outer neighbour
+            const bool edge = (lane == 0 || lane == 31) && xe >= 0 && xe < nb;
+            if (z >= 0 && z < nb) {
+#pragma unroll
+                for (int dy = -1; dy <= 1; ++dy) {
+                    const int yy = y + dy;
+                    if (yy < 0 || yy >= nb) continue;
+                    const uint8_t* row = g + ((size_t)z * nb + yy) * nb;
+                    if (x < nb) v |= row[x];
+                    if (edge) e |= row[xe];
+                }
+            }
+            const unsigned up = __shfl_up_sync(0xffffffffu, v, 1);
+            const unsigned dn = __shfl_down_sync(0xffffffffu, v, 1);
+            return v | e | (lane > 0 ? up : 0u) | (lane < 31 ? dn : 0u);
+        };
+        unsigned a = slice(z0 - 1), b = slice(z0);
+        const int z1 = min(z0 + run, nb);
+        for (int z = z0; z < z1; ++z) {
+            const unsigned c = slice(z + 1);
+            const bool any = (a | b | c) != 0u;
+            if (x < nb) {
+                occ[vd.occ_off[l] + ((size_t)z * nb + y) * nb + x] = any ? 1 : 0;
+                if (any && l == 0) {
+                    const int B = 1 << vd.occ_shift, D = vd.D;
+                    const int p[3] = {x, y, z};
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) {
+                        m[k] = max(m[k], (unsigned)(D - p[k] * B));
+                        m[3 + k] = max(m[3 + k], (unsigned)min(D, (p[k] + 1) * B));
+                    }
+                }
+            }
+            a = b;
+            b = c;
+        }
+    }
+    grow_box(m, box);
+}
+
+// Larger bricks (8 or 16 texels: 1 << k raw cells per edge), one thread each.
+__global__ void __launch_bounds__(256) k_occ_dilate_wide(VolDesc vd, OccRaw raw, uint8_t* occ,
+                                                         int total, int* box) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     unsigned m[6] = {0u, 0u, 0u, 0u, 0u, 0u};  // this brick's box terms (0 = none)
     if (i < total) {
@@ -703,56 +795,90 @@ __global__ void __launch_bounds__(256) k_occ_dilate(VolDesc vd, OccRaw raw, uint
             }
         }
     }
-    // the occupied level-0 box: block maxima (warp reductions, then warp 0),
-    // one atomic per value per block
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-    for (int a = 0; a < 6; ++a) m[a] = __reduce_max_sync(0xffffffffu, m[a]);
-    if (lane == 0)
-#pragma unroll
-        for (int a = 0; a < 6; ++a) s_box[w][a] = m[a];
-    __syncthreads();
-    if (w == 0) {
-        const int nw = blockDim.x >> 5;
-#pragma unroll
-        for (int a = 0; a < 6; ++a) {
-            const unsigned v = __reduce_max_sync(0xffffffffu, lane < nw ? s_box[lane][a] : 0u);
-            if (lane == 0 && v > 0u) atomicMax(box + a, (int)v);
-        }
-    }
+    grow_box(m, box);
 }
 
 // Parent (x, y, z) of level l + 1 as the mean of its 2x2x2 children at level
 // l (clamped at odd edges).
-__device__ __forceinline__ void mip_parent(const VolDesc& vd, void* pyr, int l, int x, int y,
+__device__ __forceinline__ float4 mip_mean(const VolDesc& vd, const void* pyr, int l, int x, int y,
                                            int z) {
     const int Nc = vd.dims[l];
     int cx0 = min(2 * x, Nc - 1), cx1 = min(2 * x + 1, Nc - 1);
     int cy0 = min(2 * y, Nc - 1), cy1 = min(2 * y + 1, Nc - 1);
     int cz0 = min(2 * z, Nc - 1), cz1 = min(2 * z + 1, Nc - 1);
-    float4 m = box8(load_voxel(vd, pyr, l, cx0, cy0, cz0), load_voxel(vd, pyr, l, cx1, cy0, cz0),
-                    load_voxel(vd, pyr, l, cx0, cy1, cz0), load_voxel(vd, pyr, l, cx1, cy1, cz0),
-                    load_voxel(vd, pyr, l, cx0, cy0, cz1), load_voxel(vd, pyr, l, cx1, cy0, cz1),
-                    load_voxel(vd, pyr, l, cx0, cy1, cz1), load_voxel(vd, pyr, l, cx1, cy1, cz1));
-    store_voxel(vd, pyr, l + 1, x, y, z, m);
+    return box8(load_voxel(vd, pyr, l, cx0, cy0, cz0), load_voxel(vd, pyr, l, cx1, cy0, cz0),
+                load_voxel(vd, pyr, l, cx0, cy1, cz0), load_voxel(vd, pyr, l, cx1, cy1, cz0),
+                load_voxel(vd, pyr, l, cx0, cy0, cz1), load_voxel(vd, pyr, l, cx1, cy0, cz1),
+                load_voxel(vd, pyr, l, cx0, cy1, cz1), load_voxel(vd, pyr, l, cx1, cy1, cz1));
+}
+__device__ __forceinline__ void mip_parent(const VolDesc& vd, void* pyr, int l, int x, int y,
+                                           int z) {
+    store_voxel(vd, pyr, l + 1, x, y, z, mip_mean(vd, pyr, l, x, y, z));
 }
 
-// Generic 2x2x2 reduction from level l to l+1 (one thread per parent).
-__global__ void k_mip_level(VolDesc vd, void* pyr, int l) {
-    const int Np = vd.dims[l + 1];
-    const long long total = (long long)Np * Np * Np;
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= total) return;
-    mip_parent(vd, pyr, l, (int)(i % Np), (int)((i / Np) % Np), (int)(i / ((long long)Np * Np)));
+// Levels l0+1 .. L-1.  A CTA reduces one 8^3 block of level l0 to its 4^3, 2^3
+// and 1^3 texels of the next three levels in shared memory, so the largest
+// level is read by the whole GPU; with `finish`, the last CTA to finish (a
+// ticket) reduces what is left, at most 8^3 texels of level l0+3, level after
+// level.  Children are the values the finer level stores (rounded for the
+// half-precision form).  Latency-bound: a single CTA read up to 64^3 texels
+// alone (with the dilation beside it, the voxelize stage after the splat took
+// 17 us at 256^3 and 84 us at 512^3 BF16, now 11 and 23 us).
+__device__ __forceinline__ float4 as_stored(const VolDesc& vd, float4 v) {
+    return vd.fmt == 0 ? v : unpack_bf16_fp16(pack_bf16_fp16(v.x, v.y));
 }
 
-// The small levels l0+1 .. L-1 in one CTA, level after level (a block
-// barrier makes each level's stores visible to the next level's loads).
-__global__ void __launch_bounds__(1024) k_mip_tail(VolDesc vd, void* pyr, int l0) {
-    for (int l = l0; l + 1 < vd.L; ++l) {
+__global__ void __launch_bounds__(64) k_mip_rest(VolDesc vd, void* pyr, int l0, int nb,
+                                                 bool finish, unsigned* ticket) {
+    __shared__ float4 t1[64], t2[8];
+    __shared__ bool last;
+    const int tid = threadIdx.x;
+    const int bx = blockIdx.x % nb, by = (blockIdx.x / nb) % nb, bz = blockIdx.x / (nb * nb);
+    // level l0+1: parent (4 bx + px, ...), present while it lies in its level
+    {
+        const int px = tid & 3, py = (tid >> 2) & 3, pz = tid >> 4;
+        const int x = 4 * bx + px, y = 4 * by + py, z = 4 * bz + pz, N = vd.dims[l0 + 1];
+        float4 m = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (x < N && y < N && z < N) {
+            m = mip_mean(vd, pyr, l0, x, y, z);
+            store_voxel(vd, pyr, l0 + 1, x, y, z, m);
+        }
+        t1[tid] = as_stored(vd, m);
+    }
+    __syncthreads();
+    if (l0 + 2 < vd.L && tid < 8) {
+        const int px = tid & 1, py = (tid >> 1) & 1, pz = tid >> 2;
+        const int x = 2 * bx + px, y = 2 * by + py, z = 2 * bz + pz, N = vd.dims[l0 + 2];
+        float4 m = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (x < N && y < N && z < N) {
+#define T4(a, b2, c) t1[((2 * pz + (c)) * 4 + (2 * py + (b2))) * 4 + (2 * px + (a))]
+            m = box8(T4(0, 0, 0), T4(1, 0, 0), T4(0, 1, 0), T4(1, 1, 0), T4(0, 0, 1), T4(1, 0, 1),
+                     T4(0, 1, 1), T4(1, 1, 1));
+#undef T4
+            store_voxel(vd, pyr, l0 + 2, x, y, z, m);
+        }
+        t2[tid] = as_stored(vd, m);
+    }
+    __syncthreads();
+    if (l0 + 3 < vd.L && tid == 0) {
+        const int N = vd.dims[l0 + 3];
+        if (bx < N && by < N && bz < N)
+            store_voxel(vd, pyr, l0 + 3, bx, by, bz,
+                        box8(t2[0], t2[1], t2[2], t2[3], t2[4], t2[5], t2[6], t2[7]));
+    }
+    if (!finish || l0 + 4 >= vd.L) return;
+    // the last CTA: every other's stores are visible once its ticket is
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    if (tid == 0) *ticket = 0u;  // for the next launch
+    for (int l = l0 + 3; l + 1 < vd.L; ++l) {
         const int Np = vd.dims[l + 1];
         const int total = Np * Np * Np;
-        for (int i = threadIdx.x; i < total; i += blockDim.x)
+        for (int i = tid; i < total; i += blockDim.x)
             mip_parent(vd, pyr, l, i % Np, (i / Np) % Np, i / (Np * Np));
         __syncthreads();
     }
@@ -841,21 +967,26 @@ cudaError_t launch_splat(const BoardsDev& b, Bins bins, const uint8_t* mask, Vol
 }
 
 cudaError_t launch_occ_dilate(VolDesc vd, OccRaw raw, uint8_t* occ, int total, cudaStream_t st) {
-    k_occ_dilate<<<(total + 255) / 256, 256, 0, st>>>(vd, raw, occ, total,
-                                                      const_cast<int*>(vd.occ_box));
+    int* box = const_cast<int*>(vd.occ_box);
+    if (vd.occ_shift == 2) {
+        DilateUnits u;
+        int n = 0;
+        for (int l = 0; l < CG_MAX_LEVELS; ++l) {
+            u.first[l] = n;
+            const int nb = vd.occ_nb[l];
+            if (l < vd.L) n += (nb + 31) / 32 * nb * ((nb + dilate_run(nb) - 1) / dilate_run(nb));
+        }
+        u.first[CG_MAX_LEVELS] = n;
+        k_occ_dilate<<<(n + 7) / 8, 256, 0, st>>>(vd, raw, u, occ, box);
+    } else {
+        k_occ_dilate_wide<<<(total + 255) / 256, 256, 0, st>>>(vd, raw, occ, total, box);
+    }
     return cudaGetLastError();
 }
 
-cudaError_t launch_mip_level(VolDesc vd, void* pyr, int l, cudaStream_t st) {
-    long long np = (long long)vd.dims[l + 1];
-    long long total = np * np * np;
-    int blocks = (int)((total + 255) / 256);
-    k_mip_level<<<blocks, 256, 0, st>>>(vd, pyr, l);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_mip_tail(VolDesc vd, void* pyr, int l0, cudaStream_t st) {
-    k_mip_tail<<<1, 1024, 0, st>>>(vd, pyr, l0);
+cudaError_t launch_mip_rest(VolDesc vd, void* pyr, int l0, unsigned* ticket, cudaStream_t st) {
+    const int nb = (vd.dims[l0] + 7) / 8;
+    k_mip_rest<<<nb * nb * nb, 64, 0, st>>>(vd, pyr, l0, nb, vd.dims[l0] <= CG_MIP_LAST, ticket);
     return cudaGetLastError();
 }
 
