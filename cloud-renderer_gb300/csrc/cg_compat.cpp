@@ -220,7 +220,7 @@ extern "C" cg_status cg_render_compat(cg_context* ctx, const cg_volume* v, const
     CG_CUDA(ctx->compat_tiles.ensure((cnt_words + off_words + cnt_words) * 4 + 16));
     CG_CUDA(ctx->compat_total.ensure(16));
     Bins bins{};
-    bins.nbricks = ntiles;
+    bins.nbins = ntiles;
     bins.count = ctx->compat_tiles.as<uint32_t>();
     bins.offset = bins.count + cnt_words;
     bins.cursor = bins.offset + off_words;

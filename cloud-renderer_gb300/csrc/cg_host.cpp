@@ -476,9 +476,12 @@ extern "C" cg_status cg_volume_create(cg_context* ctx, int dimension, float boun
     const int nb = (dimension + CG_BRICK - 1) / CG_BRICK;
     v->bins.nbx = v->bins.nby = v->bins.nbz = nb;
     v->bins.nbricks = nb * nb * nb;
-    if (e == cudaSuccess) e = v->bcount.ensure((size_t)v->bins.nbricks * 4);
-    if (e == cudaSuccess) e = v->boff.ensure(((size_t)v->bins.nbricks + 1) * 4);
-    if (e == cudaSuccess) e = v->bcursor.ensure((size_t)v->bins.nbricks * 4);
+    v->bins.bar = splat_bar(dimension);
+    v->bins.nbarz = (dimension + v->bins.bar - 1) / v->bins.bar;
+    v->bins.nbins = nb * nb * v->bins.nbarz;
+    if (e == cudaSuccess) e = v->bcount.ensure((size_t)v->bins.nbins * 4);
+    if (e == cudaSuccess) e = v->boff.ensure(((size_t)v->bins.nbins + 1) * 4);
+    if (e == cudaSuccess) e = v->bcursor.ensure((size_t)v->bins.nbins * 4);
     // every brick starts dirty: the pyramid's memory is uninitialised
     if (e == cudaSuccess) e = v->bdirty.ensure((size_t)v->bins.nbricks);
     if (e == cudaSuccess) e = cudaMemset(v->bdirty.p, 1, (size_t)v->bins.nbricks);
@@ -570,7 +573,7 @@ extern "C" cg_status cg_volume_set_billboards(cg_volume* v, const float* positio
     uint64_t* thr = reinterpret_cast<uint64_t*>(st + o_thr);
     uint32_t* dqv = reinterpret_cast<uint32_t*>(st + o_dq);
     uint8_t* cul = reinterpret_cast<uint8_t*>(st + o_cul);
-    const int D = v->D;
+    const int D = v->D, bar = v->bins.bar;
     size_t pairs = 0;
     for (size_t b = 0; b < n; ++b) {
         float r = scales[b] * fluffiness;
@@ -612,14 +615,14 @@ extern "C" cg_status cg_volume_set_billboards(cg_volume* v, const float* positio
                 if (!axis_range_host(q[a], rq, D, lo[a], hi[a])) cull = true;
         cul[b] = cull ? 1 : 0;
         if (!cull) {
-            size_t nbz = (size_t)(hi[2] / CG_BRICK - lo[2] / CG_BRICK + 1);
+            size_t nbz = (size_t)(hi[2] / bar - lo[2] / bar + 1);
             size_t nby = (size_t)(hi[1] / CG_BRICK - lo[1] / CG_BRICK + 1);
             size_t nbx = (size_t)(hi[0] / CG_BRICK - lo[0] / CG_BRICK + 1);
-            pairs += nbx * nby * nbz;
+            pairs += nbx * nby * nbz;  // the bars its box meets
         }
     }
     CG_CHECK(pairs < (size_t)0xFFFFFFFFu, CG_ERR_OUT_OF_RANGE,
-             "cg_volume_set_billboards: %zu board-brick pairs exceed 2^32", pairs);
+             "cg_volume_set_billboards: %zu board-bar pairs exceed 2^32", pairs);
     // the device records mirror the staging layout: one copy uploads them all
     CG_CUDA(v->boards.ensure(total));
     char* dev = v->boards.as<char>();
@@ -857,7 +860,7 @@ extern "C" cg_status cg_voxelize(cg_volume* v, const cg_sun* sun, void* stream) 
     }
     {
         NvtxRange r("voxelize.bins");
-        CG_CUDA(cudaMemsetAsync(bins.count, 0, (size_t)bins.nbricks * 4, s));
+        CG_CUDA(cudaMemsetAsync(bins.count, 0, (size_t)bins.nbins * 4, s));
         // raw cells, brick grids (rewritten by the dilation) and the occupied box
         CG_CUDA(cudaMemsetAsync(v->occ.p, 0, occ_box_offset(v->raw_total) + 6 * sizeof(int), s));
         // brick bins
@@ -882,6 +885,7 @@ extern "C" cg_status cg_voxelize(cg_volume* v, const cg_sun* sun, void* stream) 
     // remaining mips are independent: the dilation runs on the side stream
     CG_CUDA(cudaEventRecord(ctx->fork_ev, s));
     CG_CUDA(cudaStreamWaitEvent(sd, ctx->fork_ev, 0));
+    CG_LAUNCH(ctx, launch_occ_coarse(bins, raw_of(v), v->L, sd));
     CG_LAUNCH(ctx, launch_occ_dilate(vd, raw_of(v), v->occ.as<uint8_t>() + v->raw_total,
                                      v->occ_total, sd));
     CG_CUDA(cudaEventRecord(ctx->join_ev, sd));

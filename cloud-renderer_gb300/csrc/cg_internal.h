@@ -16,7 +16,7 @@
 #define CG_BRICK 8           // splat brick edge (voxels)
 #define CG_FUSED_MIPS 3      // levels produced inside the splat kernel
 #define CG_QUAD_BASE 2       // first level with density quads
-#define CG_SPLAT_CHUNK 256   // boards staged in shared memory per pass
+#define CG_SPLAT_CHUNK 64    // boards staged in shared memory per pass
 
 // ---- programmatic dependent launch: a kernel launched with
 // launch_dependent() may start while the kernel before it on the stream is
@@ -188,9 +188,12 @@ struct OccRaw {
 
 struct Bins {
     int nbx, nby, nbz, nbricks;
-    uint32_t* count;   // nbricks
-    uint32_t* offset;  // nbricks + 1
-    uint32_t* cursor;  // nbricks
+    // the bins: bars of 8 x 8 x bar voxels (bar = 8 or 32; nbarz along z); the
+    // compat render's are pixel tiles
+    int bar, nbarz, nbins;
+    uint32_t* count;   // nbins
+    uint32_t* offset;  // nbins + 1
+    uint32_t* cursor;  // nbins
     uint32_t* list;    // pairs
     // per brick: 1 when its level-0 voxels (and fused levels 1-3) may hold
     // non-zero values from an earlier voxelize; a brick without boards or
@@ -425,6 +428,8 @@ bool sun_frame_for_box(const float position[3], float b0, float b1, const float 
                        int H, SunFrame& fr);
 
 // ---- launchers (return cudaGetLastError of the launch) -------------------
+// Bar height of a volume's splat (k_voxelize.cu).
+int splat_bar(int dimension);
 cudaError_t launch_bin_count(const BoardsDev& b, int D, Bins bins, cudaStream_t st);
 cudaError_t launch_bin_scan(Bins bins, cudaStream_t st);
 cudaError_t launch_bin_fill(const BoardsDev& b, int D, Bins bins, cudaStream_t st);
@@ -445,6 +450,9 @@ cudaError_t launch_splat(const BoardsDev& b, Bins bins, const uint8_t* mask, Vol
 // word, left zero.
 #define CG_MIP_LAST 64
 cudaError_t launch_mip_rest(VolDesc vd, void* pyr, int l0, unsigned* ticket, cudaStream_t st);
+// Raw occupancy of levels 1 .. L-1 from the dirty flags the splat left, unless
+// the splat itself marked them.
+cudaError_t launch_occ_coarse(const Bins& bins, OccRaw raw, int L, cudaStream_t st);
 // Dilated occupancy grids of brick B = 1 << vd.occ_shift from the raw cells.
 // Builds the brick grids from the raw cells and grows the level-0 occupied
 // box (vd.occ_box, zeroed by the caller).

@@ -36,7 +36,7 @@ __device__ __forceinline__ bool axis_range(int q, int rq, int D, int& lo, int& h
     return true;
 }
 
-// ---- brick binning ---------------------------------------------------------
+// ---- bar binning -----------------------------------------------------------
 
 // Distance term along one axis from the board centre q to the nearest voxel
 // centre of the voxel range [lo, hi] (Q20).
@@ -47,9 +47,9 @@ __device__ __forceinline__ long long axis_gap(int q, int lo, int hi) {
 }
 
 // Board bin walk shared by the count and fill passes: one warp per board,
-// lanes over the bricks of its voxel box; a brick is kept only when its
-// nearest voxel centre passes the board's ball test, so no brick without an
-// inside voxel enters the bins (the per-voxel test in k_splat stays exact).
+// lanes over the bars (8 x 8 x bins.bar voxels) of its voxel box; a bar is kept
+// only when its nearest voxel centre passes the board's ball test (the
+// per-voxel test in k_splat stays exact).
 template <bool FILL>
 __device__ __forceinline__ void bin_walk(const BoardsDev& b, int D, Bins& bins) {
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -61,24 +61,25 @@ __device__ __forceinline__ void bin_walk(const BoardsDev& b, int D, Bins& bins) 
     if (!axis_range(q.x, q.w, D, xl, xh) || !axis_range(q.y, q.w, D, yl, yh) ||
         !axis_range(q.z, q.w, D, zl, zh))
         return;
-    const int bx0 = xl / CG_BRICK, by0 = yl / CG_BRICK, bz0 = zl / CG_BRICK;
+    const int bx0 = xl / CG_BRICK, by0 = yl / CG_BRICK, bz0 = zl / bins.bar;
     const int nx = xh / CG_BRICK - bx0 + 1, ny = yh / CG_BRICK - by0 + 1,
-              nz = zh / CG_BRICK - bz0 + 1;
+              nz = zh / bins.bar - bz0 + 1;
     const int total = nx * ny * nz;
     for (int t = lane; t < total; t += 32) {
         const int bx = bx0 + t % nx, by = by0 + (t / nx) % ny, bz = bz0 + t / (nx * ny);
         long long gx = axis_gap(q.x, max(bx * CG_BRICK, xl), min(bx * CG_BRICK + 7, xh));
         long long gy = axis_gap(q.y, max(by * CG_BRICK, yl), min(by * CG_BRICK + 7, yh));
-        long long gz = axis_gap(q.z, max(bz * CG_BRICK, zl), min(bz * CG_BRICK + 7, zh));
+        long long gz = axis_gap(q.z, max(bz * bins.bar, zl),
+                                min(bz * bins.bar + bins.bar - 1, zh));
         unsigned long long d2 = (unsigned long long)(gx * gx) + (unsigned long long)(gy * gy) +
                                 (unsigned long long)(gz * gz);
         if (d2 > thr) continue;
-        const int brick = (bz * bins.nby + by) * bins.nbx + bx;
+        const int bar = (bz * bins.nby + by) * bins.nbx + bx;
         if (FILL) {
-            uint32_t slot = atomicAdd(&bins.cursor[brick], 1u);
+            uint32_t slot = atomicAdd(&bins.cursor[bar], 1u);
             bins.list[slot] = (uint32_t)i;
         } else {
-            atomicAdd(&bins.count[brick], 1u);
+            atomicAdd(&bins.count[bar], 1u);
         }
     }
 }
@@ -86,7 +87,7 @@ __device__ __forceinline__ void bin_walk(const BoardsDev& b, int D, Bins& bins) 
 __global__ void k_bin_count(BoardsDev b, int D, Bins bins) { bin_walk<false>(b, D, bins); }
 __global__ void k_bin_fill(BoardsDev b, int D, Bins bins) { bin_walk<true>(b, D, bins); }
 
-// Exclusive scan of the brick counts in one CTA; seeds the cursors.  Each
+// Exclusive scan of the bin counts in one CTA; seeds the cursors.  Each
 // pass covers 1024 x 32 counts staged in shared memory: coalesced 16-byte
 // loads into a padded array (one spare word per 32 counts, so that a
 // thread's 32 consecutive counts fall in 32 different banks), per-thread sums,
@@ -103,7 +104,7 @@ __global__ void __launch_bounds__(1024) k_bin_scan(Bins bins) {
     extern __shared__ uint32_t s_cnt[];
     __shared__ uint32_t warp_sums[32];
     __shared__ uint32_t carry_s;
-    const int n = bins.nbricks;
+    const int n = bins.nbins;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     if (tid == 0) carry_s = 0;
     for (int base = 0; base < n; base += SCAN_TILE) {
@@ -465,207 +466,375 @@ __device__ __forceinline__ float4 box8(float4 c000, float4 c100, float4 c010, fl
     return make_float4(s.x * 0.125f, s.y * 0.125f, s.z * 0.125f, s.w * 0.125f);
 }
 
-// One CTA per 8^3 brick, 64 threads, one (x, y) column of eight voxels per
-// thread (each staged board is tested against all eight with one set of
-// shared-memory reads and one dx^2 + dy^2; a column that misses the ball
-// skips its eight tests).
-// Boards of the brick's bin are staged through shared memory; each voxel
-// tests its centre against each board's ball on the Q20 grid (int64 squared
-// distance) and sums count and Q16.16 density.
-// COV = false (voxelize): level 0 is assembled in registers, the next
+// The exact z run [j0, j1) of a column's voxels inside a ball, by the int64 test
+// of every voxel: only for columns whose run is too close to a voxel centre for
+// FP32 (k_splat).
+template <int BAR>
+__device__ __noinline__ int2 exact_run(int4 q, unsigned long long thr, int vx, int vy, int vz0) {
+    const int dx = vx - q.x, dy = vy - q.y;
+    const unsigned long long dxy = (unsigned long long)((long long)dx * dx) +
+                                   (unsigned long long)((long long)dy * dy);
+    int j0 = BAR, j1 = 0;
+    for (int j = 0; j < BAR; ++j) {
+        const int dz = vz0 + j * (int)CG_Q20 - q.z;
+        if (dxy + (unsigned long long)((long long)dz * dz) <= thr) {
+            j0 = min(j0, j);
+            j1 = j + 1;
+        }
+    }
+    return make_int2(j0, j1);
+}
+
+// Coverage splat.  One CTA per bar of 8 x 8 x BAR voxels, 64 threads, one
+// (x, y) column of BAR voxels per thread.  A board's ball meets a column in
+// one run of voxels, so a thread adds (1, density) where the run starts and
+// takes it off behind its end, in its own column of a shared-memory difference
+// array (no conflicts, no atomics); the running sums give every voxel's count
+// and Q16.16 density, modulo 2^32 like the sums they replace.
+// The run's ends are those of the exact test on the Q20 grid (integer squared
+// distance <= thr): FP32 gives cz -+ sqrt(r^2 - dx^2 - dy^2) in voxels relative to
+// the bar within a bound delta, and a column with an end closer than delta to a
+// voxel centre (about one in a thousand) takes the integer tests instead.  With
+// eps >= the error of r^2 - dx^2 - dy^2 (r^2 and coordinates rounded to 24 bits:
+// below 2e-6 r^2 + 6e-5), delta = 0.55 eps / s + 1e-4 + 1e-6 r covers the root's
+// share eps / 2s, its rounding and that of cz.
+// Bound by instruction issue in the board loop (about 60 of a warp per board).
+// With one integer test per voxel (an 8^3 brick per CTA, half of the time in
+// wide multiplications) and every brick marking its coarse occupancy cells:
+// 256^3 RGBA32F with 4096 boards 84 -> 45 us, 512^3 BF16 with 16384 1223 -> 342 us.
+// COV = false (voxelize): level 0 is assembled brick by brick, the next
 // `fused_levels` mip levels are reduced in shared memory, raw occupancy is
 // flagged.  COV = true: only the integer coverage (count, dq) is written
 // (the coverage readback and the active-voxel statistic compute it on demand).
-template <bool COV>
+// Byte of the raw level-l cell (l >= 1) of the brick (x, y, z).
+__device__ __forceinline__ int coarse_cell(const OccRaw& raw, int l, int x, int y, int z) {
+    const int m = raw.nb[l];
+    x = min(x >> (l - 1), m - 1);
+    y = min(y >> (l - 1), m - 1);
+    z = min(z >> (l - 1), m - 1);
+    return raw.off[l] + (z * m + y) * m + x;
+}
+
+constexpr int SPLAT_ILP = 4;
+
+// A tile's voxel: the channels the format stores (the means of the others are
+// not kept).
+__device__ __forceinline__ void put(float4& t, const float4& v) { t = v; }
+__device__ __forceinline__ void put(float2& t, const float4& v) { t = make_float2(v.x, v.y); }
+__device__ __forceinline__ float4 get(const float4& t) { return t; }
+__device__ __forceinline__ float4 get(const float2& t) { return make_float4(t.x, t.y, 0.f, 0.f); }
+template <int FMT>
+struct TileOf {
+    using T = float4;
+};
+template <>
+struct TileOf<1> {
+    using T = float2;
+};
+
+template <bool COV, int BAR, int FMT>
 __global__ void __launch_bounds__(64) k_splat(BoardsDev b, Bins bins, const uint8_t* mask,
                                                VolDesc vd, void* pyr, uint32_t* count,
                                                uint32_t* dqout, int fused_levels,
                                                OccRaw occ_raw) {
-    // the staged boards and, once every thread has left the board loop, the
-    // brick's level-0 tile share one buffer (more resident bricks per SM)
-    static_assert(CG_SPLAT_CHUNK * 28 <= CG_BRICK * CG_BRICK * CG_BRICK * 16,
-                  "board chunk larger than the tile it shares memory with");
-    __shared__ __align__(16) uint8_t s_buf[CG_BRICK * CG_BRICK * CG_BRICK * 16];
-    int4* sq = reinterpret_cast<int4*>(s_buf);
-    unsigned long long* sthr = reinterpret_cast<unsigned long long*>(s_buf + CG_SPLAT_CHUNK * 16);
-    uint32_t* sdq = reinterpret_cast<uint32_t*>(s_buf + CG_SPLAT_CHUNK * 24);
-    float4* tile = reinterpret_cast<float4*>(s_buf);
-    __shared__ unsigned s_cells;  // raw occupancy of the brick's eight 4^3 cells
+    // 4 KB ahead of the difference array hold the staged boards; brick i's
+    // level-0 tile (8 KB at 4 KB i) covers them and rows every thread has read
+    constexpr int HALF_TILE = CG_BRICK * CG_BRICK * CG_BRICK * 8;
+    __shared__ __align__(16) uint8_t s_buf[HALF_TILE + (BAR + 1) * 64 * 8];
+    static_assert(CG_SPLAT_CHUNK * 36 <= HALF_TILE && CG_SPLAT_CHUNK == 64, "staged boards");
+    static_assert(HALF_TILE == CG_BRICK * 64 * 8 && BAR % CG_BRICK == 0, "tile over the rows");
+    float4* sa = reinterpret_cast<float4*>(s_buf);                        // cx, cy, cz, r^2
+    float4* sb = reinterpret_cast<float4*>(s_buf + CG_SPLAT_CHUNK * 16);  // .55 eps, d0, eps, dq
+    uint32_t* si = reinterpret_cast<uint32_t*>(s_buf + CG_SPLAT_CHUNK * 32);  // board
+    using Tile = typename TileOf<FMT>::T;
     __shared__ float4 tile1[64];
     __shared__ float4 tile2[8];
 
-    const int brick = blockIdx.x;
-    const int bx = brick % bins.nbx;
-    const int by = (brick / bins.nbx) % bins.nby;
-    const int bz = brick / (bins.nbx * bins.nby);
+    const int bx = blockIdx.x % bins.nbx;
+    const int by = (blockIdx.x / bins.nbx) % bins.nby;
+    const int bar = blockIdx.x / (bins.nbx * bins.nby);
     const int tid = threadIdx.x;
-    // voxel j of the thread: (lx, ly, j), tile index tid + 64 j
-    const int lx = tid & 7, ly = (tid >> 3) & 7, lz = 0;
+    uint2* diff = reinterpret_cast<uint2*>(s_buf + HALF_TILE) + tid;  // row j: diff[64 j]
+    const int lx = tid & 7, ly = (tid >> 3) & 7;
+    const int w = tid >> 5;
     const int D = vd.D;
     const int x = bx * CG_BRICK + lx, y = by * CG_BRICK + ly;
-    const int z0 = bz * CG_BRICK + lz;
     const bool inxy = x < D && y < D;
-    const int vx = (2 * x + 1) * (int)CG_HALF_Q20;
-    const int vy = (2 * y + 1) * (int)CG_HALF_Q20;
-    const int vz0 = (2 * z0 + 1) * (int)CG_HALF_Q20;
-    constexpr int DZ = 2 * (int)CG_HALF_Q20;  // one voxel along z
 
-    const uint32_t beg = bins.offset[brick];
-    const uint32_t n = bins.offset[brick + 1] - beg;
-    uint32_t cnt[8] = {}, dsum[8] = {};
-    const int w = tid >> 5;
-    for (uint32_t base = 0; base < n; base += CG_SPLAT_CHUNK) {
-        const uint32_t m = min((uint32_t)CG_SPLAT_CHUNK, n - base);
-        __syncthreads();
-        for (uint32_t t = tid; t < m; t += blockDim.x) {
-            uint32_t bi = bins.list[beg + base + t];
-            sq[t] = b.q[bi];
-            sthr[t] = b.thr[bi];
-            sdq[t] = b.dq[bi];
-        }
-        __syncthreads();
-        for (uint32_t k = 0; k < m; ++k) {
-            const int4 q = sq[k];
-            const unsigned long long thr = sthr[k];
-            const uint32_t dq = sdq[k];
-            const int dx = vx - q.x, dy = vy - q.y;
-            const unsigned long long dxy = (unsigned long long)((long long)dx * dx) +
-                                           (unsigned long long)((long long)dy * dy);
-            if (dxy > thr) continue;  // the column misses the ball
-            int dz = vz0 - q.z;
+    // the bricks' flags, all at once: highlights (NULL: unknown) and voxels left
+    // from an earlier voxelize
+    unsigned hlm = 0u, dirtym = 0u;
+    if (!COV) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j, dz += DZ) {
-                const unsigned long long d = dxy + (unsigned long long)((long long)dz * dz);
-                if (d <= thr) {
-                    cnt[j] += 1u;
-                    dsum[j] += dq;
+        for (int i = 0; i < BAR / CG_BRICK; ++i) {
+            const int bz = bar * (BAR / CG_BRICK) + i;
+            if (bz >= bins.nbz) continue;
+            const int brick = (bz * bins.nby + by) * bins.nbx + bx;
+            if (bins.hl == nullptr || bins.hl[brick]) hlm |= 1u << i;
+            if (bins.dirty[brick]) dirtym |= 1u << i;
+        }
+    }
+    const uint32_t beg = bins.offset[blockIdx.x];
+    const uint32_t n = bins.offset[blockIdx.x + 1] - beg;
+    if (!COV && n == 0u && (hlm | dirtym) == 0u) return;
+    if (n > 0u) {
+        const float fx = (float)lx, fy = (float)ly;
+        // voxel centre (0, 0, 0) of the bar on the Q20 grid
+        const int ox = (2 * bx * CG_BRICK + 1) * (int)CG_HALF_Q20;
+        const int oy = (2 * by * CG_BRICK + 1) * (int)CG_HALF_Q20;
+        const int oz = (2 * bar * BAR + 1) * (int)CG_HALF_Q20;
+        for (int j = 0; j <= BAR; ++j) diff[64 * j] = make_uint2(0u, 0u);
+        for (uint32_t base = 0; base < n; base += CG_SPLAT_CHUNK) {
+            const uint32_t m = min((uint32_t)CG_SPLAT_CHUNK, n - base);
+            __syncthreads();
+            sa[tid] = make_float4(0.f, 0.f, 0.f, -1e30f);  // a miss everywhere
+            sb[tid] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (tid < m) {
+                const uint32_t bi = bins.list[beg + base + tid];
+                const int4 q = b.q[bi];
+                const float r2 = __ull2float_rn(b.thr[bi]) * 0x1p-40f;
+                const float eps = 2e-6f * r2 + 6e-5f;
+                sa[tid] = make_float4(__int2float_rn(q.x - ox) * 0x1p-20f,
+                                      __int2float_rn(q.y - oy) * 0x1p-20f,
+                                      __int2float_rn(q.z - oz) * 0x1p-20f, r2);
+                sb[tid] = make_float4(0.55f * eps, 1e-4f + 1e-6f * 0x1p-20f * __int2float_rn(q.w),
+                                      eps, __uint_as_float(b.dq[bi]));
+                si[tid] = bi;
+            }
+            __syncthreads();
+            // the runs of SPLAT_ILP boards are worked out side by side (their
+            // chains are long), then added in turn
+            for (uint32_t k0 = 0; k0 < m; k0 += SPLAT_ILP) {
+                int j0[SPLAT_ILP], j1[SPLAT_ILP];
+                uint32_t dq[SPLAT_ILP];
+                unsigned unsure = 0u;
+#pragma unroll
+                for (int u = 0; u < SPLAT_ILP; ++u) {
+                    constexpr float MAGIC = 12582912.f;  // 1.5 * 2^23
+                    constexpr int BIAS = 0x4B400000;     // its bits
+                    const float4 A = sa[k0 + u], B = sb[k0 + u];  // (past m: misses)
+                    const float dx = fx - A.x, dy = fy - A.y;
+                    const float rem = fmaf(-dy, dy, fmaf(-dx, dx, A.w));
+                    float rs;
+                    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(rs) : "f"(rem));
+                    const float s = rem * rs, clear = 0.5f - fmaf(B.x, rs, B.y);
+                    const float hi = A.z + s, lo = A.z - s;
+                    const float th = __fadd_rd(hi, MAGIC), tl = __fadd_ru(lo, MAGIC);
+                    const float fh = hi - (th - MAGIC), fl = (tl - MAGIC) - lo;
+                    // (a root of 0 or less makes these comparisons false)
+                    const bool sure = fabsf(fh - 0.5f) <= clear && fabsf(fl - 0.5f) <= clear;
+                    if (!sure && !(rem < -B.z)) unsure |= 1u << u;
+                    const int a = max(__float_as_int(tl) - BIAS, 0);
+                    const int e = min(__float_as_int(th) - BIAS + 1, BAR);
+                    // (a miss starts and ends in the row behind the bar, which
+                    // nothing reads)
+                    const bool hit = sure && a < e;
+                    j0[u] = hit ? a : BAR;
+                    j1[u] = hit ? e : BAR;
+                    dq[u] = __float_as_uint(B.w);
+                }
+#pragma unroll
+                for (int u = 0; u < SPLAT_ILP; ++u) {
+                    uint2 p = diff[64 * j0[u]], e = diff[64 * j1[u]];
+                    p.x += 1u;
+                    p.y += dq[u];
+                    e.x -= 1u;
+                    e.y -= dq[u];
+                    diff[64 * j0[u]] = p;
+                    diff[64 * j1[u]] = e;
+                }
+                while (unsure) {
+                    const uint32_t k = k0 + __ffs(unsure) - 1;
+                    unsure &= unsure - 1u;
+                    const uint32_t bi = si[k];
+                    const int2 r = exact_run<BAR>(b.q[bi], b.thr[bi], ox + lx * (int)CG_Q20,
+                                                  oy + ly * (int)CG_Q20, oz);
+                    if (r.x >= r.y) continue;
+                    diff[64 * r.x].x += 1u;
+                    diff[64 * r.x].y += b.dq[bi];
+                    diff[64 * r.y].x -= 1u;
+                    diff[64 * r.y].y -= b.dq[bi];
                 }
             }
         }
     }
-    if (COV) {
+
+    uint2 run = make_uint2(0u, 0u);  // the column's running sums
+#pragma unroll 1
+    for (int i = 0; i < BAR / CG_BRICK; ++i) {
+        const int bz = bar * (BAR / CG_BRICK) + i;
+        if (bz >= bins.nbz) break;
+        const int brick = (bz * bins.nby + by) * bins.nbx + bx;
+        const int z0 = bz * CG_BRICK;
+        const size_t o = ((size_t)z0 * D + y) * D + x, slice = (size_t)D * D;
+        const int nz = inxy ? min(D - z0, 8) : 0;  // the column's voxels in the volume
+        uint32_t cnt[8] = {}, dsum[8] = {};
+        uint32_t any = 0u;
+        if (n > 0u) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int z = z0 + j;
-            if (!(inxy && z < D)) continue;
-            const size_t i = ((size_t)z * D + y) * D + x;
-            count[i] = cnt[j];
-            dqout[i] = dsum[j];
+            for (int j = 0; j < 8; ++j) {
+                const uint2 d = diff[64 * (8 * i + j)];
+                run.x += d.x;
+                run.y += d.y;
+                cnt[j] = run.x;
+                dsum[j] = run.y;
+                any |= run.x;
+            }
         }
-        return;
-    }
-    // Raw occupancy (4^3 cells, every level): the brick's eight level-0 cells
-    // from its voxels, and at level l >= 1 the one cell holding the brick
-    // (level-l cell = brick >> (l - 1)).  Idempotent byte stores into grids
-    // cleared before the launch; k_occ_dilate builds the brick grids.
-    if (tid == 0) s_cells = 0u;
-    // the brick's highlight bits, then one block decision (which is also the
-    // barrier after the board loop: the tile may be written): a brick without
-    // boards or highlights whose voxels are still zero from an earlier
-    // voxelize writes nothing
-    // (with per-brick flags, a brick no highlight store touched reads none of
-    // its 512 mask bytes)
-    const bool hl = bins.hl == nullptr || bins.hl[brick] != 0;
-    unsigned mkb = 0u;
-    if (hl) {
+        if (COV) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int z = z0 + j;
-            if (inxy && z < D && mask[((size_t)z * D + y) * D + x]) mkb |= 1u << j;
+            for (int j = 0; j < 8; ++j) {
+                if (j >= nz) continue;
+                count[o + j * slice] = cnt[j];
+                dqout[o + j * slice] = dsum[j];
+            }
+            continue;
         }
-    }
-    const bool keep = n > 0u || (hl && __syncthreads_or(mkb != 0u));
-    if (!keep && !bins.dirty[brick]) return;
-    __syncthreads();  // every thread has read the flag
-    if (tid == 0) bins.dirty[brick] = keep ? 1 : 0;
-    {
-        // the warp's voxels lie in cell y = w & 1; voxel j in cell z = j >> 2;
-        // lanes 0-3 of each row of 8 in x cell 0, lanes 4-7 in x cell 1
-        const int cy = 2 * (w & 1);
-        unsigned bits = 0u;
+        // the brick's highlight bits (a brick whose flag is clear reads none of
+        // its 512 mask bytes), then one block decision, which is also the barrier
+        // behind the running sums (the tile may be written): a brick without
+        // coverage or highlights whose voxels are still zero from an earlier
+        // voxelize writes nothing
+        const bool hl = (hlm >> i) & 1u, dirty = (dirtym >> i) & 1u;
+        unsigned mkb = 0u;
+        if (hl) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                if (j < nz && mask[o + j * slice]) mkb |= 1u << j;
+        }
+        const bool vote = n > 0u || hl;
+        const bool keep = vote && __syncthreads_or((any != 0u && inxy) || mkb != 0u);
+        if (!keep && !dirty) continue;
+        if (!vote) __syncthreads();
+        if (tid == 0) bins.dirty[brick] = keep ? 1 : 0;
+        Tile* tile = reinterpret_cast<Tile*>(s_buf + HALF_TILE * i);
+        uint32_t dense[2] = {0u, 0u};  // density in the column's lower and upper cell
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            const int z = z0 + j;
-            const bool in = inxy && z < D;
+            const bool in = j < nz, mk = (mkb >> j) & 1u;
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
             if (in) {
-                const bool mk = (mkb >> j) & 1u;
                 v.x = __uint2float_rn(dsum[j]) * (1.0f / 65536.0f);
                 v.y = mk ? 1.0f : 0.0f;
-                v.z = __uint2float_rn(cnt[j]);
-                v.w = (cnt[j] > 0u || mk) ? 1.0f : 0.0f;
-                store_voxel(vd, pyr, 0, x, y, z, v);
+                dense[j >> 2] |= dsum[j];
+                __half2 h;
+                if (FMT == 0) {
+                    v.z = __uint2float_rn(cnt[j]);
+                    v.w = (cnt[j] > 0u || mk) ? 1.0f : 0.0f;
+                    if (CG_IN_BOUNDS(o + j * slice, vd.nvox))
+                        reinterpret_cast<float4*>(pyr)[o + j * slice] = v;
+                    h = __floats2half2_rn(v.x, v.y);
+                } else {
+                    const uint32_t p = pack_bf16_fp16(v.x, v.y);
+                    if (CG_IN_BOUNDS(o + j * slice, vd.nvox))
+                        reinterpret_cast<uint32_t*>(pyr)[o + j * slice] = p;
+                    h = __halves2half2(__float2half_rn(__uint_as_float(p << 16)),
+                                       __ushort_as_half((unsigned short)(p >> 16)));
+                }
+                if (vd.surf[0])
+                    surf3Dwrite(*reinterpret_cast<uint32_t*>(&h), vd.surf[0], x * 4, y, z0 + j);
             }
-            if (fused_levels > 0) tile[tid + 64 * j] = v;  // voxel (lx, ly, j)
-            // density v.x > 0 exactly when dsum > 0
-            const unsigned bal = __ballot_sync(0xffffffffu, in && dsum[j] > 0u);
-            const int cz = 4 * (j >> 2);
-            if (bal & 0x0F0F0F0Fu) bits |= 1u << (cy + cz);
-            if (bal & 0xF0F0F0F0u) bits |= 1u << (cy + cz + 1);
+            if (fused_levels > 0) put(tile[tid + 64 * j], v);  // voxel (lx, ly, j)
         }
-        if ((tid & 31) == 0 && bits) atomicOr(&s_cells, bits);
-    }
-    __syncthreads();
-    const unsigned cells = s_cells;
-    if (cells && tid < 8 + vd.L - 1) {
-        int l, cx, cy, cz;
-        bool set;
-        if (tid < 8) {
-            l = 0;
-            set = (cells >> tid) & 1u;
-            cx = 2 * bx + (tid & 1);
-            cy = 2 * by + ((tid >> 1) & 1);
-            cz = 2 * bz + (tid >> 2);
-        } else {
-            l = tid - 7;
-            set = true;
-            cx = bx >> (l - 1);
-            cy = by >> (l - 1);
-            cz = bz >> (l - 1);
+        // Raw occupancy: the brick's eight 4^3 cells from its voxels (density > 0
+        // exactly when the sum is).  The warp's columns lie in cell row y = w;
+        // lanes 0-3 of each row of 8 in x cell 0, lanes 4-7 in x cell 1.  Byte
+        // stores into a grid cleared before the launch.  The level-l cell (l >= 1)
+        // of a brick is brick >> (l - 1): marked here where bars are bricks (small
+        // volumes), by k_occ_coarse where thousands of bricks would meet in one.
+        const int lane = tid & 31;
+        unsigned filled = 0u;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const unsigned bal = __ballot_sync(0xffffffffu, dense[c] != 0u);
+            const int nb = occ_raw.nb[0];
+            filled |= bal;
+            if (lane < 2 && (bal & (0x0F0F0F0Fu << (4 * lane)))) {
+                const int at = ((2 * bz + c) * nb + 2 * by + w) * nb + 2 * bx + lane;
+                if (CG_IN_BOUNDS(at, nb * nb * nb)) occ_raw.raw[occ_raw.off[0] + at] = 1;
+            }
         }
-        const int nb = occ_raw.nb[l];
-        if (set) {
-            cx = min(cx, nb - 1);
-            cy = min(cy, nb - 1);
-            cz = min(cz, nb - 1);
-            uint8_t* p = occ_raw.raw + occ_raw.off[l] + ((size_t)cz * nb + cy) * nb + cx;
-            if (!*(volatile uint8_t*)p) *p = 1;
-        }
-    }
-    if (fused_levels <= 0) return;
-    // level 1: 4^3 parents
-    if (tid < 64) {
-        int px = tid & 3, py = (tid >> 2) & 3, pz = tid >> 4;
-#define T8(a, b2, c) tile[((2 * pz + (c)) * 8 + (2 * py + (b2))) * 8 + (2 * px + (a))]
-        float4 m1 = box8(T8(0, 0, 0), T8(1, 0, 0), T8(0, 1, 0), T8(1, 1, 0), T8(0, 0, 1),
-                         T8(1, 0, 1), T8(0, 1, 1), T8(1, 1, 1));
+        if (BAR == CG_BRICK && filled && lane >= 1 && lane < vd.L)
+            occ_raw.raw[coarse_cell(occ_raw, lane, bx, by, bz)] = 1;
+        __syncthreads();
+        if (fused_levels <= 0) continue;
+        // level 1: 4^3 parents, then levels 2 and 3 by the first warp alone (the
+        // other goes on; the next brick's tiles wait for both at its barriers)
+        {
+            const int px = tid & 3, py = (tid >> 2) & 3, pz = tid >> 4;
+#define T8(a, b2, c) get(tile[((2 * pz + (c)) * 8 + (2 * py + (b2))) * 8 + (2 * px + (a))])
+            const float4 m1 = box8(T8(0, 0, 0), T8(1, 0, 0), T8(0, 1, 0), T8(1, 1, 0), T8(0, 0, 1),
+                                   T8(1, 0, 1), T8(0, 1, 1), T8(1, 1, 1));
 #undef T8
-        int gx = bx * 4 + px, gy = by * 4 + py, gz = bz * 4 + pz;
-        if (gx < vd.dims[1] && gy < vd.dims[1] && gz < vd.dims[1])
-            store_voxel(vd, pyr, 1, gx, gy, gz, m1);
-        tile1[tid] = m1;
-    }
-    __syncthreads();
-    if (fused_levels < 2) return;
-    if (tid < 8) {
-        int px = tid & 1, py = (tid >> 1) & 1, pz = tid >> 2;
+            store_voxel(vd, pyr, 1, bx * 4 + px, by * 4 + py, bz * 4 + pz, m1);
+            tile1[tid] = m1;
+        }
+        if (fused_levels < 2) continue;
+        __syncthreads();
+        if (w != 0) continue;
+        if (tid < 8) {
+            const int px = tid & 1, py = (tid >> 1) & 1, pz = tid >> 2;
 #define T4(a, b2, c) tile1[((2 * pz + (c)) * 4 + (2 * py + (b2))) * 4 + (2 * px + (a))]
-        float4 m2 = box8(T4(0, 0, 0), T4(1, 0, 0), T4(0, 1, 0), T4(1, 1, 0), T4(0, 0, 1),
-                         T4(1, 0, 1), T4(0, 1, 1), T4(1, 1, 1));
+            const float4 m2 = box8(T4(0, 0, 0), T4(1, 0, 0), T4(0, 1, 0), T4(1, 1, 0), T4(0, 0, 1),
+                                   T4(1, 0, 1), T4(0, 1, 1), T4(1, 1, 1));
 #undef T4
-        int gx = bx * 2 + px, gy = by * 2 + py, gz = bz * 2 + pz;
-        if (gx < vd.dims[2] && gy < vd.dims[2] && gz < vd.dims[2])
-            store_voxel(vd, pyr, 2, gx, gy, gz, m2);
-        tile2[tid] = m2;
+            store_voxel(vd, pyr, 2, bx * 2 + px, by * 2 + py, bz * 2 + pz, m2);
+            tile2[tid] = m2;
+        }
+        __syncwarp();
+        if (fused_levels >= 3 && tid == 0)
+            store_voxel(vd, pyr, 3, bx, by, bz,
+                        box8(tile2[0], tile2[1], tile2[2], tile2[3], tile2[4], tile2[5], tile2[6],
+                             tile2[7]));
+        __syncwarp();
+    }
+}
+
+// Raw occupancy of the levels above 0 from the bricks' dirty flags (1 after a
+// splat when the brick holds coverage or highlights, which may mark a cell
+// without density: the flags only have to cover it): the level-l cell of a brick
+// is brick >> (l - 1).  A CTA reduces 8^3 bricks to their cells of levels 1 to 4
+// and marks the one cell of each level beyond.  In the splat itself every
+// brick marked its cell of every level, ten thousand reads of the same few
+// bytes (29 of the splat's 75 us at 256^3).
+__global__ void __launch_bounds__(512) k_occ_coarse(const uint8_t* dirty, int nb, OccRaw raw,
+                                                    int L) {
+    grid_dep_trigger();  // the dilation may be scheduled (it waits for the cells)
+    __shared__ uint8_t s1[512], s2[64], s3[8];
+    const int t = threadIdx.x, n8 = (nb + 7) / 8;
+    const int gx = blockIdx.x % n8 * 8, gy = blockIdx.x / n8 % n8 * 8, gz = blockIdx.x / (n8 * n8) * 8;
+    auto mark_cell = [&](int l, int x, int y, int z) { raw.raw[coarse_cell(raw, l, x, y, z)] = 1; };
+    {
+        const int x = gx + (t & 7), y = gy + ((t >> 3) & 7), z = gz + (t >> 6);
+        const bool v = x < nb && y < nb && z < nb && dirty[(z * nb + y) * nb + x];
+        s1[t] = v;
+        if (v) mark_cell(1, x, y, z);
+    }
+    if (L <= 2) return;
+    __syncthreads();
+    if (t < 64) {
+        const int x = t & 3, y = (t >> 2) & 3, z = t >> 4;
+        uint8_t v = 0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            v |= s1[((2 * z + (k >> 2)) * 8 + 2 * y + ((k >> 1) & 1)) * 8 + 2 * x + (k & 1)];
+        s2[t] = v;
+        if (v) mark_cell(2, gx + 2 * x, gy + 2 * y, gz + 2 * z);
+    }
+    if (L <= 3) return;
+    __syncthreads();
+    if (t < 8) {
+        const int x = t & 1, y = (t >> 1) & 1, z = t >> 2;
+        uint8_t v = 0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            v |= s2[((2 * z + (k >> 2)) * 4 + 2 * y + ((k >> 1) & 1)) * 4 + 2 * x + (k & 1)];
+        s3[t] = v;
+        if (v) mark_cell(3, gx + 4 * x, gy + 4 * y, gz + 4 * z);
     }
     __syncthreads();
-    if (fused_levels < 3) return;
-    if (tid == 0) {
-        float4 m3 = box8(tile2[0], tile2[1], tile2[2], tile2[3], tile2[4], tile2[5], tile2[6],
-                         tile2[7]);
-        if (bx < vd.dims[3] && by < vd.dims[3] && bz < vd.dims[3])
-            store_voxel(vd, pyr, 3, bx, by, bz, m3);
-    }
+    if (t >= 4 && t < L && (s3[0] | s3[1] | s3[2] | s3[3] | s3[4] | s3[5] | s3[6] | s3[7]))
+        mark_cell(t, gx, gy, gz);
 }
 
 // Dilated occupancy: occ[l][c] = 1 when a raw 4^3 cell of level l inside
@@ -710,6 +879,7 @@ __global__ void __launch_bounds__(256) k_occ_dilate(const __grid_constant__ VolD
                                                     const __grid_constant__ OccRaw raw,
                                                     const __grid_constant__ DilateUnits units,
                                                     uint8_t* occ, int* box) {
+    grid_dep_wait();  // the coarse levels' raw cells
     const int lane = threadIdx.x & 31;
     const int unit = blockIdx.x * 8 + (threadIdx.x >> 5);
     unsigned m[6] = {0u, 0u, 0u, 0u, 0u, 0u};  // this thread's box terms (0 = none)
@@ -954,15 +1124,38 @@ cudaError_t launch_highlight(const BoardsDev& b, const SunFrame& fr, const uint6
     return cudaGetLastError();
 }
 
+// Tall bars save board tests (a board meets fewer of them, and a column's run
+// costs the same whatever its length) but put more work behind one another in a
+// CTA: with few bricks, bars of one brick.  Voxelize, us, bars of 8 and 32 voxels:
+// 64^3 (64 boards) 58 and 63, 128^3 (1024) 75 and 77, 192^3 (2048) 103 and 98,
+// 256^3 (4096, BF16) 171 and 145; bars of 16 lie between or beside them.
+int splat_bar(int dimension) { return dimension <= 128 ? 8 : 32; }
+
+namespace {
+template <bool COV, int FMT>
+void splat(const BoardsDev& b, Bins bins, const uint8_t* mask, const VolDesc& vd, void* pyr,
+           uint32_t* count, uint32_t* dq, int fused_levels, OccRaw occ, cudaStream_t st) {
+    auto* kernel = bins.bar == 8 ? k_splat<COV, 8, FMT> : k_splat<COV, 32, FMT>;
+    kernel<<<bins.nbins, 64, 0, st>>>(b, bins, mask, vd, pyr, count, dq, fused_levels, occ);
+}
+}  // namespace
+
 cudaError_t launch_splat(const BoardsDev& b, Bins bins, const uint8_t* mask, VolDesc vd,
                          void* pyr, uint32_t* count, uint32_t* dq, int fused_levels,
                          OccRaw occ, bool coverage_only, cudaStream_t st) {
     if (coverage_only)
-        k_splat<true><<<bins.nbricks, 64, 0, st>>>(b, bins, mask, vd, pyr, count, dq,
-                                                    fused_levels, occ);
+        splat<true, 0>(b, bins, mask, vd, pyr, count, dq, fused_levels, occ, st);
+    else if (vd.fmt == 0)
+        splat<false, 0>(b, bins, mask, vd, pyr, count, dq, fused_levels, occ, st);
     else
-        k_splat<false><<<bins.nbricks, 64, 0, st>>>(b, bins, mask, vd, pyr, count, dq,
-                                                     fused_levels, occ);
+        splat<false, 1>(b, bins, mask, vd, pyr, count, dq, fused_levels, occ, st);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_occ_coarse(const Bins& bins, OccRaw raw, int L, cudaStream_t st) {
+    if (L < 2 || bins.bar == CG_BRICK) return cudaSuccess;  // (the splat marked them)
+    const int n8 = (bins.nbx + 7) / 8;
+    k_occ_coarse<<<n8 * n8 * n8, 512, 0, st>>>(bins.dirty, bins.nbx, raw, L);
     return cudaGetLastError();
 }
 
@@ -977,7 +1170,8 @@ cudaError_t launch_occ_dilate(VolDesc vd, OccRaw raw, uint8_t* occ, int total, c
             if (l < vd.L) n += (nb + 31) / 32 * nb * ((nb + dilate_run(nb) - 1) / dilate_run(nb));
         }
         u.first[CG_MAX_LEVELS] = n;
-        k_occ_dilate<<<(n + 7) / 8, 256, 0, st>>>(vd, raw, u, occ, box);
+        return launch_dependent(k_occ_dilate, dim3((n + 7) / 8), dim3(256), 0, st, vd, raw, u, occ,
+                                box);
     } else {
         k_occ_dilate_wide<<<(total + 255) / 256, 256, 0, st>>>(vd, raw, occ, total, box);
     }

@@ -7,6 +7,7 @@ import pytest
 import cloudgb
 from cloudgb import configs
 from cloudgb.scene import billboards
+from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
 
@@ -73,3 +74,42 @@ def test_images_do_not_depend_on_the_brick(ctx, dim, mips):
         assert images[0][..., 3].max() > 0.1
         for im in images[1:]:
             assert np.array_equal(im, images[0])
+
+
+@pytest.mark.parametrize("dim,mips", [(17, 3), (64, 7), (136, 5), (150, 4), (200, 4)])
+def test_coverage_of_touching_and_extreme_balls(ctx, dim, mips):
+    """Counts and Q16.16 sums against the oracle, bit for bit, where the splat's
+    runs are decided by a hair: centres on voxel centres, faces and quarter
+    voxels with radii that put voxel centres on the sphere, balls smaller than
+    a voxel and as large as the box, columns touched at their tip, boards
+    beyond the faces, and sums that wrap."""
+    rng = np.random.default_rng(dim)
+    n = 160
+    cell = np.float32(1.0 / dim)
+    centre = (rng.integers(-2, 4 * dim + 2, (n, 3)) / 4.0).astype(np.float32)  # voxels
+    radius = rng.choice([0.0, 0.25, 0.5, 1.0, 1.25, 2.5, 5.0, 6.5, 13.0], n).astype(np.float32)
+    # the coverage test keeps 0.9999 of the squared radius: on either side of it
+    radius[::3] *= np.float32(1.0 / np.sqrt(0.9999))
+    radius[1::7] = rng.uniform(0.2, 0.45 * dim, len(radius[1::7]))
+    radius[5], radius[6] = dim, 0.999 * dim
+    centre[5:7] = dim / 2 + 0.5
+    pos = centre * cell - np.float32(0.5)
+    den = rng.choice([0.5, 1.0, 32767.5], n).astype(np.float32)
+    vol = cloudgb.CloudVolume(dim, configs.VOLUME_BOUNDS, configs.VOLUME_POSITION, mips, ctx=ctx)
+    ov = O.OracleVolume(dim, configs.VOLUME_BOUNDS, configs.VOLUME_POSITION, mips)
+    sun = cloudgb.Sun((0.3, 1.0, 0.2), 40, 24)
+    for keep in (slice(0, n), slice(20, 24), slice(0, 0)):  # the bricks of the first scene empty
+        p, r, d = pos[keep], radius[keep] * cell, den[keep]
+        vol.set_billboards(p, r, d)
+        vol.update()
+        cloudgb.VoxelizeShader().voxelize(vol, sun)
+        assert ov.set_boards(p, r, d) == 0
+        assert ov.voxelize(sun.direction, 40, 24) == 0
+        cnt, dq = vol.read_coverage()
+        ocnt, odq = ov.coverage()
+        assert np.array_equal(cnt, ocnt)
+        assert np.array_equal(dq, odq)
+        raw = vol.read_level(0)
+        assert np.array_equal(raw[..., 2], ocnt.astype(np.float32))
+        assert np.array_equal(raw[..., 0], odq.astype(np.float32) * np.float32(2.0 ** -16))
+        assert np.array_equal(raw[..., 1] > 0, ov.mask() > 0)
