@@ -64,10 +64,8 @@ extern "C" cg_status cg_context_create(int device, cg_context** out) {
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->fork_ev, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->join_ev, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->clear_ev, cudaEventDisableTiming);
     if (e != cudaSuccess) {
         if (c->join_ev) cudaEventDestroy(c->join_ev);
-        if (c->clear_ev) cudaEventDestroy(c->clear_ev);
         if (c->fork_ev) cudaEventDestroy(c->fork_ev);
         if (c->side) cudaStreamDestroy(c->side);
         if (c->stream) cudaStreamDestroy(c->stream);
@@ -308,7 +306,6 @@ void context_release(cg_context* ctx) {
         if (e) cudaEventDestroy(e);
     cudaEventDestroy(ctx->fork_ev);
     cudaEventDestroy(ctx->join_ev);
-    cudaEventDestroy(ctx->clear_ev);
     cudaStreamDestroy(ctx->side);
     cudaStreamDestroy(ctx->stream);
     delete ctx;
@@ -479,8 +476,8 @@ extern "C" cg_status cg_volume_create(cg_context* ctx, int dimension, float boun
     v->bins.bar = splat_bar(dimension);
     v->bins.nbarz = (dimension + v->bins.bar - 1) / v->bins.bar;
     v->bins.nbins = nb * nb * v->bins.nbarz;
-    if (e == cudaSuccess) e = v->bcount.ensure((size_t)v->bins.nbins * 4);
-    if (e == cudaSuccess) e = v->boff.ensure(((size_t)v->bins.nbins + 1) * 4);
+    if (e == cudaSuccess) e = v->bcount.ensure(((size_t)v->bins.nbins + 1) * 4);
+    if (e == cudaSuccess) e = v->boff.ensure((size_t)v->bins.nbins * 4);
     if (e == cudaSuccess) e = v->bcursor.ensure((size_t)v->bins.nbins * 4);
     // every brick starts dirty: the pyramid's memory is uninitialised
     if (e == cudaSuccess) e = v->bdirty.ensure((size_t)v->bins.nbricks);
@@ -624,13 +621,16 @@ extern "C" cg_status cg_volume_set_billboards(cg_volume* v, const float* positio
     CG_CHECK(pairs < (size_t)0xFFFFFFFFu, CG_ERR_OUT_OF_RANGE,
              "cg_volume_set_billboards: %zu board-bar pairs exceed 2^32", pairs);
     // the device records mirror the staging layout: one copy uploads them all
-    CG_CUDA(v->boards.ensure(total));
+    // and behind them the sun-view pass keeps its own
+    const size_t o_sun = (total + 255) / 256 * 256;
+    CG_CUDA(v->boards.ensure(o_sun + n * SUN_BOARD_BYTES));
     char* dev = v->boards.as<char>();
     v->cwr = reinterpret_cast<float4*>(dev + o_cwr);
     v->q = reinterpret_cast<int4*>(dev + o_q);
     v->thr = reinterpret_cast<uint64_t*>(dev + o_thr);
     v->dqb = reinterpret_cast<uint32_t*>(dev + o_dq);
     v->culled = reinterpret_cast<uint8_t*>(dev + o_cul);
+    v->sun_boards = dev + o_sun;
     CG_CUDA(v->blist.ensure(pairs * 4));
     cudaStream_t s = v->ctx->stream;
     if (n) CG_CUDA(cudaMemcpyAsync(dev, st, total, cudaMemcpyHostToDevice, s));
@@ -805,7 +805,8 @@ extern "C" cg_status cg_voxelize(cg_volume* v, const cg_sun* sun, void* stream) 
     const size_t texels = (size_t)sun->map_width * sun->map_height;
     if (v->mapW != sun->map_width || v->mapH != sun->map_height) {
         CG_CUDA(cudaStreamSynchronize(s));
-        CG_CUDA(v->keys.ensure(texels * 8));
+        CG_CUDA(v->keys.ensure(texels * 8 +
+                               sun_aux_words(sun->map_width, sun->map_height) * 4));
         CG_CUDA(v->posmap.ensure(texels * 16));
         v->mapW = sun->map_width;
         v->mapH = sun->map_height;
@@ -835,43 +836,36 @@ extern "C" cg_status cg_voxelize(cg_volume* v, const cg_sun* sun, void* stream) 
     if (v->ready_pending && s != ctx->stream && !capturing)
         CG_CUDA(cudaStreamWaitEvent(s, v->boards_ready, 0));
     stage_begin(ctx, s);
-    // the sun-view pass does not need the bins: it runs on the side stream
-    // while the binning (latency-bound, a few SMs busy) runs on s
+    // clearGPU (CloudVolume.cpp:96-100) + clearPositionMap (VoxelizeShader.cpp:185-187):
+    // what the sun-view pass needs is cleared on s, the rest beside it on the
+    // side stream
     cudaStream_t sd = ctx->side;
     CG_CUDA(cudaEventRecord(ctx->fork_ev, s));
     CG_CUDA(cudaStreamWaitEvent(sd, ctx->fork_ev, 0));
-    // clearGPU (CloudVolume.cpp:96-100) + clearPositionMap (VoxelizeShader.cpp:185-187):
-    // the highlight mask and its brick flags are cleared on s, where the binning
-    // has time to spare, the key map on the side stream ahead of the sun map
-    CG_CUDA(cudaMemsetAsync(v->mask.p, 0, n0, s));
-    CG_CUDA(cudaMemsetAsync(v->bhl.p, 0, (size_t)bins.nbricks, s));
-    CG_CUDA(cudaEventRecord(ctx->clear_ev, s));
-    CG_CUDA(cudaMemsetAsync(v->keys.p, 0xFF, texels * 8, sd));
+    CG_CUDA(cudaMemsetAsync(v->mask.p, 0, n0, sd));
+    CG_CUDA(cudaMemsetAsync(v->bhl.p, 0, (size_t)bins.nbricks, sd));
+    // raw cells, brick grids (rewritten by the dilation) and the occupied box
+    CG_CUDA(cudaMemsetAsync(v->occ.p, 0, occ_box_offset(v->raw_total) + 6 * sizeof(int), sd));
+    CG_CUDA(cudaEventRecord(ctx->join_ev, sd));
+    // the keys and the tiles' bounds behind them (the tables there are rewritten)
+    CG_CUDA(cudaMemsetAsync(v->keys.p, 0xFF, texels * 8 + sun_aux_words(fr.W, fr.H) * 4, s));
+    // the bars' counts and, behind them, their list's total
+    CG_CUDA(cudaMemsetAsync(bins.count, 0, ((size_t)bins.nbins + 1) * 4, s));
     {
         NvtxRange r("voxelize.sun_pass");
-        // pass 1: sun-view nearest-surface map
-        if (b.n) CG_LAUNCH(ctx, launch_sunmap(b, fr, v->keys.as<uint64_t>(), sd));
-        // pass 2: highlight stores (after the mask's clearing)
-        CG_CUDA(cudaStreamWaitEvent(sd, ctx->clear_ev, 0));
+        // pass 1: sun-view nearest-surface map, and the boards' bars
+        CG_LAUNCH(ctx, launch_sun_pass(b, fr, v->keys.as<uint64_t>(),
+                                       sun_aux(v->keys.as<uint32_t>() + 2 * texels, v->sun_boards,
+                                               fr.W, fr.H),
+                                       v->D, bins, s));
+        stage_mark(ctx, s, "sun");
+        // pass 2: highlight stores (after the mask's clearing) and the bars' lists
+        CG_CUDA(cudaStreamWaitEvent(s, ctx->join_ev, 0));
         CG_LAUNCH(ctx, launch_highlight(b, fr, v->keys.as<uint64_t>(), v->posmap.as<float4>(),
                                         v->D, v->wmin, v->range, highlight_offset(v),
-                                        v->mask.as<uint8_t>(), v->bhl.as<uint8_t>(), sd));
-        CG_CUDA(cudaEventRecord(ctx->join_ev, sd));
+                                        v->mask.as<uint8_t>(), v->bhl.as<uint8_t>(), &bins, s));
     }
-    {
-        NvtxRange r("voxelize.bins");
-        CG_CUDA(cudaMemsetAsync(bins.count, 0, (size_t)bins.nbins * 4, s));
-        // raw cells, brick grids (rewritten by the dilation) and the occupied box
-        CG_CUDA(cudaMemsetAsync(v->occ.p, 0, occ_box_offset(v->raw_total) + 6 * sizeof(int), s));
-        // brick bins
-        if (b.n) CG_LAUNCH(ctx, launch_bin_count(b, v->D, bins, s));
-        CG_LAUNCH(ctx, launch_bin_scan(bins, s));
-        if (b.n) CG_LAUNCH(ctx, launch_bin_fill(b, v->D, bins, s));
-    }
-    stage_mark(ctx, s, "bins");
-    CG_CUDA(cudaStreamWaitEvent(s, ctx->join_ev, 0));
-    // the sun-view pass's time beyond the binning
-    stage_mark(ctx, s, "sun");
+    stage_mark(ctx, s, "highlight");
     // coverage splat + level 0 + fused mips
     int fused = (v->D % CG_BRICK == 0) ? std::min(CG_FUSED_MIPS, v->L - 1) : 0;
     {

@@ -81,11 +81,10 @@ struct HostBuf {
 struct cg_context {
     int device = 0;
     cudaStream_t stream = nullptr;
-    // voxelize: the sun-view pass (sun map + highlights) runs on `side`,
-    // concurrently with the brick binning, forked and joined by two events
+    // voxelize: the clearing of the highlight mask and the occupancy dilation
+    // run on `side`, forked and joined by two events
     cudaStream_t side = nullptr;
     cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
-    cudaEvent_t clear_ev = nullptr;  // voxelize: the mask cleared (on the caller's stream)
     uint64_t launches = 0;
     int refs = 1;  // the caller's handle + one per volume / model created on it
     bool shaded_valid = false;  // the status words hold a surrogate render's counters
@@ -154,6 +153,7 @@ struct cg_volume {
     // radius, int4 Q20 centre + radius, u64 ball threshold, u32 Q16 density,
     // u8 culled (offsets 0, 16n, 32n, 40n, 44n)
     DevBuf boards;
+    void* sun_boards = nullptr;  // in it
     float4* cwr = nullptr;
     int4* q = nullptr;
     uint64_t* thr = nullptr;

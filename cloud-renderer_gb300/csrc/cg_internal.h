@@ -191,8 +191,8 @@ struct Bins {
     // the bins: bars of 8 x 8 x bar voxels (bar = 8 or 32; nbarz along z); the
     // compat render's are pixel tiles
     int bar, nbarz, nbins;
-    uint32_t* count;   // nbins
-    uint32_t* offset;  // nbins + 1
+    uint32_t* count;   // nbins (+ 1 in a volume: the list's total)
+    uint32_t* offset;  // nbins (+ 1: the compat render's scan)
     uint32_t* cursor;  // nbins
     uint32_t* list;    // pairs
     // per brick: 1 when its level-0 voxels (and fused levels 1-3) may hold
@@ -430,17 +430,31 @@ bool sun_frame_for_box(const float position[3], float b0, float b1, const float 
 // ---- launchers (return cudaGetLastError of the launch) -------------------
 // Bar height of a volume's splat (k_voxelize.cu).
 int splat_bar(int dimension);
-cudaError_t launch_bin_count(const BoardsDev& b, int D, Bins bins, cudaStream_t st);
 cudaError_t launch_bin_scan(Bins bins, cudaStream_t st);
-cudaError_t launch_bin_fill(const BoardsDev& b, int D, Bins bins, cudaStream_t st);
 cudaError_t launch_sunmap(const BoardsDev& b, const SunFrame& fr, uint64_t* keys,
                           cudaStream_t st);
+// Beside the keys of a sun map: per 8 x 4 texel tile an upper bound of the depth
+// to come (float bits, set to all ones before the pass), and the texel centres.
+struct SunAux {
+    unsigned* bound = nullptr;
+    float* x = nullptr;
+    float* y = nullptr;
+    void* boards = nullptr;  // SUN_BOARD_BYTES a board
+};
+constexpr size_t SUN_BOARD_BYTES = 64;
+size_t sun_aux_words(int W, int H);
+SunAux sun_aux(uint32_t* words, void* boards, int W, int H);
+// The sun map with its bounds, every board's count in its bars (zeroed before)
+// and the bars' ranges of the list (offset and cursor).
+cudaError_t launch_sun_pass(const BoardsDev& b, const SunFrame& fr, uint64_t* keys,
+                            const SunAux& aux, int D, const Bins& bins, cudaStream_t st);
 // hl_brick (may be NULL): per 8^3 brick of the volume, set to 1 beside every
-// mask byte set (cleared by the caller before the launch)
+// mask byte set (cleared by the caller before the launch).  fill (may be NULL):
+// the same launch fills these bins' lists
 cudaError_t launch_highlight(const BoardsDev& b, const SunFrame& fr, const uint64_t* keys,
                              float4* posmap, int D, const float wmin[3],
                              const float range[3], float offset, uint8_t* mask,
-                             uint8_t* hl_brick, cudaStream_t st);
+                             uint8_t* hl_brick, const Bins* fill, cudaStream_t st);
 // coverage_only: write the integer coverage (count, dq) and nothing else
 cudaError_t launch_splat(const BoardsDev& b, Bins bins, const uint8_t* mask, VolDesc vd,
                          void* pyr, uint32_t* count, uint32_t* dq, int fused_levels,

@@ -6,7 +6,9 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <algorithm>
 #include <atomic>
+#include <cmath>
 
 #include "cg_internal.h"
 
@@ -46,14 +48,14 @@ __device__ __forceinline__ long long axis_gap(int q, int lo, int hi) {
     return (long long)q - c;
 }
 
-// Board bin walk shared by the count and fill passes: one warp per board,
+// Board bin walk of the count (in the sun-view pass) and fill (beside the
+// highlight stores) passes: one warp per board,
 // lanes over the bars (8 x 8 x bins.bar voxels) of its voxel box; a bar is kept
 // only when its nearest voxel centre passes the board's ball test (the
 // per-voxel test in k_splat stays exact).
 template <bool FILL>
-__device__ __forceinline__ void bin_walk(const BoardsDev& b, int D, Bins& bins) {
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
+__device__ __forceinline__ void bin_walk(const BoardsDev& b, int D, const Bins& bins, int i,
+                                         int lane) {
     if (i >= b.n || b.culled[i]) return;
     const int4 q = b.q[i];
     const unsigned long long thr = b.thr[i];
@@ -83,9 +85,6 @@ __device__ __forceinline__ void bin_walk(const BoardsDev& b, int D, Bins& bins) 
         }
     }
 }
-
-__global__ void k_bin_count(BoardsDev b, int D, Bins bins) { bin_walk<false>(b, D, bins); }
-__global__ void k_bin_fill(BoardsDev b, int D, Bins bins) { bin_walk<true>(b, D, bins); }
 
 // Exclusive scan of the bin counts in one CTA; seeds the cursors.  Each
 // pass covers 1024 x 32 counts staged in shared memory: coalesced 16-byte
@@ -179,6 +178,37 @@ __global__ void __launch_bounds__(1024) k_bin_scan(Bins bins) {
     if (tid == 0) bins.offset[n] = carry_s;
 }
 
+// Ranges of the list for the bars' boards: bars need disjoint ranges in any
+// order, so a CTA takes one for its 256 bars with a single atomic on the total
+// (zeroed before; a scan in bar order took one CTA 13 us for 8192 bars).
+__device__ __forceinline__ void bin_alloc(const Bins& bins, int block) {
+    __shared__ uint32_t s_sum[8], s_base;
+    const int i = block * 256 + threadIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint32_t c = i < bins.nbins ? bins.count[i] : 0u;
+    uint32_t x = c;
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) s_sum[w] = x;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t run = 0u;
+        for (int k = 0; k < 8; ++k) {
+            const uint32_t t = s_sum[k];
+            s_sum[k] = run;
+            run += t;
+        }
+        s_base = run ? atomicAdd(bins.count + bins.nbins, run) : 0u;
+    }
+    __syncthreads();
+    if (i < bins.nbins) {
+        const uint32_t at = s_base + s_sum[w] + x - c;
+        bins.offset[i] = at;
+        bins.cursor[i] = at;
+    }
+}
+
 // ---- sun-view nearest-surface map (first_voxelize.glsl:39-64) --------------
 
 __device__ __forceinline__ float dot3(const float a[3], float x, float y, float z) {
@@ -232,91 +262,216 @@ __device__ __forceinline__ void texel_range(float lo, float hi, float c, float r
     b = (int)fb;
 }
 
-// One CTA per board.  The texel-centre coordinates of the board's box are
-// tabulated once (one division per column and per row instead of two per
-// texel); each warp then takes rows and sweeps, with consecutive lanes on
-// consecutive texels, only the columns of the row's chord through the disc
-// (d^2 <= 1.0001 r^2, widened by one texel each side; the per-texel test
-// below still applies, so the chord only drops texels it would reject).
-constexpr int SUN_TAB = 1024;
+// The map is swept in tiles of 8 x 4 texels, one warp pass each.  Most boards at
+// a texel lie far behind the front one, and in submission order many exact depths
+// (three IEEE roots and a division) were worked out before a front board had
+// come by.  So a first pass takes, from every tile a board's disc covers
+// well, an upper bound of the depths it will store there; the second passes over
+// the tiles at which a board cannot beat the tile's bound, and tests the texels of
+// the others against their current depth.  Instructions, 4096 boards on 1280 x 720:
+// 33 M with one CTA per board over every texel of its rows (49 us), 5.7 M + 8.9 M
+// in the two passes (12.7 + 20.5 us with the bars' counts and ranges, which took
+// 27 us in kernels of their own); what is left is latency at half occupancy.
+// Voxelize as a whole, us: 64^3 of 64 boards 56 -> 49, 256^3 BF16 of 4096
+// 144 -> 122, 512^3 BF16 of 16384 1029 -> 879.
+constexpr int SUN_TW = 8, SUN_TH = 4;
+constexpr int SUN_AHEAD = 4;  // tiles in flight a warp (1, 2, 4: 54.5, 53.9, 53.4 us)
 
-__device__ __forceinline__ float sun_x(const SunFrame& fr, const float* tab, bool tabbed, int ia,
-                                       int ti) {
-    return tabbed ? tab[ti - ia] : texel_coord(fr.lo, fr.hi, ti, fr.W);
+// A board in sun view: its texel box (empty: ia > ib) and the smallest square
+// of the surface offset dz = (cv.z + r * prof) + near_z over prof in [0, 1]
+// (rounded steps are monotone).
+struct alignas(16) SunBoard {
+    float3 cv;
+    float r, dz2_min;
+    int ia, ib, ja, jb;
+    int tx0, ntx, ty0, tiles;  // its tiles, x fastest
+    int pad[3];
+};
+static_assert(sizeof(SunBoard) == SUN_BOARD_BYTES, "");
+
+__device__ __forceinline__ SunBoard sun_board(const BoardsDev& b, const SunFrame& fr, int i) {
+    SunBoard s;
+    const float4 c = b.cwr[i];
+    s.cv = sun_view_of(fr, c);
+    s.r = c.w;
+    texel_range(fr.lo, fr.hi, s.cv.x, s.r, fr.W, s.ia, s.ib);
+    texel_range(fr.lo, fr.hi, s.cv.y, s.r, fr.H, s.ja, s.jb);
+    const float dz_lo = fadd(s.cv.z, fr.near_z), dz_hi = fadd(fadd(s.cv.z, s.r), fr.near_z);
+    s.dz2_min = 0.0f;
+    if (dz_lo > 0.0f) s.dz2_min = fmul(dz_lo, dz_lo);
+    else if (dz_hi < 0.0f) s.dz2_min = fmul(dz_hi, dz_hi);
+    s.tx0 = s.ia / SUN_TW;
+    s.ty0 = s.ja / SUN_TH;
+    s.ntx = s.ib / SUN_TW - s.tx0 + 1;
+    s.tiles = s.ia <= s.ib && s.ja <= s.jb ? s.ntx * (s.jb / SUN_TH - s.ty0 + 1) : 0;
+    return s;
 }
 
-__global__ void __launch_bounds__(256) k_sunmap(BoardsDev b, SunFrame fr,
-                                                unsigned long long* keys) {
-    __shared__ float s_x[SUN_TAB], s_y[SUN_TAB];
-    const int i = blockIdx.x;
+// Texel centres of tile t of the board: [x0, x1] x [y0, y1], each within
+// sun_slack of the exact centres (a few roundings at the window's magnitude).
+struct SunTile {
+    int tx, ty;
+    float x0, x1, y0, y1;
+};
+__device__ __forceinline__ float sun_slack(const SunFrame& fr) {
+    return 4e-6f * fmaxf(fabsf(fr.lo), fabsf(fr.hi));
+}
+__device__ __forceinline__ SunTile sun_tile(const SunBoard& s, const SunFrame& fr, float sx,
+                                            float sy, int t) {
+    SunTile q;
+    q.tx = s.tx0 + t % s.ntx;
+    q.ty = s.ty0 + t / s.ntx;
+    q.x0 = fr.lo + ((float)(q.tx * SUN_TW) + 0.5f) * sx;
+    q.x1 = q.x0 + (float)(SUN_TW - 1) * sx;
+    q.y0 = fr.lo + ((float)(q.ty * SUN_TH) + 0.5f) * sy;
+    q.y1 = q.y0 + (float)(SUN_TH - 1) * sy;
+    return q;
+}
+
+// First pass, `parts` warps per board: the tiles' bounds (float bits, all ones =
+// none), the board's count in its bars (bins.count NULL: none); further CTAs
+// tabulate the texel centres (aux.x, aux.y).
+__global__ void __launch_bounds__(256) k_sun_bounds(BoardsDev b, SunFrame fr, SunAux aux, int parts,
+                                                    int board_blocks, int D, Bins bins) {
+    if ((int)blockIdx.x >= board_blocks) {
+        const int t = (blockIdx.x - board_blocks) * 256 + threadIdx.x;
+        if (t < fr.W) aux.x[t] = texel_coord(fr.lo, fr.hi, t, fr.W);
+        if (t < fr.H) aux.y[t] = texel_coord(fr.lo, fr.hi, t, fr.H);
+        return;
+    }
+    const int g = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const int i = g / parts, part = g % parts;
     if (i >= b.n) return;
-    float4 c = b.cwr[i];
-    float3 cv = sun_view_of(fr, c);
-    float r = c.w;
-    int ia, ib, ja, jb;
-    texel_range(fr.lo, fr.hi, cv.x, r, fr.W, ia, ib);
-    texel_range(fr.lo, fr.hi, cv.y, r, fr.H, ja, jb);
-    if (ia > ib || ja > jb) return;
-    const int nx = ib - ia + 1, ny = jb - ja + 1;
-    const bool tabbed = nx <= SUN_TAB && ny <= SUN_TAB;
-    if (tabbed) {
-        for (int t = threadIdx.x; t < nx; t += blockDim.x)
-            s_x[t] = texel_coord(fr.lo, fr.hi, ia + t, fr.W);
-        for (int t = threadIdx.x; t < ny; t += blockDim.x)
-            s_y[t] = texel_coord(fr.lo, fr.hi, ja + t, fr.H);
+    if (bins.count && part == 0) bin_walk<false>(b, D, bins, i, lane);
+    const SunBoard s = sun_board(b, fr, i);
+    if (part == 0 && lane == 0) reinterpret_cast<SunBoard*>(aux.boards)[i] = s;
+    const float span = fr.hi - fr.lo, sx = span / (float)fr.W, sy = span / (float)fr.H;
+    const float slack = sun_slack(fr);
+    const int wt = (fr.W + SUN_TW - 1) / SUN_TW;
+    for (int t = part + parts * lane; t < s.tiles; t += 32 * parts) {
+        const SunTile q = sun_tile(s, fr, sx, sy, t);
+        // the farthest texel centre lies well inside the disc: every texel's
+        // profile is at least sqrt(1 - 0.98), far above the 0.01 discard
+        const float dx = fmaxf(fabsf(q.x0 - s.cv.x), fabsf(q.x1 - s.cv.x)) + slack;
+        const float dy = fmaxf(fabsf(q.y0 - s.cv.y), fabsf(q.y1 - s.cv.y)) + slack;
+        const float d2 = dx * dx + dy * dy, r2 = s.r * s.r;
+        if (!(d2 <= 0.98f * r2)) continue;
+        const float prof = sqrtf(1.0f - d2 / r2);
+        const float z = s.cv.z + fr.near_z;
+        const float dz = fmaxf(fabsf(z + 0.999f * s.r * prof), fabsf(z + 1.001f * s.r));
+        const float x = fmaxf(fabsf(q.x0), fabsf(q.x1)), y = fmaxf(fabsf(q.y0), fabsf(q.y1));
+        const float bound = sqrtf(x * x + y * y + dz * dz) * 1.00001f + slack +
+                            1e-6f * (fabsf(s.cv.z) + fabsf(fr.near_z));
+        atomicMin(aux.bound + q.ty * wt + q.tx, __float_as_uint(bound));
+    }
+}
+
+// Second pass: the depth keys.  The first `alloc` CTAs give the bars their
+// ranges of the list instead (their counts are complete).
+__global__ void __launch_bounds__(256) k_sunmap(BoardsDev b, SunFrame fr, SunAux aux,
+                                                unsigned long long* keys, int parts, int alloc,
+                                                Bins bins) {
+    if ((int)blockIdx.x < alloc) {
+        bin_alloc(bins, blockIdx.x);
+        return;
+    }
+    __shared__ SunBoard s_board[8];
+    __shared__ int s_tile[8 * 32], s_of[8 * 32], s_n[2];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int g = (blockIdx.x - alloc) * 8 + w;
+    const int i = g % b.n, part = g / b.n;  // the CTA's warps are on different boards
+    SunBoard s;
+    s.tiles = 0;
+    if (part < parts)
+        s = aux.boards ? reinterpret_cast<const SunBoard*>(aux.boards)[i] : sun_board(b, fr, i);
+    if (lane == 0) s_board[w] = s;
+    if (threadIdx.x == 0) s_n[0] = s_n[1] = 0;
+    const float span = fr.hi - fr.lo, sx = span / (float)fr.W, sy = span / (float)fr.H;
+    const float slack = sun_slack(fr);
+    const int wt = (fr.W + SUN_TW - 1) / SUN_TW;
+    int t0 = part;
+    // rounds of 32 tiles a warp; the tiles to look at are shared out over the CTA
+    for (int round = 0; __syncthreads_or(t0 < s.tiles); round ^= 1) {
+        // this lane's tile: whether the disc (widened by a texel) meets it, and
+        // the board may be in front of what the tile is bound to hold.  The
+        // board's depths there are at least sqrt(xm^2 + ym^2 + dz_min^2)
+        const int t = t0 + parts * lane;
+        bool live = t < s.tiles;
+        int at = 0;
+        if (live) {
+            const SunTile q = sun_tile(s, fr, sx, sy, t);
+            at = q.ty << 16 | q.tx;
+            const float dx = fmaxf(fmaxf(q.x0 - s.cv.x, s.cv.x - q.x1) - sx - slack, 0.f);
+            const float dy = fmaxf(fmaxf(q.y0 - s.cv.y, s.cv.y - q.y1) - sy - slack, 0.f);
+            live = dx * dx + dy * dy <= 1.0001f * (s.r * s.r);
+            if (live && aux.bound) {
+                const float xm = fmaxf(fmaxf(q.x0, -q.x1) - slack, 0.f);
+                const float ym = fmaxf(fmaxf(q.y0, -q.y1) - slack, 0.f);
+                const float bound = __uint_as_float(__ldg(aux.bound + q.ty * wt + q.tx));
+                // (no bound is a NaN: nothing loses)
+                live = !(bound * bound < (xm * xm + ym * ym + s.dz2_min) * (1.0f - 0x1p-18f));
+            }
+        }
+        const unsigned todo = __ballot_sync(0xffffffffu, live);
+        int base = 0;
+        if (lane == 0 && todo) base = atomicAdd(&s_n[round], __popc(todo));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (live) {
+            const int e = base + __popc(todo & ((1u << lane) - 1u));
+            s_tile[e] = at;
+            s_of[e] = w;
+        }
+        t0 += 32 * parts;
         __syncthreads();
-    }
-    const float r2 = 1.0001f * (r * r);
-    // the surface offset dz = (cv.z + r * prof) + near_z over prof in [0, 1]
-    // spans [dz_lo, dz_hi] (rounded steps are monotone): its smallest square
-    float dz2_min = 0.0f;
-    {
-        const float dz_lo = fadd(cv.z, fr.near_z), dz_hi = fadd(fadd(cv.z, r), fr.near_z);
-        if (dz_lo > 0.0f) dz2_min = fmul(dz_lo, dz_lo);
-        else if (dz_hi < 0.0f) dz2_min = fmul(dz_hi, dz_hi);
-    }
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-    const float span = fr.hi - fr.lo;
-    for (int row = warp; row < ny; row += nwarps) {
-        const int tj = ja + row;
-        const float yv = tabbed ? s_y[row] : texel_coord(fr.lo, fr.hi, tj, fr.H);
-        const float ey = yv - cv.y;
-        const float rem = r2 - ey * ey;
-        if (!(rem >= 0.f)) continue;  // the whole row is outside the disc
-        // the chord's texels, one texel of margin each side, within the box
-        const float w = sqrtf(rem);
-        int ca = (int)fmaxf(floorf((cv.x - w - fr.lo) / span * (float)fr.W - 0.5f) - 1.0f,
-                            (float)ia);
-        int cb = (int)fminf(ceilf((cv.x + w - fr.lo) / span * (float)fr.W - 0.5f) + 1.0f,
-                            (float)ib);
-        unsigned long long* krow = keys + (size_t)tj * fr.W;
-        for (int ti = ca + lane; ti <= cb; ti += 32) {
-            const float xv = sun_x(fr, s_x, tabbed, ia, ti);
-            // texels well outside the disc (d^2 > 1.0001 r^2, where the exact
-            // profile test cannot pass) skip the square roots and the division
-            {
-                const float ex = xv - cv.x;
-                if (ex * ex + ey * ey > r2) continue;
+        const int n = s_n[round];
+        if (threadIdx.x == 0) s_n[round ^ 1] = 0;
+        for (int e0 = w; e0 < n; e0 += 8 * SUN_AHEAD) {
+            // some tiles at a time: their current depths in flight together
+            unsigned long long cur[SUN_AHEAD];
+            int at_x[SUN_AHEAD], at_y[SUN_AHEAD];
+#pragma unroll
+            for (int u = 0; u < SUN_AHEAD; ++u) {
+                const int e = e0 + 8 * u;
+                cur[u] = 0ull;
+                at_x[u] = -1;
+                at_y[u] = 0;
+                if (e >= n) continue;
+                const SunBoard& o = s_board[s_of[e]];
+                const int ti = (s_tile[e] & 0xFFFF) * SUN_TW + (lane & 7);
+                const int tj = (s_tile[e] >> 16) * SUN_TH + (lane >> 3);
+                if (ti < o.ia || ti > o.ib || tj < o.ja || tj > o.jb) continue;
+                at_x[u] = ti;
+                at_y[u] = tj;
+                cur[u] = *(volatile unsigned long long*)(keys + (size_t)tj * fr.W + ti);
             }
-            unsigned long long* k = krow + ti;
-            // values only decrease, so a stale read can only make the tests
-            // below pass (never skip a winner)
-            const unsigned long long cur = *(volatile unsigned long long*)k;
-            // a certain loser skips the square roots and the division: this
-            // board's depth here is at least sqrt(xy2 + dz_min^2) (every step
-            // of the depth is monotone in |dz|), and a current depth whose
-            // square is below that by 2^-20 relative is strictly smaller as a
-            // float; an empty texel (all ones, a NaN) never skips
-            {
+#pragma unroll
+            for (int u = 0; u < SUN_AHEAD; ++u) {
+                if (at_x[u] < 0) continue;
+                const int of = s_of[e0 + 8 * u];
+                const SunBoard& o = s_board[of];
+                const float3 cv = o.cv;
+                const float r = o.r;
+                const float xv = aux.x ? aux.x[at_x[u]] : texel_coord(fr.lo, fr.hi, at_x[u], fr.W);
+                const float yv = aux.y ? aux.y[at_y[u]] : texel_coord(fr.lo, fr.hi, at_y[u], fr.H);
+                // texels well outside the disc (d^2 > 1.0001 r^2, where the exact
+                // profile test cannot pass) and certain losers skip the roots and
+                // the division: every step of the depth is monotone in |dz|, and a
+                // current depth whose square is below the smallest possible one by
+                // 2^-20 relative is strictly smaller as a float; an empty texel
+                // (all ones, a NaN) never skips.  Values only decrease, so a stale
+                // key can only make the tests pass (never skip a winner)
+                const float ex = xv - cv.x, ey = yv - cv.y;
+                if (ex * ex + ey * ey > 1.0001f * (r * r)) continue;
                 const float xy2 = fadd(fmul(xv, xv), fmul(yv, yv));
-                const float cd = __uint_as_float((unsigned)(cur >> 32));
-                if (cd * cd < fadd(xy2, dz2_min) * (1.0f - 0x1p-20f)) continue;
+                const float cd = __uint_as_float((unsigned)(cur[u] >> 32));
+                if (cd * cd < fadd(xy2, o.dz2_min) * (1.0f - 0x1p-20f)) continue;
+                float zs, depth;
+                if (!sun_fragment(xv, yv, cv, r, fr.near_z, zs, depth)) continue;
+                const unsigned id = (unsigned)((blockIdx.x - alloc) * 8 + of) % (unsigned)b.n;
+                const unsigned long long key =
+                    ((unsigned long long)__float_as_uint(depth) << 32) | id;
+                if (key < cur[u]) atomicMin(keys + (size_t)at_y[u] * fr.W + at_x[u], key);
             }
-            float zs, depth;
-            if (!sun_fragment(xv, yv, cv, r, fr.near_z, zs, depth)) continue;
-            unsigned long long key =
-                ((unsigned long long)__float_as_uint(depth) << 32) | (unsigned)i;
-            if (key < cur) atomicMin(k, key);
         }
     }
 }
@@ -325,40 +480,51 @@ __global__ void __launch_bounds__(256) k_sunmap(BoardsDev b, SunFrame fr,
 
 struct HiParams {
     float wmin[3], range[3];
+    float inv_range[3];  // exact when pow2: every extent is a power of two
+    bool pow2;
     float fD, offset;
     int D;
     int nb;            // bricks per axis
     uint8_t* hl;       // per-brick highlight flags (NULL: none)
 };
 
-__device__ __forceinline__ bool voxel_index(const HiParams& hp, float x, float y, float z,
-                                            int& o, int& brick) {
-    float c[3] = {x, y, z};
-    int id[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        float t = fdiv(fsub(c[a], hp.wmin[a]), hp.range[a]);
-        float v = fmul(hp.fD, t);
-        if (!(v > -1.0f && v < hp.fD)) return false;
-        id[a] = __float2int_rz(v);  // ivec3(): truncation toward zero
-    }
-    o = (id[2] * hp.D + id[1]) * hp.D + id[0];
-    brick = ((id[2] / CG_BRICK) * hp.nb + id[1] / CG_BRICK) * hp.nb + id[0] / CG_BRICK;
-    return true;
+__device__ __forceinline__ int voxel_index(const HiParams& hp, int a, float c) {
+    const float s = fsub(c, hp.wmin[a]);
+    // (a division by a power of two is the multiplication by its inverse)
+    const float t = hp.pow2 ? fmul(s, hp.inv_range[a]) : fdiv(s, hp.range[a]);
+    const float v = fmul(hp.fD, t);
+    if (!(v > -1.0f && v < hp.fD)) return -1;
+    return __float2int_rz(v);  // ivec3(): truncation toward zero
 }
 
 // One highlight store: the voxel's mask byte and, when flags are kept, its
-// brick's flag.
-__device__ __forceinline__ void mark(const HiParams& hp, uint8_t* mask, int vi, int brick) {
-    if (!CG_IN_BOUNDS(vi, (size_t)hp.D * hp.D * hp.D)) return;
+// brick's flag (unless that is `done`, flagged by the caller); returns the brick.
+__device__ __forceinline__ int mark(const HiParams& hp, uint8_t* mask, int x, int y, int z,
+                                    int done) {
+    const int vi = (z * hp.D + y) * hp.D + x;
+    const int brick = ((z / CG_BRICK) * hp.nb + y / CG_BRICK) * hp.nb + x / CG_BRICK;
+    if (!CG_IN_BOUNDS(vi, (size_t)hp.D * hp.D * hp.D)) return done;
     mask[vi] = 1;
-    if (hp.hl && CG_IN_BOUNDS(brick, (size_t)hp.nb * hp.nb * hp.nb)) hp.hl[brick] = 1;
+    if (hp.hl && brick != done && CG_IN_BOUNDS(brick, (size_t)hp.nb * hp.nb * hp.nb))
+        hp.hl[brick] = 1;
+    return brick;
 }
 
-__global__ void k_highlight(BoardsDev b, SunFrame fr, const unsigned long long* keys,
-                            float4* posmap, HiParams hp, uint8_t* mask) {
-    const int ti = blockIdx.x * blockDim.x + threadIdx.x;
-    const int tj = blockIdx.y * blockDim.y + threadIdx.y;
+// CTAs of 32 x 8 texels.  The first `fill` CTAs do not store highlights: they
+// fill the bars' lists, a warp per board (short, latency-bound work that costs
+// little beside the stores; 0: no bins).
+__global__ void __launch_bounds__(256) k_highlight(BoardsDev b, SunFrame fr,
+                                                   const unsigned long long* keys, float4* posmap,
+                                                   HiParams hp, uint8_t* mask, int fill,
+                                                   Bins bins) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if ((int)blockIdx.x < fill) {
+        bin_walk<true>(b, hp.D, bins, blockIdx.x * 8 + warp, lane);
+        return;
+    }
+    const int tx = (fr.W + 31) / 32, block = blockIdx.x - fill;
+    const int ti = (block % tx) * 32 + lane;
+    const int tj = (block / tx) * 8 + warp;
     if (ti >= fr.W || tj >= fr.H) return;
     const size_t idx = (size_t)tj * fr.W + ti;
     unsigned long long key = keys[idx];
@@ -379,15 +545,25 @@ __global__ void k_highlight(BoardsDev b, SunFrame fr, const unsigned long long* 
         p[a] = fadd(fadd(fadd(fmul(xv, fr.right[a]), fmul(yv, fr.up[a])), fmul(zs, -fr.fwd[a])),
                     fr.eye[a]);
     posmap[idx] = make_float4(p[0], p[1], p[2], 1.0f);
+    // the voxels of the point and of the eight points offset from it: per axis
+    // three coordinates, the corners' two often in one voxel (stored once)
     const float o = hp.offset;
-    int vi, bk;
-    if (voxel_index(hp, p[0], p[1], p[2], vi, bk)) mark(hp, mask, vi, bk);
+    int id[3], lo[3], hi[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        id[a] = voxel_index(hp, a, p[a]);
+        hi[a] = voxel_index(hp, a, fadd(p[a], o));
+        lo[a] = voxel_index(hp, a, fsub(p[a], o));
+        if (lo[a] == hi[a]) lo[a] = -1;
+    }
+    int own = -1;
+    if (id[0] >= 0 && id[1] >= 0 && id[2] >= 0) own = mark(hp, mask, id[0], id[1], id[2], -1);
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-        float x = (k & 4) ? fsub(p[0], o) : fadd(p[0], o);
-        float y = (k & 2) ? fsub(p[1], o) : fadd(p[1], o);
-        float z = (k & 1) ? fsub(p[2], o) : fadd(p[2], o);
-        if (voxel_index(hp, x, y, z, vi, bk)) mark(hp, mask, vi, bk);
+        const int x = (k & 4) ? lo[0] : hi[0], y = (k & 2) ? lo[1] : hi[1],
+                  z = (k & 1) ? lo[2] : hi[2];
+        if (x < 0 || y < 0 || z < 0 || (x == id[0] && y == id[1] && z == id[2])) continue;
+        mark(hp, mask, x, y, z, own);
     }
 }
 
@@ -575,7 +751,7 @@ __global__ void __launch_bounds__(64) k_splat(BoardsDev b, Bins bins, const uint
         }
     }
     const uint32_t beg = bins.offset[blockIdx.x];
-    const uint32_t n = bins.offset[blockIdx.x + 1] - beg;
+    const uint32_t n = bins.count[blockIdx.x];
     if (!COV && n == 0u && (hlm | dirtym) == 0u) return;
     if (n > 0u) {
         const float fx = (float)lx, fy = (float)ly;
@@ -1066,12 +1242,6 @@ __global__ void k_count_active(const uint32_t* count, const uint8_t* mask, size_
 
 }  // namespace
 
-cudaError_t launch_bin_count(const BoardsDev& b, int D, Bins bins, cudaStream_t st) {
-    if (b.n == 0) return cudaSuccess;
-    k_bin_count<<<(b.n + 3) / 4, 128, 0, st>>>(b, D, bins);  // one warp per board
-    return cudaGetLastError();
-}
-
 cudaError_t launch_bin_scan(Bins bins, cudaStream_t st) {
     // the shared-memory attribute is set once per device (atomics keep
     // concurrent host threads well-defined)
@@ -1090,37 +1260,76 @@ cudaError_t launch_bin_scan(Bins bins, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_bin_fill(const BoardsDev& b, int D, Bins bins, cudaStream_t st) {
-    if (b.n == 0) return cudaSuccess;
-    k_bin_fill<<<(b.n + 3) / 4, 128, 0, st>>>(b, D, bins);
-    return cudaGetLastError();
-}
+
+// Warps per board: a few thousand in all, so that a few large boards fill the GPU,
+// no more, as each sets its board up.  Sun stage, us, for (8192, 32768),
+// (8192, 16384) and (16384, 65536) warps in the two passes: 64^3 of 1024 boards
+// 42, 36 and 58, 256^3 of 4096 55, 53 and 66, 512^3 of 16384 118, 120 and 125.
+static int sun_parts(int n, int warps) { return std::min(64, std::max(1, warps / n)); }
+static int sun_blocks(int n, int parts) { return (int)(((long long)n * parts + 7) / 8); }
+constexpr int BOUND_W = 8192, MAP_W = 16384;
 
 cudaError_t launch_sunmap(const BoardsDev& b, const SunFrame& fr, uint64_t* keys,
                           cudaStream_t st) {
     if (b.n == 0) return cudaSuccess;
-    k_sunmap<<<b.n, 256, 0, st>>>(b, fr, reinterpret_cast<unsigned long long*>(keys));
+    const int parts = sun_parts(b.n, MAP_W);
+    k_sunmap<<<sun_blocks(b.n, parts), 256, 0, st>>>(
+        b, fr, SunAux{}, reinterpret_cast<unsigned long long*>(keys), parts, 0, Bins{});
     return cudaGetLastError();
+}
+
+cudaError_t launch_sun_pass(const BoardsDev& b, const SunFrame& fr, uint64_t* keys,
+                            const SunAux& aux, int D, const Bins& bins, cudaStream_t st) {
+    const int alloc = (bins.nbins + 255) / 256;
+    int parts = 1;
+    if (b.n > 0) {
+        parts = sun_parts(b.n, BOUND_W);
+        const int blocks = sun_blocks(b.n, parts), table = (std::max(fr.W, fr.H) + 255) / 256;
+        k_sun_bounds<<<blocks + table, 256, 0, st>>>(b, fr, aux, parts, blocks, D, bins);
+        parts = sun_parts(b.n, MAP_W);
+    }
+    k_sunmap<<<alloc + sun_blocks(b.n, parts), 256, 0, st>>>(
+        b, fr, aux, reinterpret_cast<unsigned long long*>(keys), parts, alloc, bins);
+    return cudaGetLastError();
+}
+
+static size_t sun_tiles(int W, int H) {
+    return (size_t)((W + SUN_TW - 1) / SUN_TW) * ((H + SUN_TH - 1) / SUN_TH);
+}
+
+size_t sun_aux_words(int W, int H) { return (sun_tiles(W, H) + W + H + 3) / 4 * 4; }
+
+SunAux sun_aux(uint32_t* words, void* boards, int W, int H) {
+    SunAux a;
+    a.bound = words;
+    a.x = reinterpret_cast<float*>(words) + sun_tiles(W, H);
+    a.y = a.x + W;
+    a.boards = boards;
+    return a;
 }
 
 cudaError_t launch_highlight(const BoardsDev& b, const SunFrame& fr, const uint64_t* keys,
                              float4* posmap, int D, const float wmin[3],
                              const float range[3], float offset, uint8_t* mask,
-                             uint8_t* hl_brick, cudaStream_t st) {
+                             uint8_t* hl_brick, const Bins* fill, cudaStream_t st) {
     HiParams hp;
     hp.nb = (D + CG_BRICK - 1) / CG_BRICK;
     hp.hl = hl_brick;
+    hp.pow2 = true;
     for (int a = 0; a < 3; ++a) {
         hp.wmin[a] = wmin[a];
         hp.range[a] = range[a];
+        hp.inv_range[a] = 1.0f / range[a];
+        int e;
+        hp.pow2 = hp.pow2 && std::frexp(range[a], &e) == 0.5f && e > -100 && e < 100;
     }
     hp.fD = (float)D;
     hp.offset = offset;
     hp.D = D;
-    dim3 blk(32, 8);
-    dim3 grd((fr.W + 31) / 32, (fr.H + 7) / 8);
-    k_highlight<<<grd, blk, 0, st>>>(b, fr, reinterpret_cast<const unsigned long long*>(keys),
-                                     posmap, hp, mask);
+    const int nfill = fill ? (b.n + 7) / 8 : 0;
+    const int blocks = nfill + (fr.W + 31) / 32 * ((fr.H + 7) / 8);
+    k_highlight<<<blocks, 256, 0, st>>>(b, fr, reinterpret_cast<const unsigned long long*>(keys),
+                                        posmap, hp, mask, nfill, fill ? *fill : Bins{});
     return cudaGetLastError();
 }
 
