@@ -283,6 +283,7 @@ void context_release(cg_context* ctx) {
     cudaStreamSynchronize(ctx->stream);
     cudaStreamSynchronize(ctx->side);
     ctx->image.release();
+    ctx->packed.release();
     ctx->noise.release();
     ctx->samples_pw.release();
     ctx->samples_gl.release();
@@ -1299,25 +1300,34 @@ extern "C" cg_status cg_march_samples(cg_context* ctx, const cg_volume* v, const
     if (st != CG_OK) return st;
     CG_LAUNCH(ctx, launch_march(desc_of(v), cd, tp, sb, s));
     const size_t regions = (size_t)((cam->width + 15) / 16) * ((cam->height + 15) / 16) * 8;
-    std::vector<unsigned> cnt(regions);
-    CG_CUDA(cudaMemcpyAsync(cnt.data(), sb.count, regions * 4, cudaMemcpyDeviceToHost, s));
+    // packed on the device and copied a piece at a time (a copy per region with
+    // samples took 4.8 ms for 480 x 270 and 62500 samples, all of it 0.20)
+    constexpr size_t piece = 1u << 20;
+    const size_t most = std::min(std::min((size_t)capacity, piece), regions * (size_t)sb.capacity);
+    const size_t o_pos = (regions + 1) * 8, o_w = o_pos + most * 12;
+    CG_CUDA(ctx->packed.ensure(o_w + most * 4));
+    char* base = ctx->packed.as<char>();
+    auto* off = reinterpret_cast<unsigned long long*>(base);
+    float* d_pos = reinterpret_cast<float*>(base + o_pos);
+    float* d_w = reinterpret_cast<float*>(base + o_w);
+    CG_LAUNCH(ctx, launch_sample_offsets(sb, (int)regions, off, s));
+    if (most)
+        CG_LAUNCH(ctx, launch_gather_samples(sb, off, (int)regions, 0, (unsigned)most, d_pos, d_w,
+                                             s));
+    unsigned long long total = 0;
+    CG_CUDA(cudaMemcpyAsync(&total, off + regions, 8, cudaMemcpyDeviceToHost, s));
     CG_CUDA(cudaStreamSynchronize(s));
-    size_t total = 0;
-    std::vector<float4> tmp;
-    for (size_t r = 0; r < regions; ++r) {
-        if (!cnt[r]) continue;
-        tmp.resize(cnt[r]);
-        CG_CUDA(cudaMemcpy(tmp.data(), sb.pos_w + r * (size_t)sb.capacity, cnt[r] * 16,
-                           cudaMemcpyDeviceToHost));
-        for (unsigned i = 0; i < cnt[r]; ++i, ++total) {
-            if (total >= (size_t)capacity) continue;
-            positions[3 * total] = tmp[i].x;
-            positions[3 * total + 1] = tmp[i].y;
-            positions[3 * total + 2] = tmp[i].z;
-            weights[total] = tmp[i].w;
-        }
+    const size_t want = std::min((size_t)total, (size_t)capacity);
+    for (size_t lo = 0; lo < want; lo += most) {
+        const size_t n = std::min(most, want - lo);
+        if (lo)
+            CG_LAUNCH(ctx, launch_gather_samples(sb, off, (int)regions, lo, (unsigned)n, d_pos,
+                                                 d_w, s));
+        CG_CUDA(cudaMemcpyAsync(positions + 3 * lo, d_pos, n * 12, cudaMemcpyDeviceToHost, s));
+        CG_CUDA(cudaMemcpyAsync(weights + lo, d_w, n * 4, cudaMemcpyDeviceToHost, s));
     }
-    *count = (int)std::min(total, (size_t)0x7FFFFFFF);
+    CG_CUDA(cudaStreamSynchronize(s));
+    *count = (int)std::min(total, 0x7FFFFFFFull);
     return CG_OK;
 }
 

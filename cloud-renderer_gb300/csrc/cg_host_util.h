@@ -94,6 +94,7 @@ struct cg_context {
     cudaEvent_t marks[32] = {};
     char mark_names[32][24] = {};
     DevBuf image;  // render target when the caller passes a host pointer
+    DevBuf packed;  // cg_march_samples: offsets and a piece of the packed samples
     // hash-noise lattice tables of the last (noise parameters, world box)
     DevBuf noise;
     bool noise_valid = false;

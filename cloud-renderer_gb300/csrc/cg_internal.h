@@ -372,6 +372,13 @@ struct TrainArgs {
 
 // The view march (writes the samples, the step tables and sb.alpha).
 cudaError_t launch_march(VolDesc vd, CamDesc cam, TraceParams tp, SampleBuf sb, cudaStream_t st);
+// The regions' first samples in region order (regions + 1 entries), and the
+// samples [lo, lo + n) of that order packed into positions (3n) and weights (n).
+cudaError_t launch_sample_offsets(const SampleBuf& sb, int regions, unsigned long long* off,
+                                  cudaStream_t st);
+cudaError_t launch_gather_samples(const SampleBuf& sb, const unsigned long long* off, int regions,
+                                  unsigned long long lo, unsigned n, float* positions,
+                                  float* weights, cudaStream_t st);
 // The surrogate's view march: also clears the shading status (4 words), lists
 // the regions with samples and writes the finished pixels of the others to dst.
 cudaError_t launch_march_mlp(VolDesc vd, CamDesc cam, TraceParams tp, SampleBuf sb, float4* dst,

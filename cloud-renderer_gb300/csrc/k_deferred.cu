@@ -372,6 +372,65 @@ __global__ void __launch_bounds__(128) k_accumulate(CamDesc cam, TraceParams tp,
     }
 }
 
+// First sample of every region in region order (off[regions] = their number):
+// one CTA, each thread a contiguous piece of the counts.
+__global__ void __launch_bounds__(1024) k_sample_offsets(const unsigned* count, int regions,
+                                                         unsigned long long* off) {
+    __shared__ unsigned long long s_warp[32];
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    const int per = (regions + 1023) / 1024;
+    const int a = min(regions, t * per), b = min(regions, a + per);
+    unsigned long long sum = 0ull;
+#pragma unroll 8
+    for (int r = a; r < b; ++r) sum += count[r];
+    unsigned long long x = sum;
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) s_warp[w] = x;
+    __syncthreads();
+    if (w == 0) {
+        unsigned long long v = s_warp[lane];
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long y = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += y;
+        }
+        s_warp[lane] = v;
+    }
+    __syncthreads();
+    unsigned long long at = x - sum + (w ? s_warp[w - 1] : 0ull);
+#pragma unroll 8
+    for (int r = a; r < b; ++r) {
+        off[r] = at;
+        at += count[r];
+    }
+    if (t == 1023) off[regions] = at;
+}
+
+// Samples [lo, lo + n) of that order, packed: a warp per region, bound by the
+// read of 16 bytes a sample.
+__global__ void __launch_bounds__(256) k_gather_samples(SampleBuf sb, const unsigned long long* off,
+                                                        int regions, unsigned long long lo,
+                                                        unsigned n, float* positions,
+                                                        float* weights) {
+    const int region = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (region >= regions) return;
+    const unsigned long long a = off[region], b = off[region + 1];
+    if (b <= lo || a >= lo + n) return;
+    const float4* pw = sb.pos_w + (size_t)region * sb.capacity;
+    const unsigned long long end = min(b, lo + n);
+    for (unsigned long long i = max(a, lo) + lane; i < end; i += 32) {
+        if (!CG_IN_BOUNDS((size_t)region * sb.capacity + (i - a), sb.nslots)) continue;
+        const float4 s = pw[i - a];
+        const size_t o = (size_t)(i - lo);
+        positions[3 * o] = s.x;
+        positions[3 * o + 1] = s.y;
+        positions[3 * o + 2] = s.z;
+        weights[o] = s.w;
+    }
+}
+
 }  // namespace
 
 static int regions_of(const CamDesc& cam) { return ((cam.W + 15) / 16) * ((cam.H + 15) / 16) * 8; }
@@ -398,6 +457,20 @@ cudaError_t launch_march_mlp(VolDesc vd, CamDesc cam, TraceParams tp, SampleBuf 
     cudaError_t e = cudaMemsetAsync(sb.flat_total, 0, 2 * sizeof(unsigned), st);
     if (e != cudaSuccess) return e;
     k_march<0, true><<<march_grid(cam), 32 * MARCH_WARPS, 0, st>>>(vd, cam, tp, sb, dst, status);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_sample_offsets(const SampleBuf& sb, int regions, unsigned long long* off,
+                                  cudaStream_t st) {
+    k_sample_offsets<<<1, 1024, 0, st>>>(sb.count, regions, off);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_gather_samples(const SampleBuf& sb, const unsigned long long* off, int regions,
+                                  unsigned long long lo, unsigned n, float* positions,
+                                  float* weights, cudaStream_t st) {
+    k_gather_samples<<<(regions + 7) / 8, 256, 0, st>>>(sb, off, regions, lo, n, positions,
+                                                        weights);
     return cudaGetLastError();
 }
 
