@@ -61,8 +61,9 @@ void noise_map(uint32_t seed, float* out) {
 }
 
 cg_status check_compat(const cg_compat_params* p) {
-    CG_CHECK(p->num_octaves >= 0 && p->num_octaves <= 16, CG_ERR_OUT_OF_RANGE,
-             "compat params: num_octaves %d not in [0, 16]", p->num_octaves);
+    CG_CHECK(p->num_octaves >= 0 && p->num_octaves <= CG_COMPAT_MAX_OCTAVES, CG_ERR_OUT_OF_RANGE,
+             "compat params: num_octaves %d not in [0, %d]", p->num_octaves,
+             CG_COMPAT_MAX_OCTAVES);
     CG_CHECK(p->min_noise_steps >= 2 && p->max_noise_steps >= p->min_noise_steps &&
                  p->max_noise_steps <= 4096,
              CG_ERR_OUT_OF_RANGE,
@@ -151,14 +152,25 @@ extern "C" cg_status cg_render_compat(cg_context* ctx, const cg_volume* v, const
     if (!ctx->compat_noise_valid || ctx->compat_seed != params->noise_seed) {
         std::vector<float> rgba((size_t)NOISE_N * NOISE_N * NOISE_N * 4);
         noise_map(params->noise_seed, rgba.data());
-        std::vector<float> ga(rgba.size() / 2);
-        for (size_t i = 0; i < rgba.size() / 4; ++i) {
-            ga[2 * i] = rgba[4 * i + 1];
-            ga[2 * i + 1] = rgba[4 * i + 3];
-        }
+        std::vector<float> cells(rgba.size() * 4);
+        constexpr size_t W = NOISE_N - 1;
+        auto at = [&](size_t x, size_t y, size_t z, int c) {
+            return rgba[(((z & W) * NOISE_N + (y & W)) * NOISE_N + (x & W)) * 4 + c];
+        };
+        float* o = cells.data();
+        for (size_t z = 0; z < NOISE_N; ++z)
+            for (size_t y = 0; y < NOISE_N; ++y)
+                for (size_t x = 0; x < NOISE_N; ++x)
+                    for (size_t k = 0; k < 4; ++k, o += 4)
+                        for (int c = 0; c < 2; ++c) {
+                            const float a = at(x, y + (k & 1), z + (k >> 1), 2 * c + 1);
+                            o[c] = a;
+                            o[2 + c] = at(x + 1, y + (k & 1), z + (k >> 1), 2 * c + 1) - a;
+                        }
         CG_CUDA(cudaStreamSynchronize(s));
-        CG_CUDA(ctx->compat_noise.ensure(ga.size() * 4));
-        CG_CUDA(cudaMemcpy(ctx->compat_noise.p, ga.data(), ga.size() * 4, cudaMemcpyHostToDevice));
+        CG_CUDA(ctx->compat_noise.ensure(cells.size() * 4));
+        CG_CUDA(cudaMemcpy(ctx->compat_noise.p, cells.data(), cells.size() * 4,
+                           cudaMemcpyHostToDevice));
         ctx->compat_noise_valid = true;
         ctx->compat_seed = params->noise_seed;
     }
@@ -182,14 +194,11 @@ extern "C" cg_status cg_render_compat(cg_context* ctx, const cg_volume* v, const
     P.step_size = params->step_size;
     P.noise_opacity = params->noise_opacity;
     P.octaves = params->num_octaves;
-    P.freq_step = params->freq_step;
-    P.pers_step = params->pers_step;
     P.inv_adjust = 1.0f / params->adjust_size;
     P.min_steps = params->min_noise_steps;
     P.max_steps = params->max_noise_steps;
     P.min_color = params->min_noise_color;
     P.color_scale = params->noise_color_scale;
-    for (int a = 0; a < 3; ++a) P.off[a] = params->octave_offsets[a];
     for (int a = 0; a < 4; ++a) P.clear[a] = params->clear_color[a];
     P.cutoff = params->transmittance_cutoff;
     const double sx = v->sun_dir[0], sy = v->sun_dir[1], sz = v->sun_dir[2];
@@ -197,7 +206,23 @@ extern "C" cg_status cg_render_compat(cg_context* ctx, const cg_volume* v, const
     P.sun[0] = (float)(sx / sn);
     P.sun[1] = (float)(sy / sn);
     P.sun[2] = (float)(sz / sn);
-    P.noise = ctx->compat_noise.as<const float2>();
+    P.noise = ctx->compat_noise.as<const ulonglong2>();
+    {
+        // below noise_reach, |(c + off) fr N - 1/2| stays under 2^21 in every octave
+        double top = 1.0, off = 0.0;
+        float fr = 1.f, pe = 1.f;
+        for (int k = 0; k < P.octaves; ++k) {
+            auto& o = P.oct[k >> 1];
+            o.off[k & 1] = k < 3 ? params->octave_offsets[k] : 0.f;
+            o.fr[k & 1] = fr;
+            o.pe[k & 1] = pe;
+            off = std::max(off, std::fabs((double)o.off[k & 1]));
+            top = std::max(top, std::fabs((double)fr));
+            fr *= params->freq_step;
+            pe *= params->pers_step;
+        }
+        P.noise_reach = (float)std::max(0.0, 2.0e6 / (NOISE_N * top) - off);
+    }
     // traceCone's schedule (conetrace_frag.glsl:64-79): the reference cone mode
     TraceParams tp;
     std::memset(&tp, 0, sizeof(tp));
@@ -211,28 +236,28 @@ extern "C" cg_status cg_render_compat(cg_context* ctx, const cg_volume* v, const
     const ConeSchedule cs = make_cone_schedule(vd, tp);
     // tile lists: counts, scan, total (one synchronisation), fill
     const int ntiles = P.tiles_x * P.tiles_y;
-    const size_t cnt_words = ((size_t)ntiles + 3) & ~(size_t)3;
-    const size_t off_words = ((size_t)ntiles + 1 + 3) & ~(size_t)3;
+    const size_t words = ((size_t)ntiles + 1 + 3) & ~(size_t)3;
     const size_t nb = (size_t)(v->n > 0 ? v->n : 1);
     CG_CUDA(ctx->compat_rect.ensure(nb * 16));
     CG_CUDA(ctx->compat_key.ensure(nb * 4));
-    // counts | offsets | cursors (u32, 16-byte aligned regions) | 64-bit pair total
-    CG_CUDA(ctx->compat_tiles.ensure((cnt_words + off_words + cnt_words) * 4 + 16));
+    // 64-bit pair total, longest list | counts and their total | offsets | cursors
+    CG_CUDA(ctx->compat_tiles.ensure((4 + 3 * words) * 4));
     CG_CUDA(ctx->compat_total.ensure(16));
+    uint32_t* base = ctx->compat_tiles.as<uint32_t>();
+    unsigned long long* pairs64 = reinterpret_cast<unsigned long long*>(base);
+    uint32_t* most_dev = base + 2;
     Bins bins{};
     bins.nbins = ntiles;
-    bins.count = ctx->compat_tiles.as<uint32_t>();
-    bins.offset = bins.count + cnt_words;
-    bins.cursor = bins.offset + off_words;
-    unsigned long long* pairs64 = reinterpret_cast<unsigned long long*>(bins.cursor + cnt_words);
+    bins.count = base + 4;
+    bins.offset = bins.count + words;
+    bins.cursor = bins.offset + words;
     stage_begin(ctx, s);
-    CG_CUDA(cudaMemsetAsync(bins.count, 0, cnt_words * 4, s));
-    CG_CUDA(cudaMemsetAsync(pairs64, 0, 8, s));
+    CG_CUDA(cudaMemsetAsync(base, 0, (4 + words) * 4, s));
     CG_LAUNCH(ctx, launch_compat_count(P, ctx->compat_rect.as<int4>(), ctx->compat_key.as<float>(),
                                        bins.count, pairs64, s));
-    CG_LAUNCH(ctx, launch_bin_scan(bins, s));
+    CG_LAUNCH(ctx, launch_bin_alloc(bins, most_dev, s));
     uint64_t* total = reinterpret_cast<uint64_t*>(ctx->compat_total.p);
-    CG_CUDA(cudaMemcpyAsync(total, pairs64, 8, cudaMemcpyDeviceToHost, s));
+    CG_CUDA(cudaMemcpyAsync(total, pairs64, 16, cudaMemcpyDeviceToHost, s));
     CG_CUDA(cudaStreamSynchronize(s));
     // the per-tile offsets are 32-bit
     CG_CHECK(*total < 0xFFFFFFFFull, CG_ERR_OUT_OF_RANGE,
@@ -243,7 +268,7 @@ extern "C" cg_status cg_render_compat(cg_context* ctx, const cg_volume* v, const
                                       ctx->compat_key.as<const float>(), bins.cursor,
                                       ctx->compat_list.as<unsigned long long>(), s));
     stage_mark(ctx, s, "bin");
-    CG_LAUNCH(ctx, launch_compat_tiles(vd, cs, P, bins.offset,
+    CG_LAUNCH(ctx, launch_compat_tiles(vd, cs, P, bins, (uint32_t)total[1],
                                        ctx->compat_list.as<unsigned long long>(), out, s));
     stage_mark(ctx, s, "tiles");
     if (!out_on_device) {

@@ -437,7 +437,9 @@ bool sun_frame_for_box(const float position[3], float b0, float b1, const float 
 // ---- launchers (return cudaGetLastError of the launch) -------------------
 // Bar height of a volume's splat (k_voxelize.cu).
 int splat_bar(int dimension);
-cudaError_t launch_bin_scan(Bins bins, cudaStream_t st);
+// Disjoint ranges for the counts of bins.nbins (offset and cursor; count has one
+// more word, the total, zeroed before) and the largest count (*most, likewise).
+cudaError_t launch_bin_alloc(const Bins& bins, uint32_t* most, cudaStream_t st);
 cudaError_t launch_sunmap(const BoardsDev& b, const SunFrame& fr, uint64_t* keys,
                           cudaStream_t st);
 // Beside the keys of a sun map: per 8 x 4 texel tile an upper bound of the depth
@@ -517,6 +519,7 @@ cudaError_t launch_trace_batch(int fmt, int lanes_per_ray, int unroll, const Bat
 
 // ---- compat render (k_compat.cu) ------------------------------------------
 // The reference's billboard image formation; see cg_render_compat.
+constexpr int CG_COMPAT_MAX_OCTAVES = 16;
 constexpr int CG_COMPAT_TILE = 8;  // pixel tile edge
 struct CompatDev {
     CamDesc cam;
@@ -527,14 +530,20 @@ struct CompatDev {
     int show_quad, do_noise, do_cone;
     float step_size, noise_opacity;
     int octaves;
-    float freq_step, pers_step, inv_adjust;
+    float inv_adjust;
     int min_steps, max_steps;
     float min_color, color_scale;
-    float off[3];
+    // octaves 2i and 2i + 1: coordinate offset, frequency, weight
+    struct alignas(8) {
+        float off[2], fr[2], pe[2];
+    } oct[CG_COMPAT_MAX_OCTAVES / 2];
     float clear[4];
     float cutoff;
     float sun[3];
-    const float2* noise;   // green and alpha of the decoded 32^3 noise map
+    // the decoded 32^3 noise map's green and alpha, 64 bytes a cell: for each of
+    // its (z, y) corners the two values and the steps to the next texel along x
+    const ulonglong2* noise;
+    float noise_reach;     // sample coordinates below this reach no large cell number
 };
 // Per board: tile rectangle (x0, y0, x1, y1; empty when x0 > x1) and the
 // squared eye distance; per tile: the number of boards whose quad may cover it;
@@ -546,5 +555,5 @@ cudaError_t launch_compat_fill(const CompatDev& P, const int4* rect, const float
                                uint32_t* cursor, unsigned long long* list, cudaStream_t st);
 // Per tile: order its list by distance and blend its pixels front to back.
 cudaError_t launch_compat_tiles(const VolDesc& vd, const ConeSchedule& cs, const CompatDev& P,
-                                const uint32_t* offset, unsigned long long* list, float4* out,
-                                cudaStream_t st);
+                                const Bins& tiles, uint32_t most, unsigned long long* list,
+                                float4* out, cudaStream_t st);

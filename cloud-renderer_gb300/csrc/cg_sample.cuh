@@ -15,6 +15,52 @@ __device__ __forceinline__ float fp16_hi(uint32_t v) {
     return __half2float(__ushort_as_half((unsigned short)(v >> 16)));
 }
 
+// Two FP32 values in a register pair, and the operations on both at once (for
+// kernels bound by instructions).
+namespace pairs {
+typedef unsigned long long pair;
+__device__ __forceinline__ pair both(float v) {
+    pair r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ pair make(float lo, float hi) {
+    pair r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 halves(pair p) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ pair fma2(pair a, pair b, pair c) {
+    pair r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ pair sub2(pair a, pair b) {
+    pair r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ pair add2(pair a, pair b) {
+    pair r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ pair mul2(pair a, pair b) {
+    pair r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ pair add2_down(pair a, pair b) {
+    pair r;
+    asm("add.rm.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+}  // namespace pairs
+
 // One voxel's (R, G) at flat index idx.
 template <int FMT, bool WANT_G>
 __device__ __forceinline__ float2 fetch(const void* pyr, int idx) {
@@ -339,6 +385,89 @@ __device__ __forceinline__ float cone_quads(const VolDesc& vd, const ConeSchedul
     return tau + comp;
 }
 
+// Channel G of a texel.
+template <int FMT>
+__device__ __forceinline__ float fetch_light(const VolDesc& vd, int idx) {
+    if (!CG_IN_BOUNDS(idx, vd.nvox)) return 0.f;
+    if (FMT == 0) return __ldg(reinterpret_cast<const float*>(vd.pyr) + 4 * (size_t)idx + 1);
+    return __half2float(__ushort_as_half(
+        __ldg(reinterpret_cast<const unsigned short*>(vd.pyr) + 2 * (size_t)idx + 1)));
+}
+
+// tri<FMT, true, false, false>(...).y without its two paths: a coordinate
+// clamped to [0, N - 1] before the floor blends the same two texels (beyond an
+// edge, and on it, both are the edge's, so a weight of 0 gives the same value),
+// and a zero stride stands for the texel past the last.
+template <int FMT>
+__device__ __forceinline__ float tri_light(const VolDesc& vd, int l, float px, float py,
+                                           float pz) {
+    constexpr float MAGIC = 12582912.f;  // 1.5 * 2^23: floor and integer in one addition
+    constexpr int BIAS = 0x4B400000;
+    const int N = vd.dims[l];
+    const float sc = vd.lsc[l], last = (float)(N - 1);
+    const float x = fminf(fmaxf(px * sc - 0.5f, 0.f), last);
+    const float y = fminf(fmaxf(py * sc - 0.5f, 0.f), last);
+    const float z = fminf(fmaxf(pz * sc - 0.5f, 0.f), last);
+    const float mx = __fadd_rd(x, MAGIC), my = __fadd_rd(y, MAGIC), mz = __fadd_rd(z, MAGIC);
+    const float wx = x - (mx - MAGIC), wy = y - (my - MAGIC), wz = z - (mz - MAGIC);
+    const int ix = __float_as_int(mx) - BIAS, iy = __float_as_int(my) - BIAS,
+              iz = __float_as_int(mz) - BIAS;
+    const int dx = ix < N - 1 ? 1 : 0, dy = iy < N - 1 ? N : 0, dz = iz < N - 1 ? N * N : 0;
+    const int i0 = (int)vd.offs[l] + (iz * N + iy) * N + ix;
+    const int i1 = i0 + dy, i2 = i0 + dz, i3 = i1 + dz;
+    const float g[8] = {fetch_light<FMT>(vd, i0), fetch_light<FMT>(vd, i0 + dx),
+                        fetch_light<FMT>(vd, i1), fetch_light<FMT>(vd, i1 + dx),
+                        fetch_light<FMT>(vd, i2), fetch_light<FMT>(vd, i2 + dx),
+                        fetch_light<FMT>(vd, i3), fetch_light<FMT>(vd, i3 + dx)};
+    return lerp3(g, wx, wy, wz);
+}
+
+// tri_light at levels l and l + 1 together (one lane of each pair a level).
+template <int FMT>
+__device__ __forceinline__ float2 tri_light_pair(const VolDesc& vd, int l, float px, float py,
+                                                 float pz) {
+    using namespace pairs;
+    const pair magic = both(12582912.f), half = both(-0.5f);
+    constexpr int BIAS = 0x4B400000;
+    const int N[2] = {vd.dims[l], vd.dims[l + 1]};
+    const pair sc = make(vd.lsc[l], vd.lsc[l + 1]);
+    const float last[2] = {(float)(N[0] - 1), (float)(N[1] - 1)};
+    const float p[3] = {px, py, pz};
+    pair w[3];
+    int i[3][2];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const float2 u = halves(fma2(both(p[a]), sc, half));
+        const pair t = make(fminf(fmaxf(u.x, 0.f), last[0]), fminf(fmaxf(u.y, 0.f), last[1]));
+        const pair m = add2_down(t, magic);
+        w[a] = sub2(t, sub2(m, magic));
+        i[a][0] = (int)m - BIAS;
+        i[a][1] = (int)(m >> 32) - BIAS;
+    }
+    float g[8][2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const int n = N[q];
+        const int dx = i[0][q] < n - 1 ? 1 : 0, dy = i[1][q] < n - 1 ? n : 0,
+                  dz = i[2][q] < n - 1 ? n * n : 0;
+        const int i0 = (int)vd.offs[l + q] + (i[2][q] * n + i[1][q]) * n + i[0][q];
+        const int at[4] = {i0, i0 + dy, i0 + dz, i0 + dy + dz};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            g[2 * k][q] = fetch_light<FMT>(vd, at[k]);
+            g[2 * k + 1][q] = fetch_light<FMT>(vd, at[k] + dx);
+        }
+    }
+    pair x[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const pair a = make(g[2 * k][0], g[2 * k][1]);
+        x[k] = fma2(w[0], sub2(make(g[2 * k + 1][0], g[2 * k + 1][1]), a), a);
+    }
+    const pair y0 = fma2(w[1], sub2(x[1], x[0]), x[0]), y1 = fma2(w[1], sub2(x[3], x[2]), x[2]);
+    return halves(fma2(w[2], sub2(y1, y0), y0));
+}
+
 // The reference's weighted sum of the light channel (mode 1, clamp to edge).
 template <int FMT>
 __device__ __forceinline__ float cone_reference(const VolDesc& vd, const ConeSchedule& cs,
@@ -346,10 +475,17 @@ __device__ __forceinline__ float cone_reference(const VolDesc& vd, const ConeSch
                                                 float sz) {
     float acc = 0.f;
     for (int i = 0; i < cs.steps; ++i) {
-        const float h = cs.st[i].h;
-        float2 c = quad_split<FMT, true, false, false>(vd, vx + h * sx, vy + h * sy, vz + h * sz,
-                                                       cs.st[i].l0, cs.st[i].frac);
-        acc += c.y * cs.st[i].w;
+        const float h = cs.st[i].h, fr = cs.st[i].frac;
+        const int l = cs.st[i].l0;
+        const float x = vx + h * sx, y = vy + h * sy, z = vz + h * sz;
+        float g;
+        if (fr > 0.f && l + 1 < vd.L) {
+            const float2 q = tri_light_pair<FMT>(vd, l, x, y, z);
+            g = q.x + fr * (q.y - q.x);
+        } else {
+            g = tri_light<FMT>(vd, l, x, y, z);
+        }
+        acc += g * cs.st[i].w;
     }
     return acc;
 }

@@ -6,37 +6,41 @@
 // fragment with conetrace_frag.glsl:122-201 and blends back to front
 // (SRC_ALPHA, ONE_MINUS_SRC_ALPHA, main.cpp:94-95) after sorting the boards by
 // distance on the CPU (CloudVolume.cpp:65-82).  Here:
-//   count  one warp per board: the quad's conservative pixel rectangle, its
+//   count  some warps per board: the quad's conservative pixel rectangle, its
 //          8x8 tiles (atomic per-tile counts) and the squared eye distance;
-//   scan   the per-tile counts (k_bin_scan);
-//   fill   one warp per board: (distance bits << 32 | board) into each
-//          tile's list;
-//   tiles  one 256-thread CTA per 8x8 tile: sorts its list (bitonic, in
-//          shared memory up to 4096 entries, in place in global memory
-//          beyond); four threads per pixel blend a quarter of the list each
-//          front to back, C += T a src, T *= 1 - a, and the quarters combine
-//          in order (the over operator is associative), which equals the
-//          back-to-front blend; a thread stops once its T falls below the
-//          cutoff, a warp once all its threads have.
+//   alloc  each tile's range of the list (k_bin_alloc);
+//   fill   (distance bits << 32 | board) into each tile's list;
+//   tiles  two 128-thread CTAs per 8x8 tile: sort its list (by ranks up to 128
+//          entries, bitonic in shared memory up to 4096; longer ones are sorted
+//          in place in global memory before); four threads per pixel blend a
+//          quarter of the list each front to back, C += T a src, T *= 1 - a, and
+//          the quarters combine in order (the over operator is associative),
+//          which equals the back-to-front blend; a thread stops once its T falls
+//          below the cutoff, a warp once all its threads have.
 // The quad is perpendicular to the view axis f, so the fragment of pixel ray
 // d (d.f = 1) is the plane point e + z d with z = (c - e).f; the quad covers
 // the pixel when both plane coordinates (x, y) = ((p - c).s, (p - c).u) / r
 // lie in [-1, 1].
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "cg_internal.h"
 #include "cg_sample.cuh"
 
 namespace {
 
-constexpr int CAP = 4096;      // sort keys held in shared memory per tile
+using namespace cgs::pairs;
+
+constexpr int CAP = 4096;      // most sort keys held in shared memory per tile
 constexpr int NOISE_N = 32;    // noise map edge (ConeTraceShader.cpp:12)
 
-// One warp per board: lane 0 derives the board's tile rectangle, the lanes
+// `parts` warps per board: lane 0 derives the board's tile rectangle, the lanes
 // split its tiles for the per-tile count.
-__global__ void k_compat_count(CompatDev P, int4* rect, float* key, uint32_t* tile_count,
-                               unsigned long long* pairs) {
-    const int b = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+__global__ void k_compat_count(CompatDev P, int parts, int4* rect, float* key,
+                               uint32_t* tile_count, unsigned long long* pairs) {
+    const int g = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    const int b = g / parts, part = g % parts;
     const int lane = threadIdx.x & 31;
     if (b >= P.n) return;
     int4 R = make_int4(1, 1, 0, 0);
@@ -45,7 +49,7 @@ __global__ void k_compat_count(CompatDev P, int4* rect, float* key, uint32_t* ti
         const float4 c = P.cwr[b];
         const float dx = c.x - cam.eye[0], dy = c.y - cam.eye[1], dz = c.z - cam.eye[2];
         const float z = dx * cam.f[0] + dy * cam.f[1] + dz * cam.f[2];
-        key[b] = dx * dx + dy * dy + dz * dz;
+        if (part == 0) key[b] = dx * dx + dy * dy + dz * dz;
         if (z > P.near_z && z < 2500.f && c.w > 0.f) {
             // plane coordinates of the centre and the half extent at unit depth
             const float xs = (dx * cam.s[0] + dy * cam.s[1] + dz * cam.s[2]) / z;
@@ -68,7 +72,7 @@ __global__ void k_compat_count(CompatDev P, int4* rect, float* key, uint32_t* ti
                 R = make_int4(i0 / CG_COMPAT_TILE, j0 / CG_COMPAT_TILE, i1 / CG_COMPAT_TILE,
                               j1 / CG_COMPAT_TILE);
         }
-        rect[b] = R;
+        if (part == 0) rect[b] = R;
     }
     R.x = __shfl_sync(0xffffffffu, R.x, 0);
     R.y = __shfl_sync(0xffffffffu, R.y, 0);
@@ -76,15 +80,17 @@ __global__ void k_compat_count(CompatDev P, int4* rect, float* key, uint32_t* ti
     R.w = __shfl_sync(0xffffffffu, R.w, 0);
     const int nx = R.z - R.x + 1, ny = R.w - R.y + 1;
     if (nx <= 0 || ny <= 0) return;
-    if (lane == 0) atomicAdd(pairs, (unsigned long long)nx * (unsigned long long)ny);
-    for (int t = lane; t < nx * ny; t += 32)
+    if (lane == 0 && part == 0)
+        atomicAdd(pairs, (unsigned long long)nx * (unsigned long long)ny);
+    for (int t = part * 32 + lane; t < nx * ny; t += 32 * parts)
         atomicAdd(tile_count + (R.y + t / nx) * P.tiles_x + R.x + t % nx, 1u);
 }
 
-// One warp per board: the lanes split its tiles.
-__global__ void k_compat_fill(CompatDev P, const int4* rect, const float* key, uint32_t* cursor,
-                              unsigned long long* list) {
-    const int b = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+// `parts` warps per board: the lanes split its tiles.
+__global__ void k_compat_fill(CompatDev P, int parts, const int4* rect, const float* key,
+                              uint32_t* cursor, unsigned long long* list) {
+    const int g = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    const int b = g / parts, part = g % parts;
     const int lane = threadIdx.x & 31;
     if (b >= P.n) return;
     const int4 R = rect[b];
@@ -92,7 +98,7 @@ __global__ void k_compat_fill(CompatDev P, const int4* rect, const float* key, u
     if (nx <= 0 || ny <= 0) return;
     const unsigned long long k =
         ((unsigned long long)__float_as_uint(key[b]) << 32) | (unsigned long long)(unsigned)b;
-    for (int t = lane; t < nx * ny; t += 32) {
+    for (int t = part * 32 + lane; t < nx * ny; t += 32 * parts) {
         const uint32_t slot = atomicAdd(cursor + (R.y + t / nx) * P.tiles_x + R.x + t % nx, 1u);
         list[slot] = k;
     }
@@ -138,34 +144,66 @@ __device__ void sort_keys(Ptr a, int m) {
     }
 }
 
-// texture(noiseMap, q).ga: LINEAR with REPEAT at normalised coordinates (the
-// fragment program reads only the green and alpha channels of a noise cell).
-__device__ __forceinline__ float2 noise_tap(const float2* __restrict__ tab, float qx, float qy,
-                                            float qz) {
-    const float x = qx * (float)NOISE_N - 0.5f, y = qy * (float)NOISE_N - 0.5f,
-                z = qz * (float)NOISE_N - 0.5f;
-    const float fx = floorf(x), fy = floorf(y), fz = floorf(z);
-    const float wx = x - fx, wy = y - fy, wz = z - fz;
-    const int ix = ((int)fx % NOISE_N + NOISE_N) % NOISE_N;
-    const int iy = ((int)fy % NOISE_N + NOISE_N) % NOISE_N;
-    const int iz = ((int)fz % NOISE_N + NOISE_N) % NOISE_N;
-    const int jx = (ix + 1) & (NOISE_N - 1), jy = (iy + 1) & (NOISE_N - 1),
-              jz = (iz + 1) & (NOISE_N - 1);
-    const int r00 = (iz * NOISE_N + iy) * NOISE_N, r01 = (iz * NOISE_N + jy) * NOISE_N,
-              r10 = (jz * NOISE_N + iy) * NOISE_N, r11 = (jz * NOISE_N + jy) * NOISE_N;
-    const float2 c000 = __ldg(tab + r00 + ix), c001 = __ldg(tab + r00 + jx);
-    const float2 c010 = __ldg(tab + r01 + ix), c011 = __ldg(tab + r01 + jx);
-    const float2 c100 = __ldg(tab + r10 + ix), c101 = __ldg(tab + r10 + jx);
-    const float2 c110 = __ldg(tab + r11 + ix), c111 = __ldg(tab + r11 + jx);
-    auto tri = [&](float a000, float a001, float a010, float a011, float a100, float a101,
-                   float a110, float a111) {
-        const float x00 = a000 + wx * (a001 - a000), x10 = a010 + wx * (a011 - a010);
-        const float x01 = a100 + wx * (a101 - a100), x11 = a110 + wx * (a111 - a110);
-        const float y0 = x00 + wy * (x10 - x00), y1 = x01 + wy * (x11 - x01);
-        return y0 + wz * (y1 - y0);
-    };
-    return make_float2(tri(c000.x, c001.x, c010.x, c011.x, c100.x, c101.x, c110.x, c111.x),
-                       tri(c000.y, c001.y, c010.y, c011.y, c100.y, c101.y, c110.y, c111.y));
+// The blend of the noise cell (ix, iy, iz) (low five bits) at weights w.
+// `tab` holds for each cell, consecutively, what the blend along x takes: for
+// each (z, y) corner the green and alpha of the texel and the steps to its
+// neighbour along x (4 loads in place of 8, one address).
+__device__ __forceinline__ pair noise_cell(const ulonglong2* __restrict__ tab, int ix, int iy,
+                                           int iz, float wx, float wy, float wz) {
+    constexpr int M = NOISE_N - 1;
+    const ulonglong2* c = tab + (((iz & M) * NOISE_N + (iy & M)) * NOISE_N + (ix & M)) * 4;
+    const ulonglong2 c00 = __ldg(c), c10 = __ldg(c + 1), c01 = __ldg(c + 2), c11 = __ldg(c + 3);
+    const pair x = both(wx), y = both(wy), z = both(wz);
+    const pair x00 = fma2(x, c00.y, c00.x), x10 = fma2(x, c10.y, c10.x);
+    const pair x01 = fma2(x, c01.y, c01.x), x11 = fma2(x, c11.y, c11.x);
+    const pair y0 = fma2(y, sub2(x10, x00), x00), y1 = fma2(y, sub2(x11, x01), x01);
+    return fma2(z, sub2(y1, y0), y0);
+}
+
+// texture(noiseMap, q).ga summed over the octaves: LINEAR with REPEAT at
+// normalised coordinates (the fragment program reads only the green and alpha
+// channels of a noise cell).
+__device__ __forceinline__ pair noise_sum(const CompatDev& P, float cx, float cy, float cz) {
+    pair n = 0ull;
+    for (int k = 0; k < P.octaves; ++k) {
+        const float off = P.oct[k >> 1].off[k & 1], fr = P.oct[k >> 1].fr[k & 1];
+        const float x = (cx + off) * fr * (float)NOISE_N - 0.5f,
+                    y = (cy + off) * fr * (float)NOISE_N - 0.5f,
+                    z = (cz + off) * fr * (float)NOISE_N - 0.5f;
+        const float fx = floorf(x), fy = floorf(y), fz = floorf(z);
+        n = fma2(both(P.oct[k >> 1].pe[k & 1]),
+                 noise_cell(P.noise, (int)fx, (int)fy, (int)fz, x - fx, y - fy, z - fz), n);
+    }
+    return n;
+}
+
+// The same where every scaled coordinate's magnitude is below 2^21: floor and
+// cell come from one addition, and the coordinates of two octaves are made
+// together.
+__device__ __forceinline__ pair noise_sum_near(const CompatDev& P, float cx, float cy, float cz) {
+    const pair X = both(cx), Y = both(cy), Z = both(cz);
+    const pair magic = both(12582912.f);  // 1.5 * 2^23 (0x4B400000)
+    const pair scale = both((float)NOISE_N), half = both(-0.5f);
+    pair n = 0ull;
+    for (int k = 0; k < P.octaves; k += 2) {
+        const auto& o = P.oct[k >> 1];
+        const pair off = *reinterpret_cast<const pair*>(o.off),
+                   fr = *reinterpret_cast<const pair*>(o.fr);
+        const pair x = fma2(mul2(add2(X, off), fr), scale, half),
+                   y = fma2(mul2(add2(Y, off), fr), scale, half),
+                   z = fma2(mul2(add2(Z, off), fr), scale, half);
+        const pair mx = add2_down(x, magic), my = add2_down(y, magic), mz = add2_down(z, magic);
+        const float2 wx = halves(sub2(x, sub2(mx, magic))), wy = halves(sub2(y, sub2(my, magic))),
+                     wz = halves(sub2(z, sub2(mz, magic)));
+        n = fma2(both(o.pe[0]), noise_cell(P.noise, (int)mx, (int)my, (int)mz, wx.x, wy.x, wz.x),
+                 n);
+        if (k + 1 < P.octaves)
+            n = fma2(both(o.pe[1]),
+                     noise_cell(P.noise, (int)(mx >> 32), (int)(my >> 32), (int)(mz >> 32), wx.y,
+                                wy.y, wz.y),
+                     n);
+    }
+    return n;
 }
 
 __device__ __forceinline__ float sat(float x) { return fminf(fmaxf(x, 0.f), 1.f); }
@@ -207,19 +245,18 @@ __device__ bool compat_fragment(const VolDesc& vd, const ConeSchedule& cs, const
         const float lx = ex / (is - 1.f), ly = ey / (is - 1.f), lz = ez / (is - 1.f);
         const float oa = P.noise_opacity / (is - 1.f), la = 1.f / (is - 1.f);
         float ro = 0.f, rl = 0.f;
-        for (int i = 0; (float)i < is; ++i) {
-            float ng = 0.f, na = 0.f;  // the cell's green and alpha
-            float fr = 1.f, pe = 1.f;
-            for (int k = 0; k < P.octaves; ++k) {
-                const float off = k < 3 ? P.off[k] : 0.f;
-                const float2 t = noise_tap(P.noise, (cx + off) * fr, (cy + off) * fr,
-                                           (cz + off) * fr);
-                ng += pe * t.x;
-                na += pe * t.y;
-                fr *= P.freq_step;
-                pe *= P.pers_step;
-            }
-            na = fabsf(na);
+        // the samples lie between the near and the far point, so their largest
+        // coordinate is known before they are taken
+        const float reach = fmaxf(fmaxf(fmaxf(fabsf(cx), fabsf(cy)), fabsf(cz)),
+                                  fmaxf(fmaxf(fabsf(cx + ex), fabsf(cy + ey)), fabsf(cz + ez)));
+        const bool near = reach < P.noise_reach;
+        const int steps = (int)ceilf(is);
+        for (int i = 0; i < steps; ++i) {
+            // the cells' green and alpha
+            const float2 ga = halves(near ? noise_sum_near(P, cx, cy, cz)
+                                          : noise_sum(P, cx, cy, cz));
+            float ng = ga.x;
+            const float na = fabsf(ga.y);
             const float uu = ux * ux + uy * uy + uz * uz;
             ng += uy / sqrtf(uu);
             ro += na * (1.f - uu);
@@ -256,39 +293,67 @@ __device__ bool compat_fragment(const VolDesc& vd, const ConeSchedule& cs, const
     return true;
 }
 
-// One 256-thread CTA per 8x8-pixel tile: the tile's list is sorted once,
+// In place, the lists longer than cap (their tiles' CTAs hold no more keys).
+__global__ void __launch_bounds__(256) k_compat_sort(Bins bins, int cap,
+                                                     unsigned long long* list) {
+    const int m = (int)bins.count[blockIdx.x];
+    if (m > cap) sort_keys(list + bins.offset[blockIdx.x], m);
+}
+
+// One 128-thread CTA per half of an 8x8-pixel tile: the tile's list is sorted,
 // then split into SEG contiguous segments; thread (segment g, pixel p) blends
 // its segment front to back into (C_g, T_g) and the segments are combined in
 // order with the associative over operator, C = C_0 + T_0 (C_1 + T_1 (...)),
 // T = T_0 T_1 ...  A segment stops early on its own transmittance (the
 // combined image moves by at most the cutoff).
+// What bounds it: instructions (noise taps two thirds, cone samples a third) at
+// three quarters of the issue rate.  200 boards, 1080p, default noise and cone,
+// us: 2063 with eight-load taps, both paths of the general trilinear sample and a
+// 256-thread CTA a tile; 1729 with packed noise cells and clamped cone samples;
+// 1595 with two octaves' coordinates made together; 1511 with five CTAs an SM and
+// shared memory for the longest list, not for CAP keys (the L1 gets the rest); 1484
+// with two levels' cone samples together; 1447 with half tiles (a CTA waits
+// for its slowest warp; quarter tiles 1773, 2 segments 1617, 8 segments 1553).
 constexpr int SEG = 4;
-constexpr int TILE_PX = CG_COMPAT_TILE * CG_COMPAT_TILE;  // 64
+constexpr int SHARE = 2;  // CTAs a tile
+constexpr int TILE_PX = CG_COMPAT_TILE * CG_COMPAT_TILE / SHARE;
+constexpr int TILE_THREADS = SEG * TILE_PX;
 
 template <int FMT>
-__global__ void __launch_bounds__(256) k_compat_tiles(VolDesc vd, ConeSchedule cs, CompatDev P,
-                                                      const uint32_t* offset,
-                                                      unsigned long long* list, float4* out) {
-    __shared__ unsigned long long s_keys[CAP];
+__global__ void __launch_bounds__(TILE_THREADS, 1280 / TILE_THREADS)
+    k_compat_tiles(VolDesc vd, ConeSchedule cs, CompatDev P, Bins bins, int cap,
+                   const unsigned long long* list, float4* out) {
+    extern __shared__ unsigned long long s_keys[];  // cap of them
     __shared__ float4 s_c[SEG][TILE_PX];
     __shared__ float s_t[SEG][TILE_PX];
-    const int tile = blockIdx.x;
+    const int tile = blockIdx.x / SHARE, part = blockIdx.x % SHARE;
     const int tx = tile % P.tiles_x, ty = tile / P.tiles_x;
-    const uint32_t beg = offset[tile];
-    const int m = (int)(offset[tile + 1] - beg);
-    const bool in_smem = m <= CAP;
-    if (in_smem) {
-        for (int i = threadIdx.x; i < m; i += blockDim.x) s_keys[i] = list[beg + i];
+    list += bins.offset[tile];
+    const int m = (int)bins.count[tile];
+    if (m <= TILE_THREADS) {
+        // few keys (they differ): each goes where its rank says
+        const bool mine = (int)threadIdx.x < m;
+        const unsigned long long key = mine ? list[threadIdx.x] : 0ull;
+        if (mine) s_keys[threadIdx.x] = key;
+        __syncthreads();
+        int rank = 0;
+#pragma unroll 4
+        for (int i = 0; i < m; ++i) rank += s_keys[i] < key ? 1 : 0;
+        __syncthreads();
+        if (mine) s_keys[rank] = key;
+        __syncthreads();
+    } else if (m <= cap) {
+        for (int i = threadIdx.x; i < m; i += blockDim.x) s_keys[i] = list[i];
         __syncthreads();
         sort_keys(s_keys, m);
-    } else {
-        sort_keys(list + beg, m);
     }
-    const unsigned long long* keys = in_smem ? s_keys : list + beg;
+    // (a longer list has been sorted in place)
+    const unsigned long long* keys = m <= cap ? s_keys : list;
     const CamDesc& cam = P.cam;
     const int pix = threadIdx.x & (TILE_PX - 1), seg = threadIdx.x / TILE_PX;
     const int pxi = tx * CG_COMPAT_TILE + (pix & (CG_COMPAT_TILE - 1));
-    const int pyi = ty * CG_COMPAT_TILE + (pix / CG_COMPAT_TILE);
+    const int pyi =
+        ty * CG_COMPAT_TILE + part * (CG_COMPAT_TILE / SHARE) + pix / CG_COMPAT_TILE;
     const bool active = pxi < cam.W && pyi < cam.H;
     const float ndx = (2.f * ((float)pxi + 0.5f) / (float)cam.W - 1.f) * cam.tanh * cam.aspect;
     const float ndy = (1.f - 2.f * ((float)pyi + 0.5f) / (float)cam.H) * cam.tanh;
@@ -346,28 +411,36 @@ __global__ void __launch_bounds__(256) k_compat_tiles(VolDesc vd, ConeSchedule c
 
 }  // namespace
 
+// Warps per board of the count and fill passes: about 8192 in all (200 boards over
+// 32400 tiles, one warp a board: the whole binning 66 us, 37 now).
+static int board_parts(int n) { return std::min(64, std::max(1, 8192 / n)); }
+static int board_blocks(int n) { return (int)(((long long)n * board_parts(n) + 3) / 4); }
+
 cudaError_t launch_compat_count(const CompatDev& P, int4* rect, float* key, uint32_t* tile_count,
                                 unsigned long long* pairs, cudaStream_t st) {
     if (P.n == 0) return cudaSuccess;
-    k_compat_count<<<(P.n + 3) / 4, 128, 0, st>>>(P, rect, key, tile_count, pairs);
+    k_compat_count<<<board_blocks(P.n), 128, 0, st>>>(P, board_parts(P.n), rect, key, tile_count,
+                                                      pairs);
     return cudaGetLastError();
 }
 
 cudaError_t launch_compat_fill(const CompatDev& P, const int4* rect, const float* key,
                                uint32_t* cursor, unsigned long long* list, cudaStream_t st) {
     if (P.n == 0) return cudaSuccess;
-    k_compat_fill<<<(P.n + 3) / 4, 128, 0, st>>>(P, rect, key, cursor, list);
+    k_compat_fill<<<board_blocks(P.n), 128, 0, st>>>(P, board_parts(P.n), rect, key, cursor, list);
     return cudaGetLastError();
 }
 
 cudaError_t launch_compat_tiles(const VolDesc& vd, const ConeSchedule& cs, const CompatDev& P,
-                                const uint32_t* offset, unsigned long long* list, float4* out,
-                                cudaStream_t st) {
-    const int tiles = P.tiles_x * P.tiles_y;
+                                const Bins& bins, uint32_t most, unsigned long long* list,
+                                float4* out, cudaStream_t st) {
+    const int cap = (int)std::min<uint32_t>(CAP, std::max<uint32_t>(most, TILE_THREADS));
+    if (most > (uint32_t)cap) k_compat_sort<<<bins.nbins, 256, 0, st>>>(bins, cap, list);
+    const int blocks = bins.nbins * SHARE;
     if (vd.fmt == 0)
-        k_compat_tiles<0><<<tiles, 256, 0, st>>>(vd, cs, P, offset, list, out);
+        k_compat_tiles<0><<<blocks, TILE_THREADS, cap * 8, st>>>(vd, cs, P, bins, cap, list, out);
     else
-        k_compat_tiles<1><<<tiles, 256, 0, st>>>(vd, cs, P, offset, list, out);
+        k_compat_tiles<1><<<blocks, TILE_THREADS, cap * 8, st>>>(vd, cs, P, bins, cap, list, out);
     return cudaGetLastError();
 }
 

@@ -7,7 +7,6 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 
 #include "cg_internal.h"
@@ -86,98 +85,6 @@ __device__ __forceinline__ void bin_walk(const BoardsDev& b, int D, const Bins& 
     }
 }
 
-// Exclusive scan of the bin counts in one CTA; seeds the cursors.  Each
-// pass covers 1024 x 32 counts staged in shared memory: coalesced 16-byte
-// loads into a padded array (one spare word per 32 counts, so that a
-// thread's 32 consecutive counts fall in 32 different banks), per-thread sums,
-// a block scan of the thread sums, the exclusive offsets written back in
-// place, then coalesced 16-byte stores of offsets and cursors.  A running
-// carry links the passes.  count, offset and cursor are 16-byte aligned.
-constexpr int SCAN_PER = 32;
-constexpr int SCAN_TILE = 1024 * SCAN_PER;
-constexpr int SCAN_SMEM = (SCAN_TILE + SCAN_TILE / 32) * 4;
-
-__device__ __forceinline__ int scan_slot(int e) { return e + (e >> 5); }
-
-__global__ void __launch_bounds__(1024) k_bin_scan(Bins bins) {
-    extern __shared__ uint32_t s_cnt[];
-    __shared__ uint32_t warp_sums[32];
-    __shared__ uint32_t carry_s;
-    const int n = bins.nbins;
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    if (tid == 0) carry_s = 0;
-    for (int base = 0; base < n; base += SCAN_TILE) {
-        const int m = min(SCAN_TILE, n - base);
-#pragma unroll
-        for (int j = 0; j < SCAN_TILE / 4096; ++j) {
-            const int e = 4 * tid + 4096 * j;
-            uint4 q = make_uint4(0u, 0u, 0u, 0u);
-            if (e + 3 < m) {
-                q = *reinterpret_cast<const uint4*>(bins.count + base + e);
-            } else {
-                if (e < m) q.x = bins.count[base + e];
-                if (e + 1 < m) q.y = bins.count[base + e + 1];
-                if (e + 2 < m) q.z = bins.count[base + e + 2];
-            }
-            const int sl = scan_slot(e);
-            s_cnt[sl] = q.x;
-            s_cnt[sl + 1] = q.y;
-            s_cnt[sl + 2] = q.z;
-            s_cnt[sl + 3] = q.w;
-        }
-        __syncthreads();
-        uint32_t* mine = s_cnt + tid * (SCAN_PER + 1);
-        uint32_t s = 0;
-#pragma unroll
-        for (int k = 0; k < SCAN_PER; ++k) s += mine[k];
-        uint32_t x = s;
-        for (int o = 1; o < 32; o <<= 1) {
-            uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
-        }
-        if (lane == 31) warp_sums[wid] = x;
-        __syncthreads();
-        if (wid == 0) {
-            uint32_t w = warp_sums[lane], z = w;
-            for (int o = 1; o < 32; o <<= 1) {
-                uint32_t y = __shfl_up_sync(0xffffffffu, z, o);
-                if (lane >= o) z += y;
-            }
-            warp_sums[lane] = z - w;
-        }
-        __syncthreads();
-        const uint32_t carry = carry_s;
-        uint32_t run = carry + warp_sums[wid] + x - s;
-#pragma unroll
-        for (int k = 0; k < SCAN_PER; ++k) {
-            const uint32_t c = mine[k];
-            mine[k] = run;
-            run += c;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int j = 0; j < SCAN_TILE / 4096; ++j) {
-            const int e = 4 * tid + 4096 * j;
-            if (e >= m) continue;
-            const int sl = scan_slot(e);
-            const uint4 q = make_uint4(s_cnt[sl], s_cnt[sl + 1], s_cnt[sl + 2], s_cnt[sl + 3]);
-            if (e + 3 < m) {
-                *reinterpret_cast<uint4*>(bins.offset + base + e) = q;
-                *reinterpret_cast<uint4*>(bins.cursor + base + e) = q;
-            } else {
-                const uint32_t v[4] = {q.x, q.y, q.z, q.w};
-                for (int k = 0; e + k < m; ++k) {
-                    bins.offset[base + e + k] = v[k];
-                    bins.cursor[base + e + k] = v[k];
-                }
-            }
-        }
-        if (tid == 1023) carry_s = carry + warp_sums[wid] + x;
-        __syncthreads();
-    }
-    if (tid == 0) bins.offset[n] = carry_s;
-}
-
 // Ranges of the list for the bars' boards: bars need disjoint ranges in any
 // order, so a CTA takes one for its 256 bars with a single atomic on the total
 // (zeroed before; a scan in bar order took one CTA 13 us for 8192 bars).
@@ -207,6 +114,14 @@ __device__ __forceinline__ void bin_alloc(const Bins& bins, int block) {
         bins.offset[i] = at;
         bins.cursor[i] = at;
     }
+}
+
+// The ranges alone, and the largest count (*most, zeroed before).
+__global__ void __launch_bounds__(256) k_bin_alloc(Bins bins, uint32_t* most) {
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    const uint32_t m = __reduce_max_sync(0xffffffffu, i < bins.nbins ? bins.count[i] : 0u);
+    if ((threadIdx.x & 31) == 0 && m) atomicMax(most, m);
+    bin_alloc(bins, blockIdx.x);
 }
 
 // ---- sun-view nearest-surface map (first_voxelize.glsl:39-64) --------------
@@ -1242,21 +1157,8 @@ __global__ void k_count_active(const uint32_t* count, const uint8_t* mask, size_
 
 }  // namespace
 
-cudaError_t launch_bin_scan(Bins bins, cudaStream_t st) {
-    // the shared-memory attribute is set once per device (atomics keep
-    // concurrent host threads well-defined)
-    static std::atomic<bool> configured[64];
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-    if (!configured[dev].load(std::memory_order_acquire)) {
-        e = cudaFuncSetAttribute(k_bin_scan, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 SCAN_SMEM);
-        if (e != cudaSuccess) return e;
-        configured[dev].store(true, std::memory_order_release);
-    }
-    k_bin_scan<<<1, 1024, SCAN_SMEM, st>>>(bins);
+cudaError_t launch_bin_alloc(const Bins& bins, uint32_t* most, cudaStream_t st) {
+    k_bin_alloc<<<(bins.nbins + 255) / 256, 256, 0, st>>>(bins, most);
     return cudaGetLastError();
 }
 
