@@ -149,9 +149,9 @@ struct cg_volume {
     DevBuf pyr, count, dq, mask;
     // boards
     int n = 0;
-    size_t pairs = 0;
-    // board records in one allocation, uploaded with one copy: float4 centre +
-    // radius, int4 Q20 centre + radius, u64 ball threshold, u32 Q16 density,
+    size_t n_staged = 0;  // boards of the last upload (read from h_stage until boards_ready)
+    // board records in one allocation, made by one kernel: float4 centre + radius,
+    int4 Q20 centre + radius, u64 ball threshold, u32 Q16 density,
     // u8 culled (offsets 0, 16n, 32n, 40n, 44n)
     DevBuf boards;
     void* sun_boards = nullptr;  // in it
@@ -193,7 +193,7 @@ struct cg_volume {
     long long cov_gen = -1;  // voxelization whose integer coverage is in count / dq
     bool boards_dirty = false;  // billboards replaced since the last voxelize
     // cross-stream order of board uploads (context stream) and voxelizes (any
-    // stream): boards_ready follows the last upload's copies, boards_read the
+    // stream): boards_ready follows the last upload's kernel, boards_read the
     // last voxelize that read the board buffers (direct or graph replay)
     cudaEvent_t boards_ready = nullptr, boards_read = nullptr;
     bool ready_pending = false, read_pending = false;

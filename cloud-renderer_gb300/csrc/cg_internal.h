@@ -435,6 +435,14 @@ bool sun_frame_for_box(const float position[3], float b0, float b1, const float 
                        int H, SunFrame& fr);
 
 // ---- launchers (return cudaGetLastError of the launch) -------------------
+// The device records of n boards from their raw lists (3n positions, n radii, n
+// densities if `densities`), which may lie in page-locked host memory.
+struct BoardGrid {
+    float pos[3], wmin[3], range[3];
+    int D;
+};
+cudaError_t launch_boards(const float* raw, bool densities, int n, const BoardGrid& g, float4* cwr,
+                          int4* q, uint64_t* thr, uint32_t* dq, uint8_t* culled, cudaStream_t st);
 // Bar height of a volume's splat (k_voxelize.cu).
 int splat_bar(int dimension);
 // Disjoint ranges for the counts of bins.nbins (offset and cursor; count has one

@@ -37,6 +37,51 @@ __device__ __forceinline__ bool axis_range(int q, int rq, int D, int& lo, int& h
     return true;
 }
 
+// ---- board records ---------------------------------------------------------
+
+// Board quantization to the Q20 voxel grid (FP64, round to nearest even):
+//   v = (cw - wmin) / range * D per axis, q = rint(v * 2^20), culled from
+//   coverage when v is outside [-D, 2D] or no voxel centre is in the box;
+//   rq = rint(r / range_x * D * 2^20);  thr = floor(rq^2 * 9999 / 10000) (the
+//   0.01 profile discard of first_voxelize.glsl:46);  dq = rint(density * 2^16).
+// A thread per board; raw radii come with the fluffiness in them.
+__global__ void __launch_bounds__(128) k_boards(const float* __restrict__ raw, bool densities,
+                                                int n, BoardGrid g, float4* cwr, int4* qo,
+                                                uint64_t* thr, uint32_t* dq, uint8_t* culled) {
+    const int b = blockIdx.x * 128 + threadIdx.x;
+    if (b >= n) return;
+    const double D = (double)g.D;
+    const float r = raw[3 * (size_t)n + b];
+    const float d = densities ? raw[4 * (size_t)n + b] : 1.0f;
+    float c[3];
+    int q[3];
+    bool cull = false;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        c[a] = fadd(g.pos[a], raw[3 * (size_t)b + a]);
+        const double vv = __dmul_rn(
+            __ddiv_rn(__dsub_rn((double)c[a], (double)g.wmin[a]), (double)g.range[a]), D);
+        const bool in = vv >= -D && vv <= 2.0 * D;
+        q[a] = in ? (int)__double2ll_rn(__dmul_rn(vv, (double)CG_Q20)) : 0;
+        if (!in) cull = true;
+    }
+    const double rv = __dmul_rn(__ddiv_rn((double)r, (double)g.range[0]), D);
+    const int rq = (int)__double2ll_rn(__dmul_rn(rv, (double)CG_Q20));
+    // rq <= 512 * 2^20 < 2^30, so rq^2 < 2^60 fits; floor(r2 * 9999 / 10000)
+    // = r2 - ceil(r2 / 10000) without a 128-bit division
+    const uint64_t r2 = (uint64_t)rq * (uint64_t)rq;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        int lo, hi;
+        if (!axis_range(q[a], rq, g.D, lo, hi)) cull = true;
+    }
+    cwr[b] = make_float4(c[0], c[1], c[2], r);
+    qo[b] = make_int4(q[0], q[1], q[2], rq);
+    thr[b] = r2 - (r2 + 9999u) / 10000u;
+    dq[b] = (uint32_t)__double2ll_rn(__dmul_rn((double)d, 65536.0));
+    culled[b] = cull ? 1 : 0;
+}
+
 // ---- bar binning -----------------------------------------------------------
 
 // Distance term along one axis from the board centre q to the nearest voxel
@@ -1156,6 +1201,12 @@ __global__ void k_count_active(const uint32_t* count, const uint8_t* mask, size_
 }
 
 }  // namespace
+
+cudaError_t launch_boards(const float* raw, bool densities, int n, const BoardGrid& g, float4* cwr,
+                          int4* q, uint64_t* thr, uint32_t* dq, uint8_t* culled, cudaStream_t st) {
+    k_boards<<<(n + 127) / 128, 128, 0, st>>>(raw, densities, n, g, cwr, q, thr, dq, culled);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_bin_alloc(const Bins& bins, uint32_t* most, cudaStream_t st) {
     k_bin_alloc<<<(bins.nbins + 255) / 256, 256, 0, st>>>(bins, most);
