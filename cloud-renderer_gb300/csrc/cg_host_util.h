@@ -151,7 +151,7 @@ struct cg_volume {
     int n = 0;
     size_t n_staged = 0;  // boards of the last upload (read from h_stage until boards_ready)
     // board records in one allocation, made by one kernel: float4 centre + radius,
-    int4 Q20 centre + radius, u64 ball threshold, u32 Q16 density,
+    // int4 Q20 centre + radius, u64 ball threshold, u32 Q16 density,
     // u8 culled (offsets 0, 16n, 32n, 40n, 44n)
     DevBuf boards;
     void* sun_boards = nullptr;  // in it
