@@ -164,7 +164,11 @@ struct ConeSchedule {
     // odd number of steps is followed by one of weight 0 (they go in pairs)
     int quads;
     float reach;
-    int pad[3];
+    // the first `flat` steps (an even number) lie on level st[0].l0 exactly; their
+    // samples beyond flat_reach outside the box read 0
+    int flat;
+    float flat_reach;
+    int pad[1];
     ConeStep st[CG_MAX_SUN_STEPS];
 };
 

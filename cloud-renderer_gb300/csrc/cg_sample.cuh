@@ -332,6 +332,30 @@ __device__ __forceinline__ float tri_quads(const VolDesc& vd, float sc, int off,
     return y0 + wz * (y1 - y0);
 }
 
+// tri_quads where the position is known to lie in the padded grid: no clamps, the
+// cell's index from the additions' bits (the biases fall out modulo 2^32).
+template <int FMT>
+__device__ __forceinline__ float tri_flat(const VolDesc& vd, float sc, int off, int P, float px,
+                                          float py, float pz) {
+    constexpr float MAGIC = 12582912.f;
+    constexpr unsigned BIAS = 0x4B400000u - 2u;
+    const float x = px * sc - 0.5f, y = py * sc - 0.5f, z = pz * sc - 0.5f;
+    const float tx = __fadd_rd(x, MAGIC), ty = __fadd_rd(y, MAGIC), tz = __fadd_rd(z, MAGIC);
+    const float wx = x - (tx - MAGIC), wy = y - (ty - MAGIC), wz = z - (tz - MAGIC);
+    const unsigned p = (unsigned)P, base = (unsigned)off - BIAS * (p * p + p + 1u);
+    const int at = (int)(base + (__float_as_uint(tz) * p + __float_as_uint(ty)) * p +
+                         __float_as_uint(tx));
+    if (!CG_IN_BOUNDS(at, vd.quad_total) || !CG_IN_BOUNDS(at + P * P, vd.quad_total)) return 0.f;
+    const float4 a = load_quad<FMT>(vd, at), b = load_quad<FMT>(vd, at + P * P);
+    const float x00 = a.x + wx * (a.y - a.x);
+    const float x10 = a.z + wx * (a.w - a.z);
+    const float x01 = b.x + wx * (b.y - b.x);
+    const float x11 = b.z + wx * (b.w - b.z);
+    const float y0 = x00 + wy * (x10 - x00);
+    const float y1 = x01 + wy * (x11 - x01);
+    return y0 + wz * (y1 - y0);
+}
+
 // Cone steps st[i], st[i + 1] of a transmittance cone from the density quads:
 // both samples of the finer levels are in flight together, the coarser ones
 // only where a step lies between two levels.
@@ -363,20 +387,47 @@ __device__ __forceinline__ void compensate(float& sum, float& comp, float term) 
 
 // The transmittance cone over the density quads (cs.quads): the same samples
 // as cone_general's.  Steps beyond the position where the ray leaves the box
-// widened by cs.reach read exactly 0 and are not taken.
-template <int FMT>
+// widened by cs.reach read exactly 0 and are not taken.  The default cone starts at
+// its radius floor: its first 24 steps or more lie on one level exactly, and from
+// an origin in the box they need neither the level's values nor the clamps again
+// (FLAT, for view samples: 1080p over 256^3 RGBA32F 692 -> 648 us, 4K over 512^3
+// BF16 4238 -> 3938; positions from anywhere are better off without the second
+// loop, 250,000 of them 38.3 us and 39.7 with it).
+template <int FMT, bool FLAT>
 __device__ __forceinline__ float cone_quads(const VolDesc& vd, const ConeSchedule& cs, float vx,
                                             float vy, float vz, float sx, float sy, float sz) {
     const float D = (float)vd.D, E = cs.edge;
     const float h0 = cs.st[0].h;
     const float x = vx + h0 * sx, y = vy + h0 * sy, z = vz + h0 * sz;
     if (x < -E || y < -E || z < -E || x > D + E || y > D + E || z > D + E) return 0.f;
-    float out = 3e38f;
-    if (sx != 0.f) out = fminf(out, ((sx > 0.f ? D + cs.reach : -cs.reach) - vx) / sx);
-    if (sy != 0.f) out = fminf(out, ((sy > 0.f ? D + cs.reach : -cs.reach) - vy) / sy);
-    if (sz != 0.f) out = fminf(out, ((sz > 0.f ? D + cs.reach : -cs.reach) - vz) / sz);
+    // distances at which the ray leaves the box widened by cs.reach, and by
+    // cs.flat_reach
+    float out = 3e38f, flat_out = 3e38f;
+    const float v[3] = {vx, vy, vz}, d[3] = {sx, sy, sz};
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        if (d[a] == 0.f) continue;
+        const float r = 1.f / d[a], t = ((d[a] > 0.f ? D : 0.f) - v[a]) * r;
+        out = fminf(out, t + cs.reach * fabsf(r));
+        flat_out = fminf(flat_out, t + cs.flat_reach * fabsf(r));
+    }
     float tau = 0.f, comp = 0.f;
-    for (int i = 0; i < cs.steps; i += 2) {
+    int i = 0;
+    if (FLAT && fminf(fminf(vx, vy), vz) >= -0.25f &&
+        fmaxf(fmaxf(vx, vy), vz) <= D + 0.25f) {
+        const ConeStep& s = cs.st[0];
+        for (; i < cs.flat; i += 2) {
+            const float ha = cs.st[i].h, hb = cs.st[i + 1].h;
+            if (hb > flat_out) break;
+            const float a = tri_flat<FMT>(vd, s.sc0, s.off0, s.p0, vx + ha * sx, vy + ha * sy,
+                                          vz + ha * sz);
+            const float b = tri_flat<FMT>(vd, s.sc0, s.off0, s.p0, vx + hb * sx, vy + hb * sy,
+                                          vz + hb * sz);
+            compensate(tau, comp, a * cs.st[i].w);
+            compensate(tau, comp, b * cs.st[i + 1].w);
+        }
+    }
+    for (; i < cs.steps; i += 2) {
         if (cs.st[i].h > out) break;
         const float2 c = cone_pair<FMT>(vd, cs.st + i, vx, vy, vz, sx, sy, sz);
         compensate(tau, comp, c.x);
@@ -511,10 +562,10 @@ __device__ __noinline__ float cone_general(const VolDesc& vd, const ConeSchedule
 // Sun cone from level-0 voxel-space position v toward unit direction s.
 // Mode 0 returns optical depth (world units); mode 1 the reference's
 // weighted sum of the light channel.
-template <int FMT>
+template <int FMT, bool FLAT = true>
 __device__ __forceinline__ float sun_cone(const VolDesc& vd, const ConeSchedule& cs, float vx,
                                           float vy, float vz, float sx, float sy, float sz) {
-    if (cs.quads) return cone_quads<FMT>(vd, cs, vx, vy, vz, sx, sy, sz);
+    if (cs.quads) return cone_quads<FMT, FLAT>(vd, cs, vx, vy, vz, sx, sy, sz);
     return cone_general<FMT>(vd, cs, vx, vy, vz, sx, sy, sz);
 }
 

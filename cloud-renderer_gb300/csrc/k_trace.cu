@@ -269,7 +269,7 @@ __global__ void k_trace_cones(const __grid_constant__ VolDesc vd,
     // a caller's position may be a NaN, which the pyramid's own walk carries
     // through only where it samples something
     if (cs.quads && !isnan(x + y + z))
-        out[i] = cgs::cone_quads<FMT>(vd, cs, x, y, z, tp.sun[0], tp.sun[1], tp.sun[2]);
+        out[i] = cgs::cone_quads<FMT, false>(vd, cs, x, y, z, tp.sun[0], tp.sun[1], tp.sun[2]);
     else
         out[i] = cgs::cone_general<FMT>(vd, cs, x, y, z, tp.sun[0], tp.sun[1], tp.sun[2]);
 }
@@ -327,6 +327,13 @@ ConeSchedule make_cone_schedule(const VolDesc& vd, const TraceParams& tp) {
             const float half = 0.5f * (float)vd.D / (float)vd.dims[s.frac > 0.f ? l1 : s.l0];
             if (half + 1.f > cs.reach) cs.reach = half + 1.f;
         }
+        // (positions within flat_reach of the box stay in the padded quads)
+        cs.flat_reach = 0.5f / cs.st[0].sc0 + 1.f;
+        if (cs.st[0].sc0 <= 0.75f && cs.st[0].h >= 0.f)
+            while (cs.flat < cs.steps && cs.st[cs.flat].l0 == cs.st[0].l0 &&
+                   cs.st[cs.flat].frac == 0.f)
+                ++cs.flat;
+        cs.flat &= ~1;
         if (cs.steps & 1) {
             cs.st[cs.steps] = cs.st[cs.steps - 1];
             cs.st[cs.steps].w = 0.f;
