@@ -164,8 +164,19 @@ __device__ __forceinline__ float cone_part(const VolDesc& vd, const ConeSchedule
 // own cone as k_trace_fused does.  Samples, opacities and the compositing
 // order are k_trace_fused's; only the order in which a cooperative cone's
 // terms are added differs.
+// Threads of a CTA (256 / COOP_THREADS of them share a 16x16 pixel block) and the
+// warps an SM is to hold.  FP32 volumes, 1080p over 256^3, us: 256 threads and 32
+// warps 641, 128 and 32 626, 128 and 28 621 (72 registers, hardly a spill; a CTA lives
+// as long as its slowest warp), 128 and 24 635, 64 and 32 740.  Half-precision
+// volumes would gain as much (4K over 512^3 3907 -> 3791) and keep the larger CTAs
+// so that the surrogate stays the faster one next to a cone of half the steps.
 template <int FMT>
-__global__ void __launch_bounds__(256)
+constexpr int COOP_THREADS = FMT == 0 ? 128 : 256;
+template <int FMT>
+constexpr int COOP_WARPS = FMT == 0 ? 28 : 32;
+
+template <int FMT>
+__global__ void __launch_bounds__(COOP_THREADS<FMT>, COOP_WARPS<FMT> * 32 / COOP_THREADS<FMT>)
     k_trace_coop(const __grid_constant__ VolDesc vd, const __grid_constant__ CamDesc cam,
                  const __grid_constant__ TraceParams tp,
                  const __grid_constant__ ConeSchedule cone, float4* out, int coop_max) {
@@ -175,9 +186,11 @@ __global__ void __launch_bounds__(256)
     for (int i = threadIdx.x; i < (int)(sizeof(ConeSchedule) / 16); i += blockDim.x)
         reinterpret_cast<uint4*>(&cs)[i] = reinterpret_cast<const uint4*>(&cone)[i];
     __syncthreads();
-    int px, py;
-    tile_pixel(px, py);
+    constexpr int SHARE = 256 / COOP_THREADS<FMT>;
     const int lane = threadIdx.x & 31;
+    const int w = (int)(blockIdx.x % SHARE) * (8 / SHARE) + (int)(threadIdx.x >> 5);
+    const int px = (int)(blockIdx.x / SHARE) * 16 + (w & 1) * 8 + (lane & 7);
+    const int py = (int)blockIdx.y * 16 + (w >> 1) * 4 + (lane >> 3);
     const bool valid = px < cam.W && py < cam.H;
     float3 d = make_float3(0.f, 0.f, 0.f);
     float tin = 0.f, tout = 0.f;
@@ -342,15 +355,23 @@ ConeSchedule make_cone_schedule(const VolDesc& vd, const TraceParams& tp) {
     return cs;
 }
 
+template <int FMT>
+static void coop(dim3 blocks16, const VolDesc& vd, const CamDesc& cam, const TraceParams& tp,
+                 const ConeSchedule& cs, float4* out, cudaStream_t st) {
+    constexpr int T = COOP_THREADS<FMT>;
+    k_trace_coop<FMT><<<dim3(blocks16.x * (256 / T), blocks16.y), T, 0, st>>>(vd, cam, tp, cs, out,
+                                                                             tp.cone_lanes);
+}
+
 cudaError_t launch_trace_fused(VolDesc vd, CamDesc cam, TraceParams tp, float4* out,
                                unsigned long long* stats, cudaStream_t st) {
     ConeSchedule cs = make_cone_schedule(vd, tp);
     dim3 grd((cam.W + 15) / 16, (cam.H + 15) / 16);
     if (!stats && tp.cone_lanes > 0) {
         if (vd.fmt == 0)
-            k_trace_coop<0><<<grd, 256, 0, st>>>(vd, cam, tp, cs, out, tp.cone_lanes);
+            coop<0>(grd, vd, cam, tp, cs, out, st);
         else
-            k_trace_coop<1><<<grd, 256, 0, st>>>(vd, cam, tp, cs, out, tp.cone_lanes);
+            coop<1>(grd, vd, cam, tp, cs, out, st);
     } else if (stats) {
         if (vd.fmt == 0)
             k_trace_fused<0, true><<<grd, 256, 0, st>>>(vd, cam, tp, cs, out, stats);
