@@ -8,14 +8,15 @@
 // Each tile runs the exact view march of k_trace_fused (same per-sample
 // arithmetic in the same order, so images are bit-identical) with one of two
 // ray mappings:
-//   LPR = 1: one ray per thread (32 rays per warp), 16 x 16 pixels per tile;
+//   LPR = 1: one ray per thread (32 rays per warp), 16 x 8 pixels per tile;
 //   LPR = 4, 8, 32: LPR lanes per ray (8, 4 or 1 rays per warp): the lanes
 //     of a ray evaluate LPR consecutive view steps at once (density, noise,
 //     opacity), the group replays the compositing order serially through
 //     shuffles to find which steps contribute before the ray terminates, and
 //     the contributing steps' sun cones -- the expensive part -- run in
 //     parallel across the lanes.
-// UNROLL unrolls the step loop (LPR = 1) or the chunk loop (LPR > 1).
+// UNROLL unrolls the step loop (LPR = 1, where no step is skipped) or the chunk loop
+// (LPR > 1).
 #include <algorithm>
 
 #include "cg_internal.h"
@@ -51,12 +52,17 @@ __device__ __forceinline__ bool ray_of(const CamDesc& cam, const VolDesc& vd, in
     return tout > tin;
 }
 
-// Pixel tile of a CTA: 256 / LPR pixels, 16 wide for LPR = 1 (16 x 16),
-// otherwise 8 wide (8 x 32 / LPR).
+// Pixel tile of a CTA: 256 / LPR pixels, 8 wide (8 x 32 / LPR); with one thread a
+// ray 16 x 8 by 128 threads, as a CTA waits for its slowest warp before its next
+// tile (32 views of 12 clouds: 16 x 16 at 24 warps an SM 5.48 ms, 16 x 8 at 28 5.27;
+// with the steps of empty bricks skipped 4.90 at 28, 4.86 at 32).
+constexpr int BATCH_T1 = 128;
+constexpr int BATCH_W = 32;
 template <int LPR>
 struct TileShape {
     static constexpr int W = LPR == 1 ? 16 : 8;
-    static constexpr int H = (256 / LPR) / W;
+    static constexpr int THREADS = LPR == 1 ? BATCH_T1 : 256;
+    static constexpr int H = (THREADS / LPR) / W;
 };
 
 // The march of one ray, one thread (k_trace_fused's loop).
@@ -72,33 +78,55 @@ __device__ __forceinline__ float4 march_thread(const VolDesc& vd, const CamDesc&
     const float D = (float)vd.D;
     const float vsx = D / vd.range[0], vsy = D / vd.range[1], vsz = D / vd.range[2];
     const float pixk = cam.tanh / (float)cam.H * vsx;
-    // when every sample has lod 0, steps outside the occupied box read 0
-    int kbeg = 0, kend = Nv;
-    if (2.f * (tin + ((float)(Nv - 1) + 0.5f) * dt) * pixk <= 1.f) {
-        int k0, k1;
-        cgs::occupied_steps(vd, cam.eye, d, tin, dt, Nv, k0, k1);
-        kbeg = k0;
-        kend = k1 + 1;
-    }
     float T = 1.f, C = 0.f, Cc = 0.f;
-#pragma unroll UNROLL
-    for (int k = kbeg; k < kend; ++k) {
+    // shades step k; true when the ray ends there
+    auto shade = [&](int k, bool lod0) {
         float t = tin + ((float)k + 0.5f) * dt;
         float p0 = cam.eye[0] + t * d.x, p1 = cam.eye[1] + t * d.y, p2 = cam.eye[2] + t * d.z;
         float v0 = (p0 - vd.wmin[0]) * vsx, v1 = (p1 - vd.wmin[1]) * vsy,
               v2 = (p2 - vd.wmin[2]) * vsz;
-        float lod = log2f(fmaxf(1.f, 2.f * t * pixk));
-        float2 rg = cgs::quad<FMT, true, true, true>(vd, v0, v1, v2, lod);
-        if (!(rg.x > 0.f)) continue;
+        const float2 rg =
+            lod0 ? cgs::tri<FMT, true, true, false>(vd, 0, v0, v1, v2)
+                 : cgs::quad<FMT, true, true, true>(vd, v0, v1, v2,
+                                                    log2f(fmaxf(1.f, 2.f * t * pixk)));
+        if (!(rg.x > 0.f)) return false;
         float rho = rg.x * cgs::fbm(tp, p0, p1, p2);
-        if (!(rho > 0.f)) continue;
+        if (!(rho > 0.f)) return false;
         float alpha = 1.f - expf(-tp.sigma * rho * dt);
         float tau = cgs::sun_cone<FMT>(vd, cs, v0, v1, v2, tp.sun[0], tp.sun[1], tp.sun[2]);
         float Ts = expf(-tp.sigma * tau);
         float L = Ts * (tp.ambient + (1.f - tp.ambient) * rg.y);
         cgs::neumaier(C, Cc, T * alpha * L);
         T *= 1.f - alpha;
-        if (T < tp.cutoff) break;
+        return T < tp.cutoff;
+    };
+    // when every sample has lod 0, steps outside the occupied box and in empty
+    // bricks read 0: the flags of eight steps are fetched together (linear in k,
+    // off by a rounding at most, which the flags allow: they cover the bricks
+    // around), and a lane goes on with its next step that has one
+    // (12 clouds: 5.27 -> 4.86 ms)
+    if (2.f * (tin + ((float)(Nv - 1) + 0.5f) * dt) * pixk <= 1.f) {
+        int kbeg, kend;
+        cgs::occupied_steps(vd, cam.eye, d, tin, dt, Nv, kbeg, kend);
+        const float o = tin + 0.5f * dt;
+        const float v0a[3] = {(cam.eye[0] + o * d.x - vd.wmin[0]) * vsx,
+                              (cam.eye[1] + o * d.y - vd.wmin[1]) * vsy,
+                              (cam.eye[2] + o * d.z - vd.wmin[2]) * vsz};
+        const float dva[3] = {dt * d.x * vsx, dt * d.y * vsy, dt * d.z * vsz};
+        cgs::OccRay bricks;
+        bricks.set(vd, 0, v0a, dva, (float)(1 << vd.occ_shift), -0.5f);
+        bool done = false;
+        for (int k = kbeg; k <= kend && !done; k += 8) {
+            unsigned m = 0u;
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                m |= (bricks.at((float)(k + j)) && k + j <= kend ? 1u : 0u) << j;
+            for (; m && !done; m &= m - 1u) done = shade(k + __ffs(m) - 1, true);
+        }
+    } else {
+#pragma unroll UNROLL
+        for (int k = 0; k < Nv; ++k)
+            if (shade(k, false)) break;
     }
     C += Cc;
     return make_float4(C * tp.sun_color[0], C * tp.sun_color[1], C * tp.sun_color[2], 1.f - T);
@@ -196,8 +224,9 @@ __device__ __forceinline__ float4 march_group(const VolDesc& vd, const CamDesc& 
 }
 
 template <int FMT, int LPR, int UNROLL>
-__global__ void __launch_bounds__(256) k_trace_batch(const BatchView* views, int nviews,
-                                                     unsigned total_tiles, unsigned* counter) {
+__global__ void __launch_bounds__(TileShape<LPR>::THREADS, LPR == 1 ? BATCH_W * 32 / BATCH_T1 : 1)
+    k_trace_batch(const BatchView* views, int nviews,
+                  unsigned total_tiles, unsigned* counter) {
     __shared__ BatchView sv;
     __shared__ unsigned s_tile;
     __shared__ int s_view;
@@ -238,7 +267,7 @@ __global__ void __launch_bounds__(256) k_trace_batch(const BatchView* views, int
         if (LPR == 1) {
             const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
             const int px = tx * 16 + (w & 1) * 8 + (lane & 7);
-            const int py = ty * 16 + (w >> 1) * 4 + (lane >> 3);
+            const int py = ty * TS::H + (w >> 1) * 4 + (lane >> 3);
             if (px < sv.cam.W && py < sv.cam.H)
                 sv.out[(size_t)py * sv.cam.W + px] =
                     march_thread<FMT, UNROLL>(sv.vd, sv.cam, sv.tp, sv.cs, px, py);
@@ -256,7 +285,8 @@ __global__ void __launch_bounds__(256) k_trace_batch(const BatchView* views, int
 template <int FMT, int LPR, int UNROLL>
 cudaError_t launch_one(const BatchView* views, int n, unsigned total, unsigned* counter,
                        int blocks, cudaStream_t st) {
-    k_trace_batch<FMT, LPR, UNROLL><<<blocks, 256, 0, st>>>(views, n, total, counter);
+    constexpr int T = TileShape<LPR>::THREADS;
+    k_trace_batch<FMT, LPR, UNROLL><<<blocks * (256 / T), T, 0, st>>>(views, n, total, counter);
     return cudaGetLastError();
 }
 
@@ -285,7 +315,7 @@ cudaError_t launch_lpr(int lpr, int unroll, const BatchView* views, int n, unsig
 
 void batch_tiles(int lanes_per_ray, int width, int height, int& tiles_x, int& tiles_y) {
     const int tw = lanes_per_ray == 1 ? 16 : 8;
-    const int th = (256 / lanes_per_ray) / tw;
+    const int th = lanes_per_ray == 1 ? BATCH_T1 / 16 : (256 / lanes_per_ray) / tw;
     tiles_x = (width + tw - 1) / tw;
     tiles_y = (height + th - 1) / th;
 }
