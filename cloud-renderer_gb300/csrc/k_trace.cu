@@ -202,9 +202,11 @@ __global__ void __launch_bounds__(COOP_THREADS<FMT>, COOP_WARPS<FMT> * 32 / COOP
     const float vsx = D / vd.range[0], vsy = D / vd.range[1], vsz = D / vd.range[2];
     const float pixk = cam.tanh / (float)cam.H * vsx;
     int kbeg = 0, kend = Nv;
+    bool lod0 = true;
     if (live) {
         const float tlast = tin + ((float)(Nv - 1) + 0.5f) * dt;
-        if (2.f * tlast * pixk <= 1.f) {
+        lod0 = 2.f * tlast * pixk <= 1.f;
+        if (lod0) {
             int k0, k1;
             cgs::occupied_steps(vd, cam.eye, d, tin, dt, Nv, k0, k1);
             kbeg = k0;
@@ -214,20 +216,57 @@ __global__ void __launch_bounds__(COOP_THREADS<FMT>, COOP_WARPS<FMT> * 32 / COOP
     }
     float T = 1.f, C = 0.f, Cc = 0.f;
     const int wk0 = __reduce_min_sync(0xffffffffu, live ? kbeg : Nv);
-    for (int k = wk0; k < Nv; ++k) {
-        if (live && k >= kend) live = false;
-        if (!__any_sync(0xffffffffu, live)) break;
+    // SKIP: every lane's samples have lod 0 (the common case), so a step reads 0
+    // where its brick is unoccupied: the flags of eight steps are fetched together
+    // (linear in k, off by a rounding at most, which the flags allow: they cover
+    // the bricks around), and only the steps at which some lane has one are taken.
+    // FP32 volumes only, as COOP_THREADS (1080p over 256^3 621 -> 590 us).
+    const bool skip = FMT == 0 && __all_sync(0xffffffffu, !live || lod0);
+    cgs::OccRay bricks;
+    if (skip) {
+        const float o = tin + 0.5f * dt;
+        const float v0a[3] = {(cam.eye[0] + o * d.x - vd.wmin[0]) * vsx,
+                              (cam.eye[1] + o * d.y - vd.wmin[1]) * vsy,
+                              (cam.eye[2] + o * d.z - vd.wmin[2]) * vsz};
+        const float dva[3] = {dt * d.x * vsx, dt * d.y * vsy, dt * d.z * vsz};
+        bricks.set(vd, 0, v0a, dva, (float)(1 << vd.occ_shift), -0.5f);
+    }
+    unsigned mine = 0u, any = 0u;  // flags of the steps of the chunk at kc: this lane's, the warp's
+    int kc = wk0 - 8;
+    for (int k = wk0;; ++k) {
+        if (skip) {
+            while (!any) {
+                kc += 8;
+                if (live && kc >= kend) live = false;
+                if (kc >= Nv || !__any_sync(0xffffffffu, live)) break;
+                mine = 0u;
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    mine |= (bricks.at((float)(kc + j)) && kc + j >= kbeg && kc + j < kend ? 1u : 0u)
+                            << j;
+                if (!live) mine = 0u;
+                any = __reduce_or_sync(0xffffffffu, mine);
+            }
+            if (!any) break;
+            k = kc + __ffs(any) - 1;
+            any &= any - 1u;
+        } else {
+            if (live && k >= kend) live = false;
+            if (k >= Nv || !__any_sync(0xffffffffu, live)) break;
+        }
         bool emit = false;
         float v0 = 0.f, v1 = 0.f, v2 = 0.f, alpha = 0.f, G = 0.f;
-        if (live && k >= kbeg) {
+        if (live && (skip ? (mine >> (k - kc)) & 1u : k >= kbeg)) {
             const float t = tin + ((float)k + 0.5f) * dt;
             const float p0 = cam.eye[0] + t * d.x, p1 = cam.eye[1] + t * d.y,
                         p2 = cam.eye[2] + t * d.z;
             v0 = (p0 - vd.wmin[0]) * vsx;
             v1 = (p1 - vd.wmin[1]) * vsy;
             v2 = (p2 - vd.wmin[2]) * vsz;
-            const float lod = log2f(fmaxf(1.f, 2.f * t * pixk));
-            const float2 rg = cgs::quad<FMT, true, true, true>(vd, v0, v1, v2, lod);
+            const float2 rg =
+                skip ? cgs::tri<FMT, true, true, false>(vd, 0, v0, v1, v2)
+                     : cgs::quad<FMT, true, true, true>(vd, v0, v1, v2,
+                                                        log2f(fmaxf(1.f, 2.f * t * pixk)));
             if (rg.x > 0.f) {
                 const float rho = rg.x * cgs::fbm(tp, p0, p1, p2);
                 if (rho > 0.f) {
