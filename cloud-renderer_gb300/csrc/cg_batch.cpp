@@ -1,6 +1,7 @@
 // cg_batch.cpp -- many volumes and views per frame behind the C ABI: the
 // batch render (one persistent launch), the launch-shape autotuner and the
 // frame graph (every voxelize plus the batch render as one CUDA graph).
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -245,6 +246,49 @@ void free_graph(cg_frame_graph* g) {
     delete g;
 }
 
+// Branches of the captured frame that voxelize side by side: a voxelize is a chain
+// of short kernels, few of which fill the GPU.  (12 clouds and 32 views, us a frame
+// with 1, 2, 3, 4, 6 and 12 of them: 4855, 4630, 4555, 4537, 4535, 4527.)
+constexpr int FRAME_LANES = 4;
+
+// A branch's streams and events, for the time of the capture.
+struct FrameLane {
+    cudaStream_t s = nullptr, side = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr, done = nullptr;
+    cudaError_t create() {
+        cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking);
+        for (cudaEvent_t* ev : {&fork, &join, &done})
+            if (e == cudaSuccess) e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
+        return e;
+    }
+    ~FrameLane() {
+        for (cudaEvent_t ev : {fork, join, done})
+            if (ev) cudaEventDestroy(ev);
+        if (side) cudaStreamDestroy(side);
+        if (s) cudaStreamDestroy(s);
+    }
+};
+
+// Every volume's voxelize, captured on the lanes, which fork from s and join it.
+cg_status capture_voxelizes(cg_frame_graph* g, FrameLane* lanes, int n, cudaStream_t s) {
+    CG_CUDA(cudaEventRecord(lanes[0].done, s));
+    for (int i = 0; i < n; ++i) CG_CUDA(cudaStreamWaitEvent(lanes[i].s, lanes[0].done, 0));
+    for (size_t i = 0; i < g->volumes.size(); ++i) {
+        // a volume listed again follows itself
+        size_t first = 0;
+        while (g->volumes[first] != g->volumes[i]) ++first;
+        FrameLane& l = lanes[first % (size_t)n];
+        const cg_status st = voxelize_on(g->volumes[i], &g->sun, l.s, {l.side, l.fork, l.join});
+        if (st != CG_OK) return st;
+    }
+    for (int i = 0; i < n; ++i) {
+        CG_CUDA(cudaEventRecord(lanes[i].done, lanes[i].s));
+        CG_CUDA(cudaStreamWaitEvent(s, lanes[i].done, 0));
+    }
+    return CG_OK;
+}
+
 // One eager frame (allocations, noise tables, descriptors), then the capture.
 cg_status capture(cg_frame_graph* g) {
     cg_context* ctx = g->ctx;
@@ -274,10 +318,13 @@ cg_status capture(cg_frame_graph* g) {
     }
     BatchView* views_dev = g->desc.as<BatchView>();
     unsigned* counter = reinterpret_cast<unsigned*>(g->desc.as<uint8_t>() + bytes);
-    cudaError_t e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
+    FrameLane lanes[FRAME_LANES];
+    const int n = (int)std::min<size_t>(FRAME_LANES, g->volumes.size());
+    cudaError_t e = cudaSuccess;
+    for (int i = 0; i < n && e == cudaSuccess; ++i) e = lanes[i].create();
+    if (e == cudaSuccess) e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
-        for (cg_volume* v : g->volumes)
-            if (st == CG_OK) st = cg_voxelize(v, &g->sun, s);
+        st = capture_voxelizes(g, lanes, n, s);
         if (st == CG_OK)
             e = launch_trace_batch(g->fmt, g->cfg.lanes_per_ray, g->cfg.step_unroll, views_dev, nv,
                                    g->total, counter, s);

@@ -846,7 +846,7 @@ static float highlight_offset(const cg_volume* v) {
 }
 
 
-extern "C" cg_status cg_voxelize(cg_volume* v, const cg_sun* sun, void* stream) {
+cg_status voxelize_on(cg_volume* v, const cg_sun* sun, cudaStream_t s, const VoxelizeLane& lane) {
     NvtxRange nvtx_("cg_voxelize");
     CG_CHECK(v && sun, CG_ERR_INVALID_ARGUMENT, "cg_voxelize: null pointer");
     CG_CHECK(sun->map_width >= 1 && sun->map_height >= 1 && sun->map_width <= 16384 &&
@@ -862,7 +862,6 @@ extern "C" cg_status cg_voxelize(cg_volume* v, const cg_sun* sun, void* stream) 
              "cg_voxelize: sun direction is zero or parallel to the up axis (0,1,0)");
     cg_context* ctx = v->ctx;
     CG_CUDA(cudaSetDevice(ctx->device));
-    cudaStream_t s = pick_stream(ctx, stream);
     const size_t texels = (size_t)sun->map_width * sun->map_height;
     if (v->mapW != sun->map_width || v->mapH != sun->map_height) {
         CG_CUDA(cudaStreamSynchronize(s));
@@ -900,14 +899,14 @@ extern "C" cg_status cg_voxelize(cg_volume* v, const cg_sun* sun, void* stream) 
     // clearGPU (CloudVolume.cpp:96-100) + clearPositionMap (VoxelizeShader.cpp:185-187):
     // what the sun-view pass needs is cleared on s, the rest beside it on the
     // side stream
-    cudaStream_t sd = ctx->side;
-    CG_CUDA(cudaEventRecord(ctx->fork_ev, s));
-    CG_CUDA(cudaStreamWaitEvent(sd, ctx->fork_ev, 0));
+    cudaStream_t sd = lane.side;
+    CG_CUDA(cudaEventRecord(lane.fork, s));
+    CG_CUDA(cudaStreamWaitEvent(sd, lane.fork, 0));
     CG_CUDA(cudaMemsetAsync(v->mask.p, 0, n0, sd));
     CG_CUDA(cudaMemsetAsync(v->bhl.p, 0, (size_t)bins.nbricks, sd));
     // raw cells, brick grids (rewritten by the dilation) and the occupied box
     CG_CUDA(cudaMemsetAsync(v->occ.p, 0, occ_box_offset(v->raw_total) + 6 * sizeof(int), sd));
-    CG_CUDA(cudaEventRecord(ctx->join_ev, sd));
+    CG_CUDA(cudaEventRecord(lane.join, sd));
     // the keys and the tiles' bounds behind them (the tables there are rewritten)
     CG_CUDA(cudaMemsetAsync(v->keys.p, 0xFF, texels * 8 + sun_aux_words(fr.W, fr.H) * 4, s));
     // the bars' counts and, behind them, their list's total
@@ -921,7 +920,7 @@ extern "C" cg_status cg_voxelize(cg_volume* v, const cg_sun* sun, void* stream) 
                                        v->D, bins, s));
         stage_mark(ctx, s, "sun");
         // pass 2: highlight stores (after the mask's clearing) and the bars' lists
-        CG_CUDA(cudaStreamWaitEvent(s, ctx->join_ev, 0));
+        CG_CUDA(cudaStreamWaitEvent(s, lane.join, 0));
         CG_LAUNCH(ctx, launch_highlight(b, fr, v->keys.as<uint64_t>(), v->posmap.as<float4>(),
                                         v->D, v->wmin, v->range, highlight_offset(v),
                                         v->mask.as<uint8_t>(), v->bhl.as<uint8_t>(), &bins, s));
@@ -938,12 +937,12 @@ extern "C" cg_status cg_voxelize(cg_volume* v, const cg_sun* sun, void* stream) 
     stage_mark(ctx, s, "splat");
     // the occupancy dilation (raw cells -> brick grids, occupied box) and the
     // remaining mips are independent: the dilation runs on the side stream
-    CG_CUDA(cudaEventRecord(ctx->fork_ev, s));
-    CG_CUDA(cudaStreamWaitEvent(sd, ctx->fork_ev, 0));
+    CG_CUDA(cudaEventRecord(lane.fork, s));
+    CG_CUDA(cudaStreamWaitEvent(sd, lane.fork, 0));
     CG_LAUNCH(ctx, launch_occ_coarse(bins, raw_of(v), v->L, sd));
     CG_LAUNCH(ctx, launch_occ_dilate(vd, raw_of(v), v->occ.as<uint8_t>() + v->raw_total,
                                      v->occ_total, sd));
-    CG_CUDA(cudaEventRecord(ctx->join_ev, sd));
+    CG_CUDA(cudaEventRecord(lane.join, sd));
     // remaining mips (glGenerateMipmap, VoxelizeShader.cpp:105)
     {
         for (int l = fused; l + 1 < v->L; l += 3) {
@@ -951,7 +950,7 @@ extern "C" cg_status cg_voxelize(cg_volume* v, const cg_sun* sun, void* stream) 
             if (v->dims[l] <= CG_MIP_LAST) break;  // that launch made every level left
         }
     }
-    CG_CUDA(cudaStreamWaitEvent(s, ctx->join_ev, 0));
+    CG_CUDA(cudaStreamWaitEvent(s, lane.join, 0));
     stage_mark(ctx, s, "mips");
     if (!capturing) {
         CG_CUDA(cudaEventRecord(v->boards_read, s));
@@ -962,6 +961,12 @@ extern "C" cg_status cg_voxelize(cg_volume* v, const cg_sun* sun, void* stream) 
     v->gen++;
     if (write_tex) v->tex_gen = v->gen;
     return CG_OK;
+}
+
+extern "C" cg_status cg_voxelize(cg_volume* v, const cg_sun* sun, void* stream) {
+    CG_CHECK(v, CG_ERR_INVALID_ARGUMENT, "cg_voxelize: null pointer");
+    cg_context* ctx = v->ctx;
+    return voxelize_on(v, sun, pick_stream(ctx, stream), {ctx->side, ctx->fork_ev, ctx->join_ev});
 }
 
 // ---------------------------------------------------------------------------

@@ -205,6 +205,12 @@ VolDesc desc_of(const cg_volume* v);
 // Byte offset of the level-0 occupied box in the volume's occupancy buffer.
 size_t occ_box_offset(int raw_total);
 OccRaw raw_of(const cg_volume* v);
+// cg_voxelize on stream s with a side stream and the events that fork and join it.
+struct VoxelizeLane {
+    cudaStream_t side;
+    cudaEvent_t fork, join;
+};
+cg_status voxelize_on(cg_volume* v, const cg_sun* sun, cudaStream_t s, const VoxelizeLane& lane);
 void set_occ_layout(cg_volume* v, int brick);
 BoardsDev boards_of(const cg_volume* v);
 cg_status check_params(const cg_render_params* p);
