@@ -419,9 +419,9 @@ extern "C" cg_status cg_mlp_infer(const cg_mlp* m, const float* features, int n,
         CG_CUDA(tout.ensure((size_t)n * 4));
         dout = tout.as<float>();
     }
-    // the tensor-core status block: [1] records a wait that ran out
+    // the tensor-core status block: [1] records a wait that ran out (the kernel
+    // clears it first)
     CG_CUDA(ctx->fallbacks.ensure(32));
-    CG_CUDA(cudaMemsetAsync(ctx->fallbacks.p, 0, 32, s));
     ctx->shaded_valid = false;
     CG_LAUNCH(ctx, launch_mlp_infer(device_view(m), df, n, dout,
                                     ctx->fallbacks.as<unsigned long long>(), s));
