@@ -715,7 +715,7 @@ def run_ours(args):
             "gpu_launches": int(head["launches"]),
             "clocks": learned["clocks"],
             "e2e": {"value": round(e2e_val, 3), "unit": UNIT,
-                    "h2d_bytes_per_step": head_vol.count * 45, "d2h_bytes_per_step": W * H * 16}}
+                    "h2d_bytes_per_step": head_vol.count * 20, "d2h_bytes_per_step": W * H * 16}}
     vol32.close()
     vol16.close()
     img = flush = None
@@ -997,7 +997,7 @@ def run_animated(args):
             "gpu_launches": int(launches),
             "clocks": sampler.summary(),
             "e2e": {"value": round(W * H * args.steps / wall_s / 1e6, 3), "unit": "Mpix/s",
-                    "h2d_bytes_per_step": n * 45, "d2h_bytes_per_step": 0,
+                    "h2d_bytes_per_step": n * 20, "d2h_bytes_per_step": 0,
                     "note": "wall clock of the same loop (L2 flush per step, no per-step "
                             "events), host board quantization and upload included; the image "
                             "stays on the device"}}
@@ -1099,7 +1099,7 @@ def run_compat(args):
             "gpu_launches": int(launches),
             "clocks": sampler.summary(),
             "e2e": {"value": round(W * H / float(np.median(e2e)) / 1e6, 3), "unit": "Mpix/s",
-                    "h2d_bytes_per_step": vol.count * 45, "d2h_bytes_per_step": W * H * 16}}
+                    "h2d_bytes_per_step": vol.count * 20, "d2h_bytes_per_step": W * H * 16}}
     if not args.no_cpu_baseline:
         from oracle import oracle as O
         threads = os.cpu_count() or 1

@@ -918,6 +918,7 @@ cg_status voxelize_on(cg_volume* v, const cg_sun* sun, cudaStream_t s, const Vox
                                        sun_aux(v->keys.as<uint32_t>() + 2 * texels, v->sun_boards,
                                                fr.W, fr.H),
                                        v->D, bins, s));
+        if (b.n) ctx->launches++;  // (two kernels)
         stage_mark(ctx, s, "sun");
         // pass 2: highlight stores (after the mask's clearing) and the bars' lists
         CG_CUDA(cudaStreamWaitEvent(s, lane.join, 0));

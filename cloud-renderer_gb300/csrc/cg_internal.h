@@ -195,8 +195,8 @@ struct Bins {
     // the bins: bars of 8 x 8 x bar voxels (bar = 8 or 32; nbarz along z); the
     // compat render's are pixel tiles
     int bar, nbarz, nbins;
-    uint32_t* count;   // nbins (+ 1 in a volume: the list's total)
-    uint32_t* offset;  // nbins (+ 1: the compat render's scan)
+    uint32_t* count;   // nbins + 1 (behind them the list's total)
+    uint32_t* offset;  // nbins
     uint32_t* cursor;  // nbins
     uint32_t* list;    // pairs
     // per brick: 1 when its level-0 voxels (and fused levels 1-3) may hold
