@@ -251,6 +251,8 @@ extern "C" cg_status cg_render_compat(cg_context* ctx, const cg_volume* v, const
     bins.count = base + 4;
     bins.offset = bins.count + words;
     bins.cursor = bins.offset + words;
+    // after the last board upload (made on the context stream)
+    if (v->ready_pending && s != ctx->stream) CG_CUDA(cudaStreamWaitEvent(s, v->boards_ready, 0));
     stage_begin(ctx, s);
     CG_CUDA(cudaMemsetAsync(base, 0, (4 + words) * 4, s));
     CG_LAUNCH(ctx, launch_compat_count(P, ctx->compat_rect.as<int4>(), ctx->compat_key.as<float>(),
