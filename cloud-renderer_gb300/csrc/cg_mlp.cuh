@@ -75,31 +75,25 @@ __device__ __forceinline__ int half_index(int p) {
 // or half-written partials -- the loss slot is NaN and nothing is updated.
 // The partials are read past L1 (other SMs wrote them in the same launch when
 // the optimiser is fused).
-__device__ __forceinline__ void adam_param(const AdamArgs& aa, int p, int step, bool stopped) {
+// true: parameter p takes no gradient (the step has stopped, or p belongs to a
+// hidden layer the model does not use)
+__device__ __forceinline__ bool adam_skips(const AdamArgs& aa, int p, int step, bool stopped) {
     if (stopped) {
         if (p == MLP_NPARAM && aa.loss_out)
             aa.loss_out[aa.loss_slot_by_step ? step - aa.loss_base : 0] = __int_as_float(0x7fc00000);
-        return;
+        return true;
     }
-    if (p >= aa.frozen_lo && p < aa.frozen_hi) {  // a hidden layer the model does not use
+    if (p >= aa.frozen_lo && p < aa.frozen_hi) {
         if (aa.grad_out) aa.grad_out[p] = 0.f;
-        return;
+        return true;
     }
+    return false;
+}
+
+// Parameter p's update from g, the sum of its partials in CTA order.
+__device__ __forceinline__ void adam_apply(const AdamArgs& aa, int p, int step, float g) {
     // explicit roundings (no FMA contraction left to the compiler): the two
     // kernels that inline this must issue the same operations
-    // CTA order, sixteen loads in flight at a time
-    const float* src = aa.partial + p;
-    constexpr size_t STRIDE = MLP_NPARAM + 1;
-    float g = 0.f;
-    int c = 0;
-    for (; c + 16 <= aa.nparts; c += 16) {
-        float v[16];
-#pragma unroll
-        for (int u = 0; u < 16; ++u) v[u] = __ldcg(src + (size_t)(c + u) * STRIDE);
-#pragma unroll
-        for (int u = 0; u < 16; ++u) g = __fadd_rn(g, v[u]);
-    }
-    for (; c < aa.nparts; ++c) g = __fadd_rn(g, __ldcg(src + (size_t)c * STRIDE));
     g = __fmul_rn(g, aa.inv_batch);
     if (p == MLP_NPARAM) {
         if (aa.loss_out) aa.loss_out[aa.loss_slot_by_step ? step - aa.loss_base : 0] = g;
@@ -120,6 +114,24 @@ __device__ __forceinline__ void adam_param(const AdamArgs& aa, int p, int step, 
         const int hi = half_index(p);
         if (hi >= 0) aa.w16[hi] = __float2half_rn(w);
     }
+}
+
+__device__ __forceinline__ void adam_param(const AdamArgs& aa, int p, int step, bool stopped) {
+    if (adam_skips(aa, p, step, stopped)) return;
+    // CTA order, sixteen loads in flight at a time
+    const float* src = aa.partial + p;
+    constexpr size_t STRIDE = MLP_NPARAM + 1;
+    float g = 0.f;
+    int c = 0;
+    for (; c + 16 <= aa.nparts; c += 16) {
+        float v[16];
+#pragma unroll
+        for (int u = 0; u < 16; ++u) v[u] = __ldcg(src + (size_t)(c + u) * STRIDE);
+#pragma unroll
+        for (int u = 0; u < 16; ++u) g = __fadd_rn(g, v[u]);
+    }
+    for (; c < aa.nparts; ++c) g = __fadd_rn(g, __ldcg(src + (size_t)c * STRIDE));
+    adam_apply(aa, p, step, g);
 }
 
 }  // namespace mlp

@@ -73,6 +73,9 @@ static_assert(O_W2 % 1024 == 0 && O_W3 % 1024 == 0 && O_WT2 % 1024 == 0 && O_WT3
               "128B-swizzled tiles need 1024-byte alignment");
 static_assert(O_ONES % 256 == 0 && O_BIAS % 256 == 0 && O_W1 % 256 == 0, "SW32 alignment");
 static_assert(TT_SMEM <= 227 * 1024, "shared memory");
+// the optimiser's share of the partials (one a CTA and parameter, rounded up to
+// whole shares) lies below the floats
+static_assert((MLP_NPARAM + 1 + 512) * 4 <= O_F, "staged partials");
 
 constexpr uint32_t ID64 = tc::idesc_f16_f32(128, 64);
 constexpr uint32_t ID80 = tc::idesc_f16_f32(128, 80);
@@ -125,7 +128,12 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
 // (a wait that ran out plus its drain) -- and sets status bit 2 when it runs
 // out; a CTA that failed a wait set its bit before arriving, so after the
 // barrier every CTA sees it and no slice is updated.
-__device__ void fused_adam(const TrainArgs& ta, int step, int* flag) {
+// Each CTA then takes an even share of the parameters: all its partials are brought
+// into shared memory at once (nothing else is in it any more unless a wait failed,
+// and then nothing is updated) and summed from there in CTA order.  (With 128
+// parameters on each of 75 CTAs, each thread reading its 128 partials 16 at a time,
+// the step took 35.7 us, 34.9 so.)
+__device__ void fused_adam(const TrainArgs& ta, int step, int* flag, float* stage) {
     if (threadIdx.x == 0) {
         __threadfence();
         const unsigned ticket = atomicAdd(ta.grid_bar, 1u);
@@ -145,11 +153,25 @@ __device__ void fused_adam(const TrainArgs& ta, int step, int* flag) {
     }
     __syncthreads();
     const bool stopped = *flag != 0;
-    // 128 parameters per CTA (the first four warps), so that the slices spread
-    // over as many SMs as there are
-    if (threadIdx.x < 128)
-        for (int p = blockIdx.x * 128 + threadIdx.x; p <= MLP_NPARAM; p += gridDim.x * 128)
-            mlp::adam_param(ta.adam, p, step, stopped);
+    const int span = (MLP_NPARAM + 1 + (int)gridDim.x - 1) / (int)gridDim.x;
+    const int p0 = (int)blockIdx.x * span, np = min(span, MLP_NPARAM + 1 - p0);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (!stopped) {
+        for (int j = lane; j < np; j += 32) {
+            const float* src = ta.adam.partial + p0 + j;
+#pragma unroll 8
+            for (int c = warp; c < ta.adam.nparts; c += TT_THREADS / 32)
+                stage[c * span + j] = __ldcg(src + (size_t)c * (MLP_NPARAM + 1));
+        }
+        __syncthreads();
+    }
+    for (int j = threadIdx.x; j < np; j += TT_THREADS) {
+        if (mlp::adam_skips(ta.adam, p0 + j, step, stopped)) continue;
+        float g = 0.f;
+#pragma unroll 16
+        for (int c = 0; c < ta.adam.nparts; ++c) g = __fadd_rn(g, stage[c * span + j]);
+        mlp::adam_apply(ta.adam, p0 + j, step, g);
+    }
     if (blockIdx.x == 0 && threadIdx.x == 0 && !stopped) *ta.adam.step = step + 1;
 }
 
@@ -502,7 +524,8 @@ __global__ void __launch_bounds__(TT_THREADS, 1) k_mlp_train_tc(TrainArgs ta) {
     tc::fence_before_sync();
     __syncthreads();
     if (warp == 0) tc::tmem_dealloc(tmem, TT_COLS);
-    if (ta.grid_bar) fused_adam(ta, step0, reinterpret_cast<int*>(fmisc + 8));
+    if (ta.grid_bar)
+        fused_adam(ta, step0, reinterpret_cast<int*>(fmisc + 8), reinterpret_cast<float*>(base));
 }
 
 using TrainFn = void (*)(TrainArgs);
