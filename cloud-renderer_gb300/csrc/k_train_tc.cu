@@ -203,8 +203,36 @@ __global__ void __launch_bounds__(TT_THREADS, 1) k_mlp_train_tc(TrainArgs ta) {
     const int row = tid & 127, part = tid >> 7, wq = warp & 3;
     const int c0 = part * CW;
 
-    // ---- weights (FP16 image) of the NL hidden layers, the transposes of
-    // layers 2 .. NL, biases, ones
+    // ---- the row's features and target are fetched first: a random row each, the
+    // longest latency of the prologue (a part takes four of the 16 features; with
+    // part 0 reading all after the weights, and the transposes gathered from global
+    // memory before the first product, a step took 34.9 us, 33.7 so)
+    const int step0 = ta.step ? *ta.step : 0;
+    const long long r = (long long)blockIdx.x * 128 + row;
+    bool valid;
+    long long idx;
+    if (ta.sequential) {
+        idx = ta.offset + r;
+        valid = idx < ta.N;
+    } else {
+        // lin * perm_mul mod N with both factors reduced mod N first (perm_mul
+        // < N from the host, N <= 2^31): the product stays below 2^62 for any
+        // step count, so the walk remains a permutation of the rows
+        const unsigned long long N = (unsigned long long)ta.N;
+        const unsigned long long lin = ((unsigned long long)step0 * (unsigned long long)ta.batch +
+                                        (unsigned long long)r) % N;
+        idx = (long long)((lin * ta.perm_mul) % N);
+        valid = true;
+    }
+    const float tau = valid && part == 0 ? ta.tau[idx] : -1.f;  // < 0: padding row
+    const float* xsrc = ta.feat + (size_t)(valid ? idx : 0) * MLP_IN + 4 * part;
+    float4 xf = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (valid)
+        xf = (reinterpret_cast<uintptr_t>(ta.feat) & 15) == 0
+                 ? __ldg(reinterpret_cast<const float4*>(xsrc))
+                 : make_float4(xsrc[0], xsrc[1], xsrc[2], xsrc[3]);
+
+    // ---- weights (FP16 image) of the NL hidden layers, biases, ones
     for (int i = tid; i < 64 * 2; i += TT_THREADS) {
         const int r = i >> 1, c = i & 1;
         *reinterpret_cast<uint4*>(base + O_W1 + tc::sw32_offset(r, c)) =
@@ -214,17 +242,10 @@ __global__ void __launch_bounds__(TT_THREADS, 1) k_mlp_train_tc(TrainArgs ta) {
     for (int l = 1; l < NL; ++l) {
         const int src = l == 1 ? MLP_H_W2 : MLP_H_W3;
         uint8_t* w = base + (l == 1 ? O_W2 : O_W3);
-        uint8_t* wt = base + (l == 1 ? O_WT2 : O_WT3);
         for (int i = tid; i < 64 * 8; i += TT_THREADS) {
             const int r = i >> 3, c = i & 7;
             *reinterpret_cast<uint4*>(w + tc::sw128_offset(r, c)) =
                 *reinterpret_cast<const uint4*>(ta.w16 + src + r * 64 + 8 * c);
-            // W^T row r (input r), K = outputs 8c .. 8c+7
-            __align__(16) __half t[8];
-#pragma unroll
-            for (int q = 0; q < 8; ++q) t[q] = ta.w16[src + (8 * c + q) * 64 + r];
-            *reinterpret_cast<uint4*>(wt + tc::sw128_offset(r, c)) =
-                *reinterpret_cast<const uint4*>(t);
         }
     }
     for (int r = tid; r < 64; r += TT_THREADS) fw4[r] = __half2float(ta.w16[MLP_H_W4 + r]);
@@ -261,37 +282,14 @@ __global__ void __launch_bounds__(TT_THREADS, 1) k_mlp_train_tc(TrainArgs ta) {
         }
     }
 
-    // ---- the row's features (normalised, FP16) into x (part 0)
-    const int step0 = ta.step ? *ta.step : 0;
-    const long long r = (long long)blockIdx.x * 128 + row;
-    bool valid;
-    long long idx;
-    if (ta.sequential) {
-        idx = ta.offset + r;
-        valid = idx < ta.N;
-    } else {
-        // lin * perm_mul mod N with both factors reduced mod N first (perm_mul
-        // < N from the host, N <= 2^31): the product stays below 2^62 for any
-        // step count, so the walk remains a permutation of the rows
-        const unsigned long long N = (unsigned long long)ta.N;
-        const unsigned long long lin = ((unsigned long long)step0 * (unsigned long long)ta.batch +
-                                        (unsigned long long)r) % N;
-        idx = (long long)((lin * ta.perm_mul) % N);
-        valid = true;
-    }
-    float tau = -1.f;  // < 0: padding row
-    if (part == 0) {
-        __align__(16) __half xh[16];
-#pragma unroll
-        for (int j = 0; j < MLP_IN; ++j) {
-            const float f = valid ? ta.feat[(size_t)idx * MLP_IN + j] : 0.f;
-            xh[j] = __float2half_rn((f - ta.mu[j]) * ta.inv_sd[j]);
-        }
-        tau = valid ? ta.tau[idx] : -1.f;
-#pragma unroll
-        for (int c = 0; c < 2; ++c)
-            *reinterpret_cast<uint4*>(base + O_X + tc::sw128_offset(row, c)) =
-                *reinterpret_cast<const uint4*>(xh + 8 * c);
+    // ---- the row's features (normalised, FP16) into x
+    {
+        const int j = 4 * part;
+        const uint2 xh = make_uint2(h2u(__floats2half2_rn((xf.x - ta.mu[j]) * ta.inv_sd[j],
+                                                          (xf.y - ta.mu[j + 1]) * ta.inv_sd[j + 1])),
+                                    h2u(__floats2half2_rn((xf.z - ta.mu[j + 2]) * ta.inv_sd[j + 2],
+                                                          (xf.w - ta.mu[j + 3]) * ta.inv_sd[j + 3])));
+        *reinterpret_cast<uint2*>(base + O_X + tc::sw128_offset(row, part >> 1) + 8 * (part & 1)) = xh;
     }
 
     if (tid == 0) {
@@ -328,6 +326,24 @@ __global__ void __launch_bounds__(TT_THREADS, 1) k_mlp_train_tc(TrainArgs ta) {
             tc::mma_f16(tmem, tc::desc_sw32(sb + O_ONES, 0u), tc::desc_sw32(sb + O_BIAS + 2048u * l),
                         ID64, 1u);
             tc::mma_commit(bar);
+        }
+        // while the first product runs: the transposes of layers 2 .. NL, which
+        // the backward pass takes (row = input, K = outputs 8c .. 8c + 7)
+        if (l == 0) {
+#pragma unroll
+            for (int k = 1; k < NL; ++k) {
+                const uint8_t* w = base + (k == 1 ? O_W2 : O_W3);
+                uint8_t* wt = base + (k == 1 ? O_WT2 : O_WT3);
+                for (int i = tid; i < 64 * 8; i += TT_THREADS) {
+                    const int in = i & 63, c = i >> 6;
+                    __align__(16) __half t[8];
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        t[q] = *reinterpret_cast<const __half*>(w + kt_addr(8 * c + q, in, 0));
+                    *reinterpret_cast<uint4*>(wt + tc::sw128_offset(in, c)) =
+                        *reinterpret_cast<const uint4*>(t);
+                }
+            }
         }
         wait();
         if (!bad) {
