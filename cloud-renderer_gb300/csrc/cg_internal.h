@@ -252,6 +252,9 @@ struct SampleBuf {
 #define MLP_W4 9408
 #define MLP_B4 9472
 #define MLP_NPARAM 9473
+// floats of one CTA's gradient partials: the parameters and the loss, padded for
+// 16-byte stores
+#define MLP_PART_STRIDE ((MLP_NPARAM + 1 + 3) / 4 * 4)
 // FP16 weight image: W1 [64][16], W2 [64][64], W3 [64][64], W4 [8][64] (rows 1-7 zero)
 #define MLP_H_W1 0
 #define MLP_H_W2 1024
@@ -351,7 +354,7 @@ struct TrainArgs {
     float tau_scale, sigma;
     const float* params;
     const __half* w16;
-    float* partial;   // [ctas][MLP_NPARAM + 1]
+    float* partial;   // [ctas][MLP_PART_STRIDE]
     const int* step;  // device step counter (NULL: 0)
     int layers;       // hidden layers (1 .. MLP_MAX_LAYERS)
     int batch;

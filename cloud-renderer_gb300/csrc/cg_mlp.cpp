@@ -501,7 +501,7 @@ extern "C" cg_status cg_mlp_gradient(cg_mlp* m, const float* features, const flo
     if (st != CG_OK) return st;
     const int ctas = (n + 127) / 128;
     CG_CUDA(cudaStreamSynchronize(s));
-    CG_CUDA(m->partial.ensure((size_t)ctas * (MLP_NPARAM + 1) * 4));
+    CG_CUDA(m->partial.ensure((size_t)ctas * MLP_PART_STRIDE * 4));
     CG_CUDA(cudaMemsetAsync(m->status.p, 0, 16, s));
     TrainArgs ta = train_args(m, df, dt, n, sigma);
     ta.sequential = 1;
@@ -598,7 +598,7 @@ static cg_status train_impl(cg_mlp* m, const float* d_features, const float* d_t
     cudaStream_t s = ctx->stream;
     const int ctas = tp->batch / 128;
     CG_CUDA(cudaStreamSynchronize(s));
-    CG_CUDA(m->partial.ensure((size_t)ctas * (MLP_NPARAM + 1) * 4));
+    CG_CUDA(m->partial.ensure((size_t)ctas * MLP_PART_STRIDE * 4));
     CG_CUDA(m->loss.ensure((size_t)tp->steps * 4));
     // multiplier coprime with n, from the seed
     static const unsigned long long primes[] = {2654435761ull, 2246822519ull, 3266489917ull,

@@ -120,7 +120,7 @@ __device__ __forceinline__ void adam_param(const AdamArgs& aa, int p, int step, 
     if (adam_skips(aa, p, step, stopped)) return;
     // CTA order, sixteen loads in flight at a time
     const float* src = aa.partial + p;
-    constexpr size_t STRIDE = MLP_NPARAM + 1;
+    constexpr size_t STRIDE = MLP_PART_STRIDE;
     float g = 0.f;
     int c = 0;
     for (; c + 16 <= aa.nparts; c += 16) {
