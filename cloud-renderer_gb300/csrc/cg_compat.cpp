@@ -209,6 +209,7 @@ extern "C" cg_status cg_render_compat(cg_context* ctx, const cg_volume* v, const
     P.noise = ctx->compat_noise.as<const ulonglong2>();
     {
         // below noise_reach, |(c + off) fr N - 1/2| stays under 2^21 in every octave
+        // (the margin to 2.0e6 covers the roundings of 4096 added steps)
         double top = 1.0, off = 0.0;
         float fr = 1.f, pe = 1.f;
         for (int k = 0; k < P.octaves; ++k) {

@@ -245,12 +245,15 @@ __device__ bool compat_fragment(const VolDesc& vd, const ConeSchedule& cs, const
         const float lx = ex / (is - 1.f), ly = ey / (is - 1.f), lz = ez / (is - 1.f);
         const float oa = P.noise_opacity / (is - 1.f), la = 1.f / (is - 1.f);
         float ro = 0.f, rl = 0.f;
-        // the samples lie between the near and the far point, so their largest
-        // coordinate is known before they are taken
-        const float reach = fmaxf(fmaxf(fmaxf(fabsf(cx), fabsf(cy)), fabsf(cz)),
-                                  fmaxf(fmaxf(fabsf(cx + ex), fabsf(cy + ey)), fabsf(cz + ez)));
-        const bool near = reach < P.noise_reach;
+        // the samples run from the near point to the last one, which lies past the far
+        // point where the step count is no whole number (by a chord, at two steps and
+        // a little), so their largest coordinate is known before they are taken
         const int steps = (int)ceilf(is);
+        const float span = (float)(steps - 1);
+        const float reach = fmaxf(fmaxf(fmaxf(fabsf(cx), fabsf(cy)), fabsf(cz)),
+                                  fmaxf(fmaxf(fabsf(cx + span * lx), fabsf(cy + span * ly)),
+                                        fabsf(cz + span * lz)));
+        const bool near = reach < P.noise_reach;
         for (int i = 0; i < steps; ++i) {
             // the cells' green and alpha
             const float2 ga = halves(near ? noise_sum_near(P, cx, cy, cz)
