@@ -254,6 +254,8 @@ extern "C" cg_status cg_render_compat(cg_context* ctx, const cg_volume* v, const
     bins.cursor = bins.offset + words;
     // after the last board upload (made on the context stream)
     if (v->ready_pending && s != ctx->stream) CG_CUDA(cudaStreamWaitEvent(s, v->boards_ready, 0));
+    // (and the last render of them, so that boards_drawn follows every one)
+    if (v->draw_pending) CG_CUDA(cudaStreamWaitEvent(s, v->boards_drawn, 0));
     stage_begin(ctx, s);
     CG_CUDA(cudaMemsetAsync(base, 0, (4 + words) * 4, s));
     CG_LAUNCH(ctx, launch_compat_count(P, ctx->compat_rect.as<int4>(), ctx->compat_key.as<float>(),
@@ -274,6 +276,14 @@ extern "C" cg_status cg_render_compat(cg_context* ctx, const cg_volume* v, const
     CG_LAUNCH(ctx, launch_compat_tiles(vd, cs, P, bins, (uint32_t)total[1],
                                        ctx->compat_list.as<unsigned long long>(), out, s));
     stage_mark(ctx, s, "tiles");
+    // the next upload comes after the tiles, which still read the boards when a call
+    // with a device image returns
+    if (s != ctx->stream && out_on_device) {
+        if (!v->boards_drawn)
+            CG_CUDA(cudaEventCreateWithFlags(&v->boards_drawn, cudaEventDisableTiming));
+        CG_CUDA(cudaEventRecord(v->boards_drawn, s));
+        v->draw_pending = true;
+    }
     if (!out_on_device) {
         CG_CUDA(cudaMemcpyAsync(rgba_out, out, pixels * 16, cudaMemcpyDeviceToHost, s));
         CG_CUDA(cudaStreamSynchronize(s));

@@ -508,6 +508,7 @@ extern "C" void cg_volume_destroy(cg_volume* v) {
     v->h_stage.release();
     if (v->boards_ready) cudaEventDestroy(v->boards_ready);
     if (v->boards_read) cudaEventDestroy(v->boards_read);
+    if (v->boards_drawn) cudaEventDestroy(v->boards_drawn);
     for (int l = 0; l < CG_MAX_LEVELS; ++l) {
         if (v->tex_obj[l]) cudaDestroyTextureObject(v->tex_obj[l]);
         if (v->tex_surf[l]) cudaDestroySurfaceObject(v->tex_surf[l]);
@@ -669,12 +670,13 @@ extern "C" cg_status cg_volume_set_billboards(cg_volume* v, const float* positio
     // the device records, and behind them those that the sun-view pass keeps
     const size_t o_sun = (total + 255) / 256 * 256;
     const size_t need = o_sun + n * SUN_BOARD_BYTES;
-    // a voxelize still running on another stream reads the board buffers that
-    // this upload overwrites: it comes after it; where they are reallocated, so
-    // does the host
+    // a voxelize or a compat render still running on another stream reads the board
+    // buffers that this upload overwrites: it comes after them; where they are
+    // reallocated, so does the host
     if (v->read_pending) CG_CUDA(cudaStreamWaitEvent(s, v->boards_read, 0));
+    if (v->draw_pending) CG_CUDA(cudaStreamWaitEvent(s, v->boards_drawn, 0));
     if (need > v->boards.bytes || pairs * 4 > v->blist.bytes) CG_CUDA(cudaStreamSynchronize(s));
-    v->read_pending = false;
+    v->read_pending = v->draw_pending = false;
     CG_CUDA(v->boards.ensure(need));
     char* dev = v->boards.as<char>();
     v->cwr = reinterpret_cast<float4*>(dev + o_cwr);

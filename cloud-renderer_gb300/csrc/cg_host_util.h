@@ -197,6 +197,10 @@ struct cg_volume {
     // last voxelize that read the board buffers (direct or graph replay)
     cudaEvent_t boards_ready = nullptr, boards_read = nullptr;
     bool ready_pending = false, read_pending = false;
+    // the last compat render that blends the boards on a caller's stream (the event
+    // is made by the first one)
+    mutable cudaEvent_t boards_drawn = nullptr;
+    mutable bool draw_pending = false;
 };
 
 cg_status ensure_textures(cg_volume* v, cudaStream_t s);
