@@ -65,13 +65,17 @@ extern "C" cg_status cg_context_create(int device, cg_context** out) {
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->fork_ev, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->join_ev, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = c->fallbacks.ensure(32 + sizeof(InferStatus));
+    if (e == cudaSuccess) e = cudaMemsetAsync(c->fallbacks.p, 0, c->fallbacks.bytes, c->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) {
+        c->fallbacks.release();
         if (c->join_ev) cudaEventDestroy(c->join_ev);
         if (c->fork_ev) cudaEventDestroy(c->fork_ev);
         if (c->side) cudaStreamDestroy(c->side);
         if (c->stream) cudaStreamDestroy(c->stream);
         delete c;
-        return fail(CG_ERR_CUDA, "cudaStreamCreate: %s", cudaGetErrorString(e));
+        return fail(CG_ERR_CUDA, "cg_context_create: %s", cudaGetErrorString(e));
     }
     *out = c;
     return CG_OK;
@@ -139,7 +143,7 @@ extern "C" cg_status cg_context_bounds_violations(cg_context* ctx, uint64_t* cou
 extern "C" cg_status cg_context_last_samples(cg_context* ctx, uint64_t* samples) {
     CG_CHECK(ctx && samples, CG_ERR_INVALID_ARGUMENT, "cg_context_last_samples: null pointer");
     *samples = 0;
-    if (!ctx->fallbacks.p || !ctx->shaded_valid) return CG_OK;
+    if (!ctx->shaded_valid) return CG_OK;
     CG_CUDA(cudaSetDevice(ctx->device));
     CG_CUDA(cudaDeviceSynchronize());
     unsigned long long h[3] = {0, 0, 0};
@@ -1272,6 +1276,7 @@ extern "C" cg_status cg_render(cg_context* ctx, const cg_volume* v, const cg_cam
         if (st != CG_OK) return st;
         CG_CUDA(cudaMemsetAsync(ctx->fallbacks.p, 0, 32, s));
         ctx->shaded_valid = true;
+        ctx->infer_last = false;
         CG_LAUNCH(ctx, launch_render_mlp_tc(vd, cd, tp, md, contrib, steps, dst,
                                             ctx->fallbacks.as<unsigned long long>(), s));
         stage_mark(ctx, s, "render_mlp");
@@ -1290,6 +1295,7 @@ extern "C" cg_status cg_render(cg_context* ctx, const cg_volume* v, const cg_cam
         stage_mark(ctx, s, "march");
         if (params->use_mlp) {
             ctx->shaded_valid = true;
+            ctx->infer_last = false;
             CG_LAUNCH(ctx, launch_shade_mlp_tc(vd, cd, tp, md, sb,
                                                ctx->fallbacks.as<unsigned long long>(), s));
             stage_mark(ctx, s, "shade_mlp");

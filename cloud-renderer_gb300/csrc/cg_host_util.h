@@ -109,7 +109,14 @@ struct cg_context {
     NoiseTab noise_tab{};
     // deferred renderer: recorded view samples and the MLP fallback counter
     DevBuf samples_pw, samples_gl, samples_cnt, samples_c, samples_alpha;
-    DevBuf fallbacks;  // surrogate render status (see launch_shade_mlp_tc)
+    // surrogate render status (4 words, see launch_shade_mlp_tc), and behind it the
+    // inference launches' (InferStatus); zeroed with the context
+    DevBuf fallbacks;
+    unsigned long long infer_launch = 0;  // number of the last inference launch
+    bool infer_last = false;  // it came after the last surrogate render
+    InferStatus* infer_status() const {
+        return reinterpret_cast<InferStatus*>(fallbacks.as<unsigned long long>() + 4);
+    }
     DevBuf stats_scratch, stats_a, stats_ref;  // cg_image_error_stats staging
     // batch render: launch shape, descriptors (host, pinned staging, device
     // descriptors + tile counter)

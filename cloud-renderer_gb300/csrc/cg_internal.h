@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include "cg_check.cuh"
+#include "cg_infer_status.h"
 
 #define CG_MAX_LEVELS 16
 #define CG_Q20 1048576LL
@@ -419,10 +420,10 @@ cudaError_t launch_accumulate(CamDesc cam, TraceParams tp, SampleBuf sb, float4*
                               cudaStream_t st);
 cudaError_t launch_mlp_features(VolDesc vd, const MlpDev& m, const float* pos, int n,
                                 const float dir[3], float* out, cudaStream_t st);
-// network evaluation on the tensor cores (k_shade_tc.cu); status[1] |= 1 when
-// a tensor-core wait ran out of its time limit
+// network evaluation on the tensor cores (k_shade_tc.cu); status: how launch number
+// `launch` says that a tensor-core wait ran out of its time limit
 cudaError_t launch_mlp_infer(const MlpDev& m, const float* feat, int n, float* out,
-                             unsigned long long* status, cudaStream_t st);
+                             InferStatus* status, unsigned long long launch, cudaStream_t st);
 // one training step on the tensor cores (k_train_tc.cu); a tensor-core wait
 // that ran out of its time limit sets ta.status and leaves a NaN in the CTA's
 // loss slot

@@ -273,7 +273,6 @@ cg_status ensure_samples(cg_context* ctx, int width, int height, int view_steps,
         CG_CUDA(ctx->samples_cnt.ensure(idx_words * 4));
         CG_CUDA(ctx->samples_alpha.ensure(pixels * 4));
     }
-    CG_CUDA(ctx->fallbacks.ensure(32));
     sb.pos_w = ctx->samples_pw.as<float4>();
     sb.light_lane = ctx->samples_gl.as<float2>();
     sb.contrib = ctx->samples_c.as<float>();
@@ -305,7 +304,6 @@ cg_status ensure_render_slots(cg_context* ctx, int width, int height, int view_s
         CG_CUDA(ctx->samples_c.ensure(n * 4));
         CG_CUDA(ctx->samples_cnt.ensure(step_words * 4));
     }
-    CG_CUDA(ctx->fallbacks.ensure(32));
     contrib = ctx->samples_c.as<float>();
     steps = reinterpret_cast<uint2*>(ctx->samples_cnt.as<unsigned>());
     return CG_OK;
@@ -314,16 +312,28 @@ cg_status ensure_render_slots(cg_context* ctx, int width, int height, int view_s
 extern "C" cg_status cg_context_mlp_fallbacks(cg_context* ctx, uint64_t* out) {
     CG_CHECK(ctx && out, CG_ERR_INVALID_ARGUMENT, "cg_context_mlp_fallbacks: null pointer");
     *out = 0;
-    if (!ctx->fallbacks.p) return CG_OK;
     CG_CUDA(cudaSetDevice(ctx->device));
     CG_CUDA(cudaDeviceSynchronize());
-    unsigned long long h[2] = {0, 0};
-    CG_CUDA(cudaMemcpy(h, ctx->fallbacks.p, 16, cudaMemcpyDeviceToHost));
-    *out = h[0];
-    CG_CHECK((h[1] & 2ull) == 0, CG_ERR_DEVICE_FAULT,
+    struct {
+        unsigned long long render[4];
+        InferStatus infer;
+    } h = {};
+    CG_CUDA(cudaMemcpy(&h, ctx->fallbacks.p, sizeof(h), cudaMemcpyDeviceToHost));
+    if (h.infer.bits) {
+        CG_CUDA(cudaMemset(ctx->infer_status(), 0, sizeof(InferStatus)));  // taken
+        return fail(CG_ERR_DEVICE_FAULT,
+                    h.infer.bits & 2ull
+                        ? "cg_mlp_infer: a tensor-core wait ran out of its time limit (1 s) and "
+                          "the drain after it did not complete; the device must be treated as "
+                          "faulted"
+                        : "cg_mlp_infer: a tensor-core wait ran out of its time limit (1 s)");
+    }
+    if (ctx->infer_last) return CG_OK;
+    *out = h.render[0];
+    CG_CHECK((h.render[1] & 2ull) == 0, CG_ERR_DEVICE_FAULT,
              "surrogate render: a tensor-core wait ran out of its time limit (1 s) and the "
              "drain after it did not complete; the device must be treated as faulted");
-    CG_CHECK(h[1] == 0, CG_ERR_DEVICE_FAULT,
+    CG_CHECK(h.render[1] == 0, CG_ERR_DEVICE_FAULT,
              "surrogate render: a tensor-core wait ran out of its time limit (1 s)");
     return CG_OK;
 }
@@ -335,7 +345,6 @@ extern "C" cg_status cg_context_check_wait_timeout(cg_context* ctx, uint32_t lim
     CG_CHECK(limit_us >= 1 && limit_us <= 1000000, CG_ERR_OUT_OF_RANGE,
              "cg_context_check_wait_timeout: limit %u us not in [1, 1e6]", limit_us);
     CG_CUDA(cudaSetDevice(ctx->device));
-    CG_CUDA(ctx->fallbacks.ensure(32));
     cudaStream_t s = ctx->stream;
     CG_CUDA(cudaMemsetAsync(ctx->fallbacks.p, 0, 32, s));
     CG_LAUNCH(ctx, launch_wait_probe((uint64_t)limit_us * 1000ull,
@@ -344,7 +353,7 @@ extern "C" cg_status cg_context_check_wait_timeout(cg_context* ctx, uint32_t lim
     unsigned long long h[4] = {0, 0, 0, 0};
     CG_CUDA(cudaMemcpy(h, ctx->fallbacks.p, 32, cudaMemcpyDeviceToHost));
     *waited_us = h[3] / 1000ull;
-    ctx->shaded_valid = false;
+    ctx->shaded_valid = ctx->infer_last = false;
     CG_CHECK(h[1] == 0, CG_ERR_DEVICE_FAULT,
              "wait probe: the bounded mbarrier wait ran out after %llu us, as it must",
              (unsigned long long)(h[3] / 1000ull));
@@ -419,18 +428,16 @@ extern "C" cg_status cg_mlp_infer(const cg_mlp* m, const float* features, int n,
         CG_CUDA(tout.ensure((size_t)n * 4));
         dout = tout.as<float>();
     }
-    // the tensor-core status block: [1] records a wait that ran out (the kernel
-    // clears it first)
-    CG_CUDA(ctx->fallbacks.ensure(32));
     ctx->shaded_valid = false;
-    CG_LAUNCH(ctx, launch_mlp_infer(device_view(m), df, n, dout,
-                                    ctx->fallbacks.as<unsigned long long>(), s));
+    ctx->infer_last = true;
+    const unsigned long long launch = ++ctx->infer_launch;
+    CG_LAUNCH(ctx, launch_mlp_infer(device_view(m), df, n, dout, ctx->infer_status(), launch, s));
     if (!on_device) {
         CG_CUDA(cudaMemcpyAsync(out, dout, (size_t)n * 4, cudaMemcpyDeviceToHost, s));
-        unsigned long long h[2] = {0, 0};
-        CG_CUDA(cudaMemcpyAsync(h, ctx->fallbacks.p, 16, cudaMemcpyDeviceToHost, s));
+        InferStatus h{};
+        CG_CUDA(cudaMemcpyAsync(&h, ctx->infer_status(), sizeof(h), cudaMemcpyDeviceToHost, s));
         CG_CUDA(cudaStreamSynchronize(s));
-        CG_CHECK(h[1] == 0, CG_ERR_DEVICE_FAULT,
+        CG_CHECK(!infer_failed(h, launch), CG_ERR_DEVICE_FAULT,
                  "cg_mlp_infer: a tensor-core wait ran out of its time limit (1 s)");
     }
     return CG_OK;

@@ -125,13 +125,16 @@ __device__ __forceinline__ bool sync_for_mma(bool bad) {
 // After a failed barrier (CTA-uniform): drain the outstanding commit, bounded
 // (only warps whose wait ran out have one: no MMA is issued after a failed
 // barrier), agree across the CTA whether every drain completed, and report:
-// status[1] |= 1, and |= 2 when a drain ran out too (tensor memory is then
+// bits |= 1, and |= 2 when a drain ran out too (tensor memory is then
 // freed with an MMA possibly in flight: the host treats the device as faulted).
 __device__ __forceinline__ void report_failure(uint64_t* bar, unsigned phase, bool bad,
-                                               unsigned long long* status) {
+                                               InferStatus* status, unsigned long long launch) {
     const bool drained = !bad || tc::mbar_wait(bar, phase, TC_WAIT_NS);
     const bool undrained = __syncthreads_or(!drained) != 0;
-    if (threadIdx.x == 0) atomicOr(status + 1, undrained ? 3ull : 1ull);
+    if (threadIdx.x == 0) {
+        atomicOr(&status->bits, undrained ? 3ull : 1ull);
+        atomicMax(&status->launch, launch);
+    }
 }
 
 // ---- the shade kernel: SHADE_GROUPS independent 4-warp groups per CTA, each
@@ -336,13 +339,13 @@ __global__ void __launch_bounds__(128 * SHADE_GROUPS, ctas_per_sm<NL>())
 // staged weights, layers, epilogues and bounded waits.  A CTA has one or two tiles
 // behind one another, so its latencies show: a row is read 16 bytes at a time where
 // the caller's pointer allows, the first before the weights are staged, the next
-// while a tile is computed, and the status block is cleared here rather than by a
-// memset before (200,001 rows, two layers: 20.5 -> 18.5 us a call, 17.1 without
-// the memset; the tanh alone hold the special-function unit for 5.5).
+// while a tile is computed, and its status words need no memset before the launch
+// (200,001 rows, two layers: 20.5 -> 18.5 us a call, 17.1 without the memset; the
+// tanh alone hold the special-function unit for 5.5).
 template <int NL>
 __global__ void __launch_bounds__(128, ctas_per_sm<NL>())
     k_mlp_infer_tc(const __grid_constant__ MlpDev m, const float* feat, int n, float* out,
-                   unsigned long long* status) {
+                   InferStatus* status, unsigned long long launch) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = tc::smem_addr(smem_raw);
     uint8_t* base = smem_raw + (((raw + 1023u) & ~1023u) - raw);
@@ -350,8 +353,6 @@ __global__ void __launch_bounds__(128, ctas_per_sm<NL>())
     uint64_t* bar = reinterpret_cast<uint64_t*>(base + InferSmem<NL>::OFF_BAR);
     uint32_t* tslot = reinterpret_cast<uint32_t*>(base + InferSmem<NL>::OFF_BAR + 8);
     const int tid = threadIdx.x, warp = tid >> 5;
-    // (a wait that runs out is recorded a second later at the earliest)
-    if (blockIdx.x == 0 && tid < 4) status[tid] = 0ull;
     // this thread's row of a tile; rows past the end read the mean (input 0)
     const bool wide = (reinterpret_cast<uintptr_t>(feat) & 15) == 0;
     float4 f[4];
@@ -427,7 +428,7 @@ __global__ void __launch_bounds__(128, ctas_per_sm<NL>())
         if (row < n && !bad) out[row] = m.tau_scale * mlp::softplus(y);
     }
     if (!failed) failed = sync_for_mma(bad);  // the last tile's waits
-    if (failed) report_failure(bar, phase, bad, status);
+    if (failed) report_failure(bar, phase, bad, status, launch);
     tc::fence_before_sync();
     __syncthreads();
     if (warp == 0) tc::tmem_dealloc(tmem, TC_TMEM_COLS);
@@ -461,12 +462,12 @@ cudaError_t launch_wait_probe(uint64_t limit_ns, unsigned long long* status, cud
 }
 
 cudaError_t launch_mlp_infer(const MlpDev& m, const float* feat, int n, float* out,
-                             unsigned long long* status, cudaStream_t st) {
+                             InferStatus* status, unsigned long long launch, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
     if (m.layers < 1 || m.layers > MLP_MAX_LAYERS) return cudaErrorInvalidValue;
     // the shared-memory attributes and the SM count are set up once per device
     static std::atomic<int> sm_count[64];
-    using InferFn = void (*)(MlpDev, const float*, int, float*, unsigned long long*);
+    using InferFn = void (*)(MlpDev, const float*, int, float*, InferStatus*, unsigned long long);
     const InferFn fns[MLP_MAX_LAYERS] = {k_mlp_infer_tc<1>, k_mlp_infer_tc<2>, k_mlp_infer_tc<3>};
     const int smem[MLP_MAX_LAYERS] = {InferSmem<1>::BYTES, InferSmem<2>::BYTES,
                                       InferSmem<3>::BYTES};
@@ -489,7 +490,7 @@ cudaError_t launch_mlp_infer(const MlpDev& m, const float* feat, int n, float* o
     const int L = m.layers - 1;
     const int ntiles = (n + 127) / 128;
     const int blocks = std::min(sm_count[dev].load(std::memory_order_acquire) * per_sm[L], ntiles);
-    fns[L]<<<blocks, 128, smem[L], st>>>(m, feat, n, out, status);
+    fns[L]<<<blocks, 128, smem[L], st>>>(m, feat, n, out, status, launch);
     return cudaGetLastError();
 }
 

@@ -379,7 +379,8 @@ cg_status cg_image_error_stats(cg_context* ctx, const float* image, const void* 
                                double out[10], void* stream);
 /* Samples of the last MLP render that fell back to the exact cone.  Returns
  * CG_ERR_DEVICE_FAULT when that render's tensor-core pass stopped on a bounded
- * wait (the image is then incomplete). */
+ * wait (the image is then incomplete), or when a cg_mlp_infer did since the last
+ * such report. */
 cg_status cg_context_mlp_fallbacks(cg_context* ctx, uint64_t* out);
 /* View samples the last MLP render shaded (one surrogate inference each). */
 cg_status cg_context_last_samples(cg_context* ctx, uint64_t* samples);
