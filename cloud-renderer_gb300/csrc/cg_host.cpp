@@ -2,7 +2,6 @@
 // quantization, pass orchestration and readback.
 #include <cuda_runtime.h>
 
-#include <cfloat>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -10,6 +9,7 @@
 #include <string>
 #include <vector>
 
+#include "cg_boards.h"
 #include "cg_host_util.h"
 
 // ---------------------------------------------------------------------------
@@ -587,53 +587,6 @@ static cg_status check_boards(const cg_volume* v, const float* positions, const 
     return CG_OK;
 }
 
-// Every test of check_boards without its branches and divisions, and an upper
-// bound of the pairs: a board of radius rv voxels meets at most 2 rv + 1 voxels
-// an axis, n of which lie in at most floor((n + edge - 2) / edge) + 1 bricks or
-// bars.  False: check_boards has to look.  Copies the boards into `raw`.
-static bool boards_fine(const cg_volume* v, const float* positions, const float* scales,
-                        const float* densities, size_t n, float fluffiness, float* raw,
-                        size_t& pairs) {
-    float* const pos = raw;
-    float* const rad = raw + 3 * n;
-    float* const den = raw + 4 * n;
-    if (n) std::memcpy(pos, positions, n * 12);
-    if (n && densities) std::memcpy(den, densities, n * 4);
-    const float p0 = v->pos[0], p1 = v->pos[1], p2 = v->pos[2], big = FLT_MAX;
-    const float to_voxels = 2.0f * (float)v->D / v->range[0];
-    const float nb = (float)v->bins.nbx, nz = (float)v->bins.nbarz;
-    const float rb = 1.0f / CG_BRICK, rz = 1.0f / (float)v->bins.bar;
-    // integer sums and maxima (of the radii's bits): the compiler vectorizes them
-    int bad = 0, largest = 0;
-    double sum = 0.0;
-    for (size_t base = 0; base < n; base += 256) {
-        const size_t end = std::min(n, base + 256);
-        int part = 0;
-        for (size_t b = base; b < end; ++b) {
-            const float r = scales[b] * fluffiness;
-            rad[b] = r;
-            const float x = std::fabs(p0 + pos[3 * b]), y = std::fabs(p1 + pos[3 * b + 1]),
-                        z = std::fabs(p2 + pos[3 * b + 2]);
-            bad |= !(r >= 0.f) | !(r <= big) | !(x <= big) | !(y <= big) | !(z <= big);
-            int bits;
-            std::memcpy(&bits, &r, 4);
-            largest = std::max(largest, bits);
-            const float m = r * to_voxels * 1.001f + 1.01f;  // (a margin for the roundings)
-            const float kb = (m + (CG_BRICK - 2)) * rb + 1.f, kz = (m - 2.f) * rz + 2.f;
-            const int ib = (int)(kb < nb ? kb : nb), iz = (int)(kz < nz ? kz : nz);
-            part += ib * ib * iz;
-        }
-        sum += part;
-    }
-    if (densities)
-        for (size_t b = 0; b < n; ++b) bad |= !(den[b] >= 0.f) | !(den[b] < 32768.f);
-    if (bad || !(sum <= (double)(1u << 28))) return false;
-    pairs = (size_t)sum + 1;
-    float top;
-    std::memcpy(&top, &largest, 4);
-    return (double)top / (double)v->range[0] * (double)v->D <= (double)v->D;
-}
-
 // The boards' records are made on the device (k_boards, which has the rules)
 // from the raw lists in page-locked memory: made here they took 24 ns a board,
 // 105 us of an update of 4096 (21 now, 355 -> 45 of 16384), and the upload waited for the context's
@@ -666,7 +619,16 @@ extern "C" cg_status cg_volume_set_billboards(cg_volume* v, const float* positio
     CG_CUDA(v->h_stage.ensure(n * 20 + 16));
     float* raw = reinterpret_cast<float*>(v->h_stage.p);
     size_t pairs = 0;
-    if (!boards_fine(v, positions, scales, densities, n, fluffiness, raw, pairs)) {
+    BoardBox box;
+    for (int a = 0; a < 3; ++a) {
+        box.pos[a] = v->pos[a];
+        box.range[a] = v->range[a];
+    }
+    box.D = v->D;
+    box.nbx = v->bins.nbx;
+    box.nbz = v->bins.nbarz;
+    box.bar = v->bins.bar;
+    if (!boards_fine(box, positions, scales, densities, n, fluffiness, raw, pairs)) {
         const cg_status st =
             check_boards(v, positions, scales, densities, n, fluffiness, pairs);
         if (st != CG_OK) return st;
