@@ -622,6 +622,7 @@ extern "C" cg_status cg_volume_set_billboards(cg_volume* v, const float* positio
     BoardBox box;
     for (int a = 0; a < 3; ++a) {
         box.pos[a] = v->pos[a];
+        box.wmin[a] = v->wmin[a];
         box.range[a] = v->range[a];
     }
     box.D = v->D;
@@ -632,6 +633,11 @@ extern "C" cg_status cg_volume_set_billboards(cg_volume* v, const float* positio
         const cg_status st =
             check_boards(v, positions, scales, densities, n, fluffiness, pairs);
         if (st != CG_OK) return st;
+    } else if (pairs > BOARD_PAIRS_SHORT && pairs * 4 > v->blist.bytes) {
+        // a long list would have to grow: not by boards that lie outside the volume
+        // (where a quarter is not saved, it grows by the rough bound, once)
+        const size_t met = pairs_met(box, raw, n);
+        if (met < pairs / 4 * 3) pairs = met;
     }
     // the device records, and behind them those that the sun-view pass keeps
     const size_t o_sun = (total + 255) / 256 * 256;

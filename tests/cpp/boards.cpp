@@ -15,6 +15,7 @@ int main() {
         BoardBox g;
         for (int a = 0; a < 3; ++a) {
             g.pos[a] = 0.5f;
+            g.wmin[a] = 0.0f;
             g.range[a] = 1.0f;
         }
         g.D = D;
