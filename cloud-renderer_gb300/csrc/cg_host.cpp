@@ -63,6 +63,7 @@ extern "C" cg_status cg_context_create(int device, cg_context** out) {
     c->device = device;
     cudaError_t e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->clear, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->fork_ev, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->join_ev, cudaEventDisableTiming);
     if (e == cudaSuccess) e = c->fallbacks.ensure(32 + sizeof(InferStatus));
@@ -72,6 +73,7 @@ extern "C" cg_status cg_context_create(int device, cg_context** out) {
         c->fallbacks.release();
         if (c->join_ev) cudaEventDestroy(c->join_ev);
         if (c->fork_ev) cudaEventDestroy(c->fork_ev);
+        if (c->clear) cudaStreamDestroy(c->clear);
         if (c->side) cudaStreamDestroy(c->side);
         if (c->stream) cudaStreamDestroy(c->stream);
         delete c;
@@ -287,6 +289,7 @@ void context_release(cg_context* ctx) {
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
     cudaStreamSynchronize(ctx->side);
+    cudaStreamSynchronize(ctx->clear);
     ctx->image.release();
     ctx->packed.release();
     ctx->noise.release();
@@ -312,6 +315,7 @@ void context_release(cg_context* ctx) {
         if (e) cudaEventDestroy(e);
     cudaEventDestroy(ctx->fork_ev);
     cudaEventDestroy(ctx->join_ev);
+    cudaStreamDestroy(ctx->clear);
     cudaStreamDestroy(ctx->side);
     cudaStreamDestroy(ctx->stream);
     delete ctx;
@@ -439,13 +443,6 @@ extern "C" cg_status cg_volume_create(cg_context* ctx, int dimension, float boun
     v->total = off;
     const size_t n0 = (size_t)dimension * dimension * dimension;
     const size_t bpv = format == CG_FORMAT_RGBA32F ? 16 : 4;
-    cudaError_t e = cudaSuccess;
-    if (e == cudaSuccess) e = v->pyr.ensure(off * bpv);
-    if (e == cudaSuccess) e = v->count.ensure(n0 * 4);
-    if (e == cudaSuccess) e = v->dq.ensure(n0 * 4);
-    if (e == cudaSuccess) e = v->mask.ensure(n0);
-    if (e == cudaSuccess) e = v->scratch.ensure(64);
-    if (e == cudaSuccess) e = cudaMemsetAsync(v->scratch.p, 0, 64, ctx->stream);
     // raw 4^3-cell grids (written by the splat) followed by the dilated brick
     // grids (at most as many bytes as the raw ones: bricks are >= 4 texels)
     int raw_total = 0;
@@ -467,28 +464,63 @@ extern "C" cg_status cg_volume_create(cg_context* ctx, int dimension, float boun
         cells += p * p * (p + 1);
     }
     v->quad_total = (int)cells;
-    if (cells > 0) {
-        const size_t bytes = cells * (format == CG_FORMAT_RGBA32F ? 16 : 8);
-        if (e == cudaSuccess) e = v->quads.ensure(bytes);
-        if (e == cudaSuccess) e = cudaMemsetAsync(v->quads.p, 0, bytes, ctx->stream);
-    }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     set_occ_layout(v, 4);  // the autotuner's pick on the batching and 1080p workloads
-    // + the level-0 occupied box (6 ints) after the grids, 16-byte aligned
-    if (e == cudaSuccess) e = v->occ.ensure(occ_box_offset(raw_total) + 32);
     const int nb = (dimension + CG_BRICK - 1) / CG_BRICK;
     v->bins.nbx = v->bins.nby = v->bins.nbz = nb;
     v->bins.nbricks = nb * nb * nb;
     v->bins.bar = splat_bar(dimension);
     v->bins.nbarz = (dimension + v->bins.bar - 1) / v->bins.bar;
     v->bins.nbins = nb * nb * v->bins.nbarz;
-    if (e == cudaSuccess) e = v->bcount.ensure(((size_t)v->bins.nbins + 1) * 4);
-    if (e == cudaSuccess) e = v->boff.ensure((size_t)v->bins.nbins * 4);
-    if (e == cudaSuccess) e = v->bcursor.ensure((size_t)v->bins.nbins * 4);
-    // every brick starts dirty: the pyramid's memory is uninitialised
-    if (e == cudaSuccess) e = v->bdirty.ensure((size_t)v->bins.nbricks);
-    if (e == cudaSuccess) e = cudaMemset(v->bdirty.p, 1, (size_t)v->bins.nbricks);
-    if (e == cudaSuccess) e = v->bhl.ensure((size_t)v->bins.nbricks);
+    // Few allocations (a volume made and destroyed in turn, us of cudaMalloc and of
+    // cudaFree: 256^3 RGBA32F 226 + 496 with one for each buffer, 143 + 246 in one, 129 +
+    // 406 in three; 512^3 BF16 294 + 1485, 536 + 866 and 211 + 1355: a large block that
+    // was just freed is slow to come back whole, so large volumes take three)
+    const size_t nbricks = (size_t)v->bins.nbricks, nbins = (size_t)v->bins.nbins;
+    const size_t quad_bytes = cells * (format == CG_FORMAT_RGBA32F ? 16 : 8);
+    const struct {
+        DevBuf* buf;
+        size_t bytes;
+        int block;  // of a large volume
+    } parts[] = {
+        {&v->pyr, off * bpv, 0},
+        {&v->count, n0 * 4, 1},
+        {&v->dq, n0 * 4, 1},
+        {&v->mask, n0, 2},
+        {&v->bcount, (nbins + 1) * 4, 2},
+        {&v->boff, nbins * 4, 2},
+        {&v->bcursor, nbins * 4, 2},
+        {&v->bhl, nbricks, 2},
+        // + the level-0 occupied box (6 ints) after the grids, 16-byte aligned
+        {&v->occ, occ_box_offset(raw_total) + 32, 2},
+        {&v->bdirty, nbricks, 2},
+        {&v->scratch, 64, 2},  // (next to the quads: one clear)
+        {&v->quads, quad_bytes, 2},
+    };
+    auto padded = [](size_t bytes) { return (bytes + 255) & ~(size_t)255; };
+    size_t total = 0, block_bytes[3] = {0, 0, 0};
+    for (const auto& p : parts) total += padded(p.bytes);
+    const bool large = total > ((size_t)512 << 20);
+    for (const auto& p : parts) block_bytes[large ? p.block : 0] += padded(p.bytes);
+    cudaError_t e = cudaSuccess;
+    char* at[3] = {nullptr, nullptr, nullptr};
+    for (int k = 0; k < (large ? 3 : 1); ++k) {
+        if (e == cudaSuccess) e = v->fixed[k].ensure(block_bytes[k]);
+        at[k] = v->fixed[k].as<char>();
+    }
+    if (e == cudaSuccess) {
+        for (const auto& p : parts) {
+            char*& next = at[large ? p.block : 0];
+            if (p.bytes) p.buf->p = next;
+            p.buf->bytes = p.bytes;
+            next += padded(p.bytes);
+        }
+        // every brick starts dirty: the pyramid's memory is uninitialised
+        e = cudaMemsetAsync(v->bdirty.p, 1, nbricks, ctx->clear);
+    }
+    if (e == cudaSuccess) e = cudaMemsetAsync(v->scratch.p, 0, padded(64) + quad_bytes, ctx->clear);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&v->cleared, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventRecord(v->cleared, ctx->clear);
+    v->clear_pending = true;
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&v->boards_ready, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&v->boards_read, cudaEventDisableTiming);
     if (e != cudaSuccess) {
@@ -504,12 +536,11 @@ extern "C" void cg_volume_destroy(cg_volume* v) {
     if (!v) return;
     cudaSetDevice(v->ctx->device);
     cudaStreamSynchronize(v->ctx->stream);
-    DevBuf* bufs[] = {&v->pyr, &v->count, &v->dq, &v->mask, &v->boards,
-                      &v->bcount, &v->boff, &v->bcursor, &v->blist,
-                      &v->bdirty, &v->bhl,
-                      &v->keys, &v->posmap, &v->scratch, &v->occ, &v->quads};
+    DevBuf* bufs[] = {&v->fixed[0], &v->fixed[1], &v->fixed[2], &v->boards,
+                      &v->blist,    &v->keys,     &v->posmap};
     for (DevBuf* b : bufs) b->release();
     v->h_stage.release();
+    if (v->cleared) cudaEventDestroy(v->cleared);
     if (v->boards_ready) cudaEventDestroy(v->boards_ready);
     if (v->boards_read) cudaEventDestroy(v->boards_read);
     if (v->boards_drawn) cudaEventDestroy(v->boards_drawn);
@@ -869,6 +900,8 @@ cg_status voxelize_on(cg_volume* v, const cg_sun* sun, cudaStream_t s, const Vox
     const bool capturing = cap != cudaStreamCaptureStatusNone;
     if (v->ready_pending && s != ctx->stream && !capturing)
         CG_CUDA(cudaStreamWaitEvent(s, v->boards_ready, 0));
+    // (a captured voxelize is never a volume's first: that one allocates its sun map)
+    if (v->clear_pending && !capturing) CG_CUDA(cudaStreamWaitEvent(s, v->cleared, 0));
     stage_begin(ctx, s);
     // clearGPU (CloudVolume.cpp:96-100) + clearPositionMap (VoxelizeShader.cpp:185-187):
     // what the sun-view pass needs is cleared on s, the rest beside it on the
@@ -931,6 +964,7 @@ cg_status voxelize_on(cg_volume* v, const cg_sun* sun, cudaStream_t s, const Vox
         CG_CUDA(cudaEventRecord(v->boards_read, s));
         v->read_pending = true;
     }
+    v->clear_pending = v->clear_pending && capturing;
     v->voxelized = true;
     v->boards_dirty = false;
     v->gen++;

@@ -85,6 +85,7 @@ struct cg_context {
     // run on `side`, forked and joined by two events
     cudaStream_t side = nullptr;
     cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
+    cudaStream_t clear = nullptr;  // a new volume's clears, beside whatever is queued
     uint64_t launches = 0;
     int refs = 1;  // the caller's handle + one per volume / model created on it
     bool shaded_valid = false;  // the status words hold a surrogate render's counters
@@ -153,7 +154,13 @@ struct cg_volume {
     int dims[CG_MAX_LEVELS];
     size_t offs[CG_MAX_LEVELS];
     size_t total = 0;
+    // the buffers whose sizes the volume's shape gives are parts of these (pyr, count,
+    // dq, mask, bcount, boff, bcursor, bdirty, bhl, scratch, quads, occ)
+    DevBuf fixed[3];
     DevBuf pyr, count, dq, mask;
+    // the clears of a new volume: the first voxelize comes after them
+    cudaEvent_t cleared = nullptr;
+    bool clear_pending = false;
     // boards
     int n = 0;
     size_t n_staged = 0;  // boards of the last upload (read from h_stage until boards_ready)
