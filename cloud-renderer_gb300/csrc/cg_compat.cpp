@@ -148,31 +148,23 @@ extern "C" cg_status cg_render_compat(cg_context* ctx, const cg_volume* v, const
     if (st != CG_OK) return st;
     CG_CUDA(cudaSetDevice(ctx->device));
     cudaStream_t s = pick_stream(ctx, stream);
-    // the noise map's green and alpha channels (the fragment program reads no other)
-    if (!ctx->compat_noise_valid || ctx->compat_seed != params->noise_seed) {
-        std::vector<float> rgba((size_t)NOISE_N * NOISE_N * NOISE_N * 4);
+    // the noise map's green and alpha channels (the fragment program reads no other),
+    // from which the device makes the cells; valid once this call has waited for s
+    const bool new_noise = !ctx->compat_noise_valid || ctx->compat_seed != params->noise_seed;
+    if (new_noise) {
+        constexpr size_t texels = (size_t)NOISE_N * NOISE_N * NOISE_N;
+        std::vector<float> rgba(texels * 4), ga(texels * 2);
         noise_map(params->noise_seed, rgba.data());
-        std::vector<float> cells(rgba.size() * 4);
-        constexpr size_t W = NOISE_N - 1;
-        auto at = [&](size_t x, size_t y, size_t z, int c) {
-            return rgba[(((z & W) * NOISE_N + (y & W)) * NOISE_N + (x & W)) * 4 + c];
-        };
-        float* o = cells.data();
-        for (size_t z = 0; z < NOISE_N; ++z)
-            for (size_t y = 0; y < NOISE_N; ++y)
-                for (size_t x = 0; x < NOISE_N; ++x)
-                    for (size_t k = 0; k < 4; ++k, o += 4)
-                        for (int c = 0; c < 2; ++c) {
-                            const float a = at(x, y + (k & 1), z + (k >> 1), 2 * c + 1);
-                            o[c] = a;
-                            o[2 + c] = at(x + 1, y + (k & 1), z + (k >> 1), 2 * c + 1) - a;
-                        }
+        for (size_t i = 0; i < texels; ++i) {
+            ga[2 * i] = rgba[4 * i + 1];
+            ga[2 * i + 1] = rgba[4 * i + 3];
+        }
         CG_CUDA(cudaStreamSynchronize(s));
-        CG_CUDA(ctx->compat_noise.ensure(cells.size() * 4));
-        CG_CUDA(cudaMemcpy(ctx->compat_noise.p, cells.data(), cells.size() * 4,
-                           cudaMemcpyHostToDevice));
-        ctx->compat_noise_valid = true;
-        ctx->compat_seed = params->noise_seed;
+        ctx->compat_noise_valid = false;
+        CG_CUDA(ctx->compat_noise.ensure(texels * (64 + 8)));
+        float2* map = reinterpret_cast<float2*>(ctx->compat_noise.as<char>() + texels * 64);
+        CG_CUDA(cudaMemcpyAsync(map, ga.data(), texels * 8, cudaMemcpyHostToDevice, s));
+        CG_LAUNCH(ctx, launch_compat_noise(map, ctx->compat_noise.as<float4>(), s));
     }
     const size_t pixels = (size_t)cam->width * cam->height;
     float4* out = reinterpret_cast<float4*>(rgba_out);
@@ -264,6 +256,10 @@ extern "C" cg_status cg_render_compat(cg_context* ctx, const cg_volume* v, const
     uint64_t* total = reinterpret_cast<uint64_t*>(ctx->compat_total.p);
     CG_CUDA(cudaMemcpyAsync(total, pairs64, 16, cudaMemcpyDeviceToHost, s));
     CG_CUDA(cudaStreamSynchronize(s));
+    if (new_noise) {
+        ctx->compat_noise_valid = true;
+        ctx->compat_seed = params->noise_seed;
+    }
     // the per-tile offsets are 32-bit
     CG_CHECK(*total < 0xFFFFFFFFull, CG_ERR_OUT_OF_RANGE,
              "cg_render_compat: %llu board-tile pairs exceed 2^32 (fewer boards or pixels)",

@@ -561,6 +561,8 @@ struct CompatDev {
     const ulonglong2* noise;
     float noise_reach;     // sample coordinates below this reach no large cell number
 };
+// CompatDev::noise (64 bytes a texel) from the map's green and alpha.
+cudaError_t launch_compat_noise(const float2* map, float4* cells, cudaStream_t st);
 // Per board: tile rectangle (x0, y0, x1, y1; empty when x0 > x1) and the
 // squared eye distance; per tile: the number of boards whose quad may cover it;
 // *pairs (64-bit) += every board's tile count.

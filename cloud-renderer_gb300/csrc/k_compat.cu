@@ -35,6 +35,19 @@ using namespace cgs::pairs;
 constexpr int CAP = 4096;      // most sort keys held in shared memory per tile
 constexpr int NOISE_N = 32;    // noise map edge (ConeTraceShader.cpp:12)
 
+// The noise map's cells (CompatDev::noise): thread 4 i + k makes corner k of texel i's,
+// REPEAT.  (A new seed, us beyond the render: 582 with a map of texels, 697 with the
+// cells made and uploaded by the host, 585 so, nearly all of it the host's map.)
+__global__ void __launch_bounds__(256) k_compat_noise(const float2* map, float4* cells) {
+    constexpr int M = NOISE_N - 1;
+    const int t = blockIdx.x * 256 + threadIdx.x, k = t & 3, i = t >> 2;
+    const int x = i & M, y = ((i / NOISE_N) + (k & 1)) & M,
+              z = (i / (NOISE_N * NOISE_N) + (k >> 1)) & M;
+    const int row = (z * NOISE_N + y) * NOISE_N;
+    const float2 a = map[row + x], b = map[row + ((x + 1) & M)];
+    cells[t] = make_float4(a.x, a.y, b.x - a.x, b.y - a.y);
+}
+
 // `parts` warps per board: lane 0 derives the board's tile rectangle, the lanes
 // split its tiles for the per-tile count.
 __global__ void k_compat_count(CompatDev P, int parts, int4* rect, float* key,
@@ -413,6 +426,11 @@ __global__ void __launch_bounds__(TILE_THREADS, 1280 / TILE_THREADS)
 }
 
 }  // namespace
+
+cudaError_t launch_compat_noise(const float2* map, float4* cells, cudaStream_t st) {
+    k_compat_noise<<<NOISE_N * NOISE_N * NOISE_N * 4 / 256, 256, 0, st>>>(map, cells);
+    return cudaGetLastError();
+}
 
 // Warps per board of the count and fill passes: about 8192 in all (200 boards over
 // 32400 tiles, one warp a board: the whole binning 66 us, 37 now).
