@@ -291,6 +291,8 @@ void context_release(cg_context* ctx) {
     cudaStreamSynchronize(ctx->side);
     cudaStreamSynchronize(ctx->clear);
     ctx->image.release();
+    ctx->rows_in.release();
+    ctx->rows_out.release();
     ctx->packed.release();
     ctx->noise.release();
     ctx->samples_pw.release();

@@ -59,6 +59,25 @@ struct DevBuf {
     }
 };
 
+// Device memory for the host rows of one call that waits for its result: up to KEPT
+// bytes in a buffer of the context's (grown, released with it), more in an allocation
+// given back with the call.
+struct RowBuf {
+    static constexpr size_t KEPT = (size_t)64 << 20;
+    DevBuf& kept;
+    DevBuf own;
+    explicit RowBuf(DevBuf& k) : kept(k) {}
+    ~RowBuf() { own.release(); }
+    RowBuf(const RowBuf&) = delete;
+    RowBuf& operator=(const RowBuf&) = delete;
+    cudaError_t ensure(size_t want, float*& p) {
+        DevBuf& b = want <= KEPT ? kept : own;
+        const cudaError_t e = b.ensure(want);
+        p = b.as<float>();
+        return e;
+    }
+};
+
 struct HostBuf {
     void* p = nullptr;
     size_t bytes = 0;
@@ -95,6 +114,7 @@ struct cg_context {
     cudaEvent_t marks[32] = {};
     char mark_names[32][24] = {};
     DevBuf image;  // render target when the caller passes a host pointer
+    DevBuf rows_in, rows_out;  // host rows of the surrogate's calls (RowBuf)
     DevBuf packed;  // cg_march_samples: offsets and a piece of the packed samples
     // hash-noise lattice tables of the last (noise parameters, world box)
     DevBuf noise;

@@ -360,16 +360,15 @@ extern "C" cg_status cg_context_check_wait_timeout(cg_context* ctx, uint32_t lim
     return CG_OK;
 }
 
-// Stage host inputs on the device when needed (tmp receives the copy).
-static cg_status stage_in(const float* src, size_t n, int on_device, DevBuf& tmp, const float*& dst,
-                          cudaStream_t s) {
-    if (on_device) {
-        dst = src;
-        return CG_OK;
-    }
-    CG_CUDA(tmp.ensure(n * 4));
-    CG_CUDA(cudaMemcpyAsync(tmp.p, src, n * 4, cudaMemcpyHostToDevice, s));
-    dst = tmp.as<const float>();
+// Stage host inputs on the device when needed (rows receives the copy).
+static cg_status stage_in(const float* src, size_t n, int on_device, RowBuf& rows,
+                          const float*& dst, cudaStream_t s) {
+    dst = src;
+    if (on_device) return CG_OK;
+    float* p = nullptr;
+    CG_CUDA(rows.ensure(n * 4, p));
+    CG_CUDA(cudaMemcpyAsync(p, src, n * 4, cudaMemcpyHostToDevice, s));
+    dst = p;
     return CG_OK;
 }
 
@@ -391,15 +390,12 @@ extern "C" cg_status cg_mlp_features(const cg_volume* v, const cg_mlp* m, const 
     cg_context* ctx = v->ctx;
     CG_CUDA(cudaSetDevice(ctx->device));
     cudaStream_t s = pick_stream(ctx, stream);
-    DevBuf tin, tout;
+    RowBuf tin(ctx->rows_in), tout(ctx->rows_out);
     const float* dpos;
     cg_status st = stage_in(positions, (size_t)n * 3, on_device, tin, dpos, s);
     if (st != CG_OK) return st;
     float* dout = out;
-    if (!on_device) {
-        CG_CUDA(tout.ensure((size_t)n * MLP_IN * 4));
-        dout = tout.as<float>();
-    }
+    if (!on_device) CG_CUDA(tout.ensure((size_t)n * MLP_IN * 4, dout));
     st = ensure_textures(const_cast<cg_volume*>(v), s);
     if (st != CG_OK) return st;
     CG_LAUNCH(ctx, launch_mlp_features(desc_of(v), device_view(m), dpos, n, dir, dout, s));
@@ -419,15 +415,12 @@ extern "C" cg_status cg_mlp_infer(const cg_mlp* m, const float* features, int n,
     cg_context* ctx = m->ctx;
     CG_CUDA(cudaSetDevice(ctx->device));
     cudaStream_t s = pick_stream(ctx, stream);
-    DevBuf tin, tout;
+    RowBuf tin(ctx->rows_in), tout(ctx->rows_out);
     const float* df;
     cg_status st = stage_in(features, (size_t)n * MLP_IN, on_device, tin, df, s);
     if (st != CG_OK) return st;
     float* dout = out;
-    if (!on_device) {
-        CG_CUDA(tout.ensure((size_t)n * 4));
-        dout = tout.as<float>();
-    }
+    if (!on_device) CG_CUDA(tout.ensure((size_t)n * 4, dout));
     ctx->shaded_valid = false;
     ctx->infer_last = true;
     const unsigned long long launch = ++ctx->infer_launch;
@@ -500,7 +493,7 @@ extern "C" cg_status cg_mlp_gradient(cg_mlp* m, const float* features, const flo
     cg_context* ctx = m->ctx;
     CG_CUDA(cudaSetDevice(ctx->device));
     cudaStream_t s = ctx->stream;
-    DevBuf tf, tt;
+    RowBuf tf(ctx->rows_in), tt(ctx->rows_out);
     const float *df, *dt;
     cg_status st = stage_in(features, (size_t)n * MLP_IN, on_device, tf, df, s);
     if (st != CG_OK) return st;
