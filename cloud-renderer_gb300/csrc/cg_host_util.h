@@ -23,9 +23,11 @@ cg_status fail(cg_status s, const char* fmt, ...);
 #define CG_CUDA(call)                                                                      \
     do {                                                                                   \
         cudaError_t e_ = (call);                                                           \
-        if (e_ != cudaSuccess)                                                             \
+        if (e_ != cudaSuccess) {                                                           \
+            (void)cudaGetLastError(); /* reported here: not once more by the next launch */ \
             return fail(e_ == cudaErrorMemoryAllocation ? CG_ERR_OUT_OF_MEMORY : CG_ERR_CUDA, \
                         "%s: %s", #call, cudaGetErrorString(e_));                          \
+        }                                                                                  \
     } while (0)
 
 #define CG_CHECK(cond, status, ...)                  \
@@ -46,6 +48,7 @@ struct DevBuf {
         bytes = 0;
         cudaError_t e = cudaMalloc(&p, want ? want : 16);
         if (e == cudaSuccess) bytes = want;
+        else (void)cudaGetLastError();
         return e;
     }
     void release() {
@@ -88,6 +91,7 @@ struct HostBuf {
         bytes = 0;
         cudaError_t e = cudaMallocHost(&p, want ? want : 16);
         if (e == cudaSuccess) bytes = want;
+        else (void)cudaGetLastError();
         return e;
     }
     void release() {
