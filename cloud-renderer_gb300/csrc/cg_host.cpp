@@ -682,7 +682,10 @@ extern "C" cg_status cg_volume_set_billboards(cg_volume* v, const float* positio
     if (v->draw_pending) CG_CUDA(cudaStreamWaitEvent(s, v->boards_drawn, 0));
     if (need > v->boards.bytes || pairs * 4 > v->blist.bytes) CG_CUDA(cudaStreamSynchronize(s));
     v->read_pending = v->draw_pending = false;
+    // (growing gives the old records up first: where that fails the volume has no boards)
+    v->n = 0;
     CG_CUDA(v->boards.ensure(need));
+    CG_CUDA(v->blist.ensure(pairs * 4));
     char* dev = v->boards.as<char>();
     v->cwr = reinterpret_cast<float4*>(dev + o_cwr);
     v->q = reinterpret_cast<int4*>(dev + o_q);
@@ -690,7 +693,6 @@ extern "C" cg_status cg_volume_set_billboards(cg_volume* v, const float* positio
     v->dqb = reinterpret_cast<uint32_t*>(dev + o_dq);
     v->culled = reinterpret_cast<uint8_t*>(dev + o_cul);
     v->sun_boards = dev + o_sun;
-    CG_CUDA(v->blist.ensure(pairs * 4));
     if (n) {
         BoardGrid g;
         for (int a = 0; a < 3; ++a) {
@@ -872,6 +874,7 @@ cg_status voxelize_on(cg_volume* v, const cg_sun* sun, cudaStream_t s, const Vox
     const size_t texels = (size_t)sun->map_width * sun->map_height;
     if (v->mapW != sun->map_width || v->mapH != sun->map_height) {
         CG_CUDA(cudaStreamSynchronize(s));
+        v->mapW = v->mapH = 0;  // (none, until both have grown)
         CG_CUDA(v->keys.ensure(texels * 8 +
                                sun_aux_words(sun->map_width, sun->map_height) * 4));
         CG_CUDA(v->posmap.ensure(texels * 16));
@@ -1539,7 +1542,8 @@ extern "C" cg_status cg_volume_read_coverage(const cg_volume* v, uint32_t* count
 extern "C" cg_status cg_volume_read_sun_map(const cg_volume* v, uint64_t* keys, float* positions) {
     CG_CHECK(v && keys && positions, CG_ERR_INVALID_ARGUMENT,
              "cg_volume_read_sun_map: null pointer");
-    CG_CHECK(v->voxelized, CG_ERR_NOT_READY, "cg_volume_read_sun_map: not voxelized");
+    CG_CHECK(v->voxelized && v->mapW > 0, CG_ERR_NOT_READY,
+             "cg_volume_read_sun_map: not voxelized");
     cg_status st = sync_volume(v);
     if (st != CG_OK) return st;
     const size_t t = (size_t)v->mapW * v->mapH;
