@@ -312,7 +312,9 @@ cg_status capture(cg_frame_graph* g) {
     const int nv = (int)g->views.size();
     const size_t bytes = sizeof(BatchView) * (size_t)nv;
     if (g->desc.ensure(bytes + 16) != cudaSuccess ||
-        cudaMemcpy(g->desc.p, ctx->batch_dev.p, bytes, cudaMemcpyDeviceToDevice) != cudaSuccess) {
+        cudaMemcpyAsync(g->desc.p, ctx->batch_dev.p, bytes, cudaMemcpyDeviceToDevice, s) !=
+            cudaSuccess ||
+        cudaStreamSynchronize(s) != cudaSuccess) {
         ctx->timing = timing;
         return fail(CG_ERR_OUT_OF_MEMORY, "cg_frame_graph: descriptor buffer");
     }

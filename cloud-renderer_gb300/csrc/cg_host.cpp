@@ -391,6 +391,7 @@ extern "C" void cg_device_free(void* p) {
 extern "C" cg_status cg_memcpy(void* dst, const void* src, size_t bytes, int kind) {
     CG_CHECK(dst && src, CG_ERR_INVALID_ARGUMENT, "cg_memcpy: null pointer");
     CG_CUDA(cudaMemcpy(dst, src, bytes, (cudaMemcpyKind)kind));
+    if (kind != cudaMemcpyDeviceToHost) CG_CUDA(legacy_arrived());
     return CG_OK;
 }
 

@@ -35,6 +35,11 @@ cg_status fail(cg_status s, const char* fmt, ...);
         if (!(cond)) return fail(status, __VA_ARGS__); \
     } while (0)
 
+// cudaMemcpy and cudaMemset run on the legacy stream and may return before the device
+// has the data; the library's streams and most callers' do not wait for that stream.
+// Called behind the last of them, before anything that reads the data can be queued.
+inline cudaError_t legacy_arrived() { return cudaStreamSynchronize(cudaStreamLegacy); }
+
 // ---------------------------------------------------------------------------
 // device buffers
 // ---------------------------------------------------------------------------

@@ -87,6 +87,7 @@ cg_status upload_params(cg_mlp* m, const float* src) {
     set_consts(m, &p[MLP_B1], &p[MLP_B2], &p[MLP_B3], &p[MLP_W4], p[MLP_B4]);
     CG_CUDA(cudaMemcpy(m->params.p, p.data(), MLP_NPARAM * 4, cudaMemcpyHostToDevice));
     CG_CUDA(cudaMemcpy(m->w16.p, h.data(), MLP_NHALF * 2, cudaMemcpyHostToDevice));
+    CG_CUDA(legacy_arrived());
     return CG_OK;
 }
 
@@ -321,6 +322,7 @@ extern "C" cg_status cg_context_mlp_fallbacks(cg_context* ctx, uint64_t* out) {
     CG_CUDA(cudaMemcpy(&h, ctx->fallbacks.p, sizeof(h), cudaMemcpyDeviceToHost));
     if (h.infer.bits) {
         CG_CUDA(cudaMemset(ctx->infer_status(), 0, sizeof(InferStatus)));  // taken
+        CG_CUDA(legacy_arrived());
         return fail(CG_ERR_DEVICE_FAULT,
                     h.infer.bits & 2ull
                         ? "cg_mlp_infer: a tensor-core wait ran out of its time limit (1 s) and "
@@ -740,6 +742,7 @@ extern "C" cg_status cg_mlp_set_params(cg_mlp* m, const float* params, const flo
                            cudaMemcpyHostToDevice));
     }
     CG_CUDA(cudaMemcpy(m->step.p, &step, 4, cudaMemcpyHostToDevice));
+    CG_CUDA(legacy_arrived());
     m->host_step = step;
     return CG_OK;
 }
