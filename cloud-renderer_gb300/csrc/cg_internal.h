@@ -60,9 +60,10 @@ struct SunFrame {
 // Occupancy: for every level l a grid of occ_nb[l]^3 bytes, one per brick of
 // B^3 level-l texels, B = 1 << occ_shift (4, 8 or 16; a texel (x,y,z) is in
 // brick (x,y,z) >> occ_shift).  A byte is 1 when the brick or one of its 26
-// neighbours holds a voxel with density R > 0.  Because the mips are means of
-// non-negative values, a trilinear footprint whose brick reads 0 has R = 0
-// exactly, so samplers may skip it.
+// neighbours holds a voxel with density R > 0; above level 0, in volumes whose bars
+// are taller than a brick, also where they hold highlights alone (k_occ_coarse).
+// Because the mips are means of non-negative values, a trilinear footprint whose
+// brick reads 0 has R = 0 exactly, so samplers may skip it.
 struct VolDesc {
     int D, L, fmt;
     int dims[CG_MAX_LEVELS];
@@ -532,6 +533,11 @@ void batch_tiles(int lanes_per_ray, int width, int height, int& tiles_x, int& ti
 cudaError_t launch_trace_batch(int fmt, int lanes_per_ray, int unroll, const BatchView* views,
                                int n, unsigned total_tiles, unsigned* counter, cudaStream_t st);
 
+
+// cg_trace_cones with the reference's rule (k_compat.cu).
+cudaError_t launch_reference_cones(const VolDesc& vd, const TraceParams& tp,
+                                   const ConeSchedule& cs, const float* pos, int n, float* out,
+                                   cudaStream_t st);
 
 // ---- compat render (k_compat.cu) ------------------------------------------
 // The reference's billboard image formation; see cg_render_compat.

@@ -519,7 +519,8 @@ __device__ __forceinline__ float2 tri_light_pair(const VolDesc& vd, int l, float
     return halves(fma2(w[2], sub2(y1, y0), y0));
 }
 
-// The reference's weighted sum of the light channel (mode 1, clamp to edge).
+// The reference's weighted sum of the light channel (mode 1, clamp to edge), for a
+// finite position (tri_light's clamps take any other to an edge).
 template <int FMT>
 __device__ __forceinline__ float cone_reference(const VolDesc& vd, const ConeSchedule& cs,
                                                 float vx, float vy, float vz, float sx, float sy,
@@ -546,13 +547,7 @@ __device__ __forceinline__ float cone_reference(const VolDesc& vd, const ConeSch
 template <int FMT>
 __device__ __noinline__ float cone_general(const VolDesc& vd, const ConeSchedule& cs, float vx,
                                            float vy, float vz, float sx, float sy, float sz) {
-    if (cs.mode == 1) {
-        // tri_light's clamps would take a coordinate that is not finite to an edge;
-        // the blend of a NaN or of an infinity with its own floor is a NaN
-        if (cs.steps > 0 && !(isfinite(vx) && isfinite(vy) && isfinite(vz)))
-            return __int_as_float(0x7fc00000);
-        return cone_reference<FMT>(vd, cs, vx, vy, vz, sx, sy, sz);
-    }
+    if (cs.mode == 1) return cone_reference<FMT>(vd, cs, vx, vy, vz, sx, sy, sz);
     const float D = (float)vd.D, E = cs.edge;
     float tau = 0.f, comp = 0.f;
     for (int i = 0; i < cs.steps; ++i) {

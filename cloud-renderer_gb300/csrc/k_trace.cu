@@ -450,6 +450,7 @@ cudaError_t launch_trace_cones(VolDesc vd, TraceParams tp, const float* pos, int
                                cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
     ConeSchedule cs = make_cone_schedule(vd, tp);
+    if (cs.mode == 1) return launch_reference_cones(vd, tp, cs, pos, n, out, st);
     int blocks = (n + 127) / 128;
     if (vd.fmt == 0)
         k_trace_cones<0><<<blocks, 128, 0, st>>>(vd, tp, cs, pos, n, out);
