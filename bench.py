@@ -854,9 +854,9 @@ def animated_positions(base, frames, dt, seed=11):
 
 def run_animated(args):
     """Time-stepped form: every step moves the 4096 billboards, uploads them
-    (host quantization + copies), re-voxelizes the 256^3 BF16/FP16 volume and
-    renders one 1080p view with the BF16+MLP surrogate while the noise moves
-    with the wind (octaveOffsets = windVel * runTime, 60 steps per second of
+    (checked on the host, quantized on the device), re-voxelizes the 256^3
+    BF16/FP16 volume and renders one 1080p view with the BF16+MLP surrogate
+    while the noise moves with the wind (octaveOffsets = windVel * runTime, 60 steps per second of
     run time).  Metric: pixels / per-frame device time; the wall-clock rate
     of the same loop (host work included) is the e2e figure."""
     import numpy as np
@@ -948,7 +948,7 @@ def run_animated(args):
     ms = np.array([a.elapsed_time(b) for a, b in ev])
     total_ms = float(ms.sum())
     value = W * H * args.steps / (total_ms / 1e3) / 1e6
-    # the upload call alone on an idle device (host quantization + copies)
+    # the upload call alone on an idle device
     idle = []
     for k in range(min(20, frames)):
         torch.cuda.synchronize()
@@ -999,7 +999,7 @@ def run_animated(args):
             "e2e": {"value": round(W * H * args.steps / wall_s / 1e6, 3), "unit": "Mpix/s",
                     "h2d_bytes_per_step": n * 20, "d2h_bytes_per_step": 0,
                     "note": "wall clock of the same loop (L2 flush per step, no per-step "
-                            "events), host board quantization and upload included; the image "
+                            "events), board uploads included; the image "
                             "stays on the device"}}
     print(json.dumps(line), flush=True)
     vol32.close()

@@ -19,6 +19,11 @@
  * failures called exit(), Shader.cpp:35-36.)
  *
  * Threading: a context and its volumes are used from one thread at a time.
+ * Streams: the calls of a context share its scratch memory, so calls given to
+ * different streams are put in order by the caller (an event between them),
+ * like the images and volumes that they pass on.  Board uploads need no such
+ * care: they come after every voxelize, frame graph and compat render that
+ * still reads the boards, and before the next one.
  */
 #ifndef CLOUDGB_H
 #define CLOUDGB_H
@@ -439,7 +444,8 @@ cg_status cg_sun_map_noalloc(int dimension, float bound_min, float bound_max,
 cg_status cg_volume_set_occupancy_brick(cg_volume* vol, int brick);
 
 /* Launch shape of the fused renderer: lanes per ray 1 (one ray per thread,
- * 32 rays per warp), 4, 8 or 32 (one ray per warp); step-loop unroll 1, 2 or 4;
+ * 32 rays per warp), 4, 8 or 32 (one ray per warp); step-loop unroll 1, 2 or 4
+ * (with one lane per ray only the loop of rays with samples above level 0);
  * occupancy brick 4, 8 or 16 (0 = leave the volumes' own). */
 typedef struct cg_trace_config {
     int lanes_per_ray;
