@@ -150,11 +150,14 @@ extern "C" cg_status cg_render_compat(cg_context* ctx, const cg_volume* v, const
     cudaStream_t s = pick_stream(ctx, stream);
     // the noise map's green and alpha channels (the fragment program reads no other),
     // from which the device makes the cells; valid once this call has waited for s
+    // (until then the copy may still read `ga`)
+    std::vector<float> ga;
     const bool new_noise = !ctx->compat_noise_valid || ctx->compat_seed != params->noise_seed;
     if (new_noise) {
         constexpr size_t texels = (size_t)NOISE_N * NOISE_N * NOISE_N;
-        std::vector<float> rgba(texels * 4), ga(texels * 2);
+        std::vector<float> rgba(texels * 4);
         noise_map(params->noise_seed, rgba.data());
+        ga.resize(texels * 2);
         for (size_t i = 0; i < texels; ++i) {
             ga[2 * i] = rgba[4 * i + 1];
             ga[2 * i + 1] = rgba[4 * i + 3];

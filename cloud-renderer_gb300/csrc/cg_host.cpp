@@ -624,9 +624,9 @@ static cg_status check_boards(const cg_volume* v, const float* positions, const 
 }
 
 // The boards' records are made on the device (k_boards, which has the rules)
-// from the raw lists in page-locked memory: made here they took 24 ns a board,
-// 105 us of an update of 4096 (21 now, 355 -> 45 of 16384), and the upload waited for the context's
-// stream; it now only waits for the kernel that read the last one.
+// from the raw lists in page-locked memory: made here they took 24 ns a board, 102 us
+// of an update of 4096 (16.5 now; 384 -> 37 of 16384), and the upload waited for the
+// context's stream; it now only waits for the kernel that read the last one.
 extern "C" cg_status cg_volume_set_billboards(cg_volume* v, const float* positions,
                                               const float* scales, const float* densities,
                                               int count, float fluffiness) {
