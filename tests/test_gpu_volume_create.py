@@ -42,7 +42,7 @@ def _busy(ctx, frames):
 
 
 def test_creation_does_not_wait_for_queued_frames(ctx):
-    queue, whole = _busy(ctx, 60)
+    queue, whole = _busy(ctx, 200)
     for fmt in (cloudgb.FORMAT_RGBA32F, cloudgb.FORMAT_BF16_FP16):
         queue()
         vol = cloudgb.CloudVolume(64, configs.VOLUME_BOUNDS, configs.VOLUME_POSITION, 7, fmt=fmt,
